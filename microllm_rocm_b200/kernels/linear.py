@@ -1,7 +1,7 @@
 """Matrix products of the projections: y[M,N] = x[M,K] @ W[N,K]^T (+ bias).
 
-fp32 path: the hand-written CUDA-core kernel (`gemm_f32.cu`), plain fp32 FMA, fixed
-summation order.  bf16 path: bf16 operands with fp32 accumulation; the library product
+fp32 path: the hand-written CUDA-core kernels (`gemm_f32.cu`), plain fp32 FMA, one
+summation order whatever the number of rows.  bf16 path: bf16 operands with fp32 accumulation; the library product
 (cuBLASLt, see gemm_bf16.library_linear) stands where the reference calls hipBLASLt for the same
 projections (src/ops/optimized.cpp:349-403, BF16 x BF16 with 32-bit compute), and the
 hand-written weight-streaming kernels take over for steps of up to 128 tokens.
@@ -33,7 +33,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             raise KernelError("linear: the fp32 path produces fp32")
         if out is None:
             out = alloc((M, N), torch.float32) if alloc is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
-        ops.gemm_f32(x, weight, out, bias=bias)
+        ops.gemm_f32(x, weight, out, bias=bias, w_constant=True)
         return out
     if x.dtype != torch.bfloat16:
         raise KernelError(f"linear: unsupported dtype {x.dtype}")

@@ -71,7 +71,7 @@ _SIGNATURES = {
     },
     "gemm_f32.cu": {
         "mlb_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                         c_longlong, c_longlong, c_longlong, c_int, c_void_p],
+                         c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p],
     },
     "rope_kv.cu": {
         "mlb_rope_kv_write": [c_void_p, c_longlong, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -674,8 +674,9 @@ def stream_synchronize() -> None:
 
 # ------------------------------------------------------------------------------ fp32 GEMM
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-             accumulate: bool = False) -> None:
-    """out[M,N] (+)= a[M,K] @ w[N,K]^T (+ bias[N]); plain fp32 FMA on CUDA cores."""
+             accumulate: bool = False, w_constant: bool = False) -> None:
+    """out[M,N] (+)= a[M,K] @ w[N,K]^T (+ bias[N]); plain fp32 FMA on CUDA cores.  `w_constant`: no kernel of the same step
+    writes w, which may then be read while the kernel in front still runs."""
     _need(a, "a", torch.float32, 2); _need(w, "w", torch.float32, 2); _need(out, "out", torch.float32, 2)
     M, K = a.shape
     N = w.shape[0]
@@ -687,7 +688,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
             raise KernelError("gemm_f32: bias length differs from N")
     L = lib("gemm_f32.cu")
     build.check(L, L.mlb_gemm_f32(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, K, K, N,
-                                  1 if accumulate else 0, _stream()))
+                                  1 if accumulate else 0, 1 if w_constant else 0, _stream()))
 
 
 # ------------------------------------------------------------------------------ rope + kv store

@@ -114,6 +114,54 @@ def test_gemm_f32_row_does_not_depend_on_the_batch():
     assert torch.equal(full[40], one[0])
 
 
+def _fp32_product_in_its_order(a, w):
+    """The product's order of additions, spelled out: sixteen ranges of K, each an even and an odd chain of fused multiply-adds
+    (a product of two fp32 numbers is exact in fp64, and one fp64 addition rounded to fp32 is the fused result but for double
+    rounding), four ranges to a quarter, four quarters to the result."""
+    (M, K), N = a.shape, w.shape[0]
+    length = -(-K // 512) * 32
+    a, w = (torch.nn.functional.pad(t.cpu(), (0, 16 * length - K)).double() for t in (a, w))
+    total = None
+    for q in range(4):
+        quarter = None
+        for r in range(4 * q, 4 * q + 4):
+            chain = [torch.zeros(M, N), torch.zeros(M, N)]
+            for k in range(r * length, min((r + 1) * length, -(-K // 2) * 2)):
+                chain[k % 2] = (chain[k % 2].double() + a[:, k, None] * w[None, :, k]).float()
+            one = chain[0] + chain[1]
+            quarter = one if quarter is None else quarter + one
+        total = quarter if total is None else total + quarter
+    return total
+
+
+@pytest.mark.parametrize("K,pad", [(1, 0), (31, 0), (64, 1), (512, 0), (516, 3), (1100, 0)])
+def test_gemm_f32_has_one_order_of_additions_for_every_number_of_rows(K, pad):
+    """Every kernel form (1, 2, 4, 8, 16 rows streamed, tiles beyond 32), full and ragged, rows on 16 bytes and not, gives the
+    same bits; and they are those of the order that the kernel states."""
+    torch.manual_seed(K)
+    N, most = 70, 131
+    rows = torch.randn(most, K + pad, device=DEV)
+    w = torch.randn(N, K, device=DEV)
+    a = rows[:, :K].contiguous()
+    whole = torch.empty(most, N, device=DEV)
+    ops().gemm_f32(a, w, whole)
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65):
+        out = torch.empty(M, N, device=DEV)
+        ops().gemm_f32(a[:M].contiguous(), w, out, w_constant=M % 2 == 0)
+        assert torch.equal(out, whole[:M]), M
+    if pad:                                             # rows that do not start on 16 bytes: the same order
+        L = ops().lib("gemm_f32.cu")
+        for M in (2, 12, 50):
+            out = torch.empty(M, N, device=DEV)
+            assert L.mlb_gemm_f32(rows.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, K + pad, K, N, 0, 0,
+                                  torch.cuda.current_stream().cuda_stream) == 0
+            assert torch.equal(out, whole[:M]), M
+    want = _fp32_product_in_its_order(a[:9], w)
+    # the restatement rounds twice (to fp64, then to fp32): at most an ulp of a chain now and then
+    assert torch.allclose(whole[:9].cpu(), want, rtol=1e-6, atol=2e-7 * math.sqrt(K))
+    assert (whole[:9].cpu() == want).float().mean() > 0.99
+
+
 # ------------------------------------------------------------------------------ paged cache helpers
 def paged_from_dense(k, v, page_size, num_pages, dtype, seed=0):
     """k, v: lists (one per sequence) of [n, NKV, D].  Returns pages and a block table with
@@ -212,6 +260,26 @@ def test_paged_attention_prompts_and_decodes_in_one_batch(dtype, nh, nkv, d, win
     want = torch.cat([plain_attention_rows(q, k, v, l - n, window).reshape(n, nh * d)
                       for q, k, v, l, n in zip(qs, ks, vs, lens, news)])
     assert torch.allclose(got, want, **tol(dtype)), float((got - want).abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,d,window,page", [(1, 1, 4, None, 16), (9, 1, 20, None, 24), (6, 2, 36, 31, 24), (10, 1, 96, 300, 24), (4, 1, 100, None, 24),
+                                                  (12, 1, 128, None, 24), (2, 1, 136, 33, 24), (5, 1, 256, None, 24), (3, 1, 132, None, 24), (2, 2, 10, 64, 24)])
+def test_plain_attention_over_head_sizes_groups_and_cuts(dtype, nh, nkv, d, window, page):
+    """Head sizes on both sides of every column width (4 .. 256, and two that take the other kernel), groups of one to twelve heads, keys
+    behind several rounds of the eight warps; a token's bits are the same alone and among others."""
+    torch.manual_seed(nh * d + 1)
+    lens, news = [600, 257, 1, 32, 33], [5, 1, 1, 32, 2]
+    ks, vs = ([torch.randn(n, nkv, d) for n in lens] for _ in range(2))
+    qs = [torch.randn(n, nh, d) for n in news]
+    if dtype == torch.bfloat16:
+        ks, vs, qs = ([x.to(dtype).float() for x in y] for y in (ks, vs, qs))
+    pos0 = [l - n for l, n in zip(lens, news)]
+    got = run_attention(qs, ks, vs, pos0, nh, nkv, d, window, dtype, page_size=page)
+    want = torch.cat([plain_attention_rows(q, k, v, p, window).reshape(-1, nh * d) for q, k, v, p in zip(qs, ks, vs, pos0)])
+    assert torch.allclose(got, want, **tol(dtype)), float((got - want).abs().max())
+    alone = run_attention([qs[0][3:4]], ks[:1], vs[:1], [pos0[0] + 3], nh, nkv, d, window, dtype, page_size=page)
+    assert torch.equal(alone[0], got[3])
 
 
 @pytest.mark.parametrize("nh,nkv,d", [(12, 2, 128), (4, 4, 64), (6, 1, 64)])
