@@ -1,8 +1,7 @@
 // Plain attention over the paged cache: any mix of prompt portions and decoded tokens.
 //
-// One warp per (query token, query head).  The query at absolute position `pos` of its
-// sequence sees keys lo..pos, lo = max(0, pos - window + 1) for a windowed layer and 0
-// otherwise; keys beyond `pos` are never read (the reference computes no masked scores
+// The query at absolute position `pos` of its sequence sees keys lo..pos, lo = max(0, pos - window + 1) for a windowed layer
+// and 0 otherwise; keys beyond `pos` are never read (the reference computes no masked scores
 // either: src/ops/ops.cpp:2343-2384).  Query head h uses kv head h / (NH/NKV)
 // (ops.cpp:2357; consecutive query heads share one).  score = dot(q, k) * scale with the
 // scale applied after the dot product (ops.cpp:2365-2369); softmax and the value sum are
@@ -12,8 +11,11 @@
 // position, with a running maximum and sum.  The order of every addition therefore depends
 // only on (pos, window), not on how the prompt was cut into steps, on the other requests of
 // the batch, or on which physical pages hold the keys: in the fp32 path the same token gets
-// bit-identical output however it is scheduled.  This kernel is the whole fp32 path's
+// bit-identical output however it is scheduled.  These kernels are the whole fp32 path's
 // attention and the reference beside the tensor-core kernels.
+//
+//   paged_attention_rows_kernel    head sizes that are multiples of 4 (beyond 128: of 8)
+//   paged_attention_plain_kernel   the others, whose rows have no such pieces: a warp per (token, head)
 #include "common.cuh"
 
 using namespace mlb;
@@ -119,6 +121,225 @@ paged_attention_plain_kernel(AttnParams p) {
     }
 }
 
+// A CTA per query token and up to R query heads of one kv head, which share every key and value read.  Tile t of 32 keys
+// belongs to warp t % ROW_WARPS, so that one decoded token's keys are read from many places at once; each warp keeps its own
+// running maximum, sum and accumulator per row, and they meet in the order of the warps at the end.  Scores: eight lanes a key,
+// 16 bytes each, so that a warp's load takes whole 128-byte lines of four keys (a lane per key would touch 32 lines, and
+// did: 390 us for two decoded tokens of 12 heads behind 300 keys, 730 us for a prompt of 333; now 16 and 77); a lane
+// works on eight keys beside one another, and seven shuffles a row leave lane l with the score of key l.  Values: a lane per
+// VW neighbouring columns, VW * 32 >= head size.  What a row's bits are does not depend on R: few rows (two CTAs an SM at
+// most) get a CTA each, which then waits for memory only, so more of a tile is asked for at once (six heads together: 35 us
+// for the two decoded tokens).
+constexpr int ROW_WARPS = 8;
+
+template <typename KVT> __device__ __forceinline__ float4 load4(const KVT* p);
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+template <typename KVT, int VW> __device__ __forceinline__ void load_columns(const KVT* p, float (&v)[VW]) {
+    if constexpr (VW >= 4) {
+#pragma unroll
+        for (int i = 0; i < VW / 4; ++i) {
+            const float4 x = load4(p + 4 * i);
+            v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < VW; ++i) v[i] = to_f32(p[i]);
+    }
+}
+
+template <typename KVT, int VW, int R>
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) {
+    pdl_prologue();
+    extern __shared__ __align__(16) float shared[];
+    const int D = p.head_dim;
+    float* q_s = shared;                                       // [R][D]
+    float* acc_s = q_s + R * D;                                // [ROW_WARPS][R][D]
+    float* m_s = acc_s + ROW_WARPS * R * D;                    // [ROW_WARPS][R]
+    float* l_s = m_s + ROW_WARPS * R;
+    float* p_s = l_s + ROW_WARPS * R + (threadIdx.x >> 5) * (R * 32);        // this warp's probabilities of a tile
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = p.num_heads / p.num_kv_heads;
+    const int chunk = blockIdx.x % chunks, kvh = (blockIdx.x / chunks) % p.num_kv_heads, t = blockIdx.x / (chunks * p.num_kv_heads);
+    const int h0 = kvh * group + chunk * R, rows = min(R, group - chunk * R);
+    const int pos = p.positions[t], seq = p.token_seq[t];
+    const int lo = first_visible_key(pos, p.window, p.chunk);
+    const size_t q_at = ((size_t)t * p.num_heads + h0) * D;
+    for (int e = tid; e < R * D; e += ROW_WARPS * 32)
+        q_s[e] = e >= rows * D ? 0.0f : q_bf16 ? to_f32(((const __nv_bfloat16*)p.q)[q_at + e]) : ((const float*)p.q)[q_at + e];
+    __syncthreads();
+
+    float acc[R][VW], m[R], l[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        m[r] = -INFINITY; l[r] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VW; ++i) acc[r][i] = 0.0f;
+    }
+    const size_t page_stride = (size_t)2 * p.num_kv_heads * p.page_size * D;
+    const size_t v_offset = (size_t)p.num_kv_heads * p.page_size * D;
+    const int* table = p.block_table + (size_t)seq * p.max_blocks;
+    const KVT* pages = (const KVT*)p.pages;
+    const int key_group = lane >> 3, c = lane & 7, pieces = D / 4;
+    const bool column = lane * VW < D;
+
+    const int first = lo / 32, last = pos / 32;
+    for (int tile = first + (warp - first % ROW_WARPS + ROW_WARPS) % ROW_WARPS; tile <= last; tile += ROW_WARPS) {
+        const int kp = tile * 32 + lane;
+        bool valid = kp >= lo && kp <= pos;
+        long long k_off = 0;                                   // (a key that is not visible is read from the pool's first row)
+        if (valid) {
+            const int block = kp / p.page_size;
+            const int page = block < p.max_blocks ? table[block] : -1;
+            if (page < 0 || page >= p.num_pages) {
+                if (p.error_flag) atomicExch(p.error_flag, 2);
+                valid = false;
+            } else {
+                k_off = (long long)((size_t)page * page_stride + ((size_t)kvh * p.page_size + kp % p.page_size) * D);
+            }
+        }
+        float dot[R][8];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) dot[r][j] = 0.0f;
+        long long key_at[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) key_at[j] = __shfl_sync(0xffffffffu, k_off, key_group * 8 + j);
+        if (R == 1 && valid) {                                 // this lane's key and value, all lines of them
+            const char* row = (const char*)(pages + k_off);
+            for (int b = 0; b < D * (int)sizeof(KVT); b += 128) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(row + v_offset * sizeof(KVT) + b));
+            }
+        }
+#pragma unroll (R == 1 ? 4 : 1)
+        for (int piece = c; piece < pieces; piece += 8) {
+            float4 k[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) k[j] = load4(pages + key_at[j] + piece * 4);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float4 q = *reinterpret_cast<const float4*>(q_s + r * D + piece * 4);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dot[r][j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, fmaf(q.x, k[j].x, dot[r][j]))));
+            }
+        }
+        __syncwarp();                                          // every lane is done with the last tile's probabilities
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            // lane c of a key group ends up with the sum over the group's lanes of dot[r][c]
+            float a4[4], a2[2];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float keep = c & 4 ? dot[r][j + 4] : dot[r][j], give = c & 4 ? dot[r][j] : dot[r][j + 4];
+                a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float keep = c & 2 ? a4[j + 2] : a4[j], give = c & 2 ? a4[j] : a4[j + 2];
+                a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+            }
+            const float keep = c & 1 ? a2[1] : a2[0], give = c & 1 ? a2[0] : a2[1];
+            const float full = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+            const float s = valid ? full * p.scale : -INFINITY;
+            const float m_new = fmaxf(m[r], warp_max(s));
+            float prob = 0.0f;
+            if (m_new != -INFINITY) {                          // else: no readable key in this tile yet
+                prob = valid ? expf(s - m_new) : 0.0f;
+                const float corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
+                l[r] = l[r] * corr + warp_sum(prob);
+                m[r] = m_new;
+#pragma unroll
+                for (int i = 0; i < VW; ++i) acc[r][i] *= corr;
+            }
+            p_s[r * 32 + lane] = prob;
+        }
+        __syncwarp();
+        const unsigned seen = __ballot_sync(0xffffffffu, valid);
+#pragma unroll (R == 1 ? 4 : 2)
+        for (int j0 = 0; j0 < 32; j0 += 4) {
+            float v[4][VW];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const long long at = __shfl_sync(0xffffffffu, k_off, j0 + j);
+                if (column && ((seen >> (j0 + j)) & 1u)) {
+                    load_columns<KVT, VW>(pages + at + v_offset + lane * VW, v[j]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) v[j][i] = 0.0f;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float4 w = *reinterpret_cast<const float4*>(p_s + r * 32 + j0);
+#pragma unroll
+                for (int i = 0; i < VW; ++i) acc[r][i] = fmaf(w.w, v[3][i], fmaf(w.z, v[2][i], fmaf(w.y, v[1][i], fmaf(w.x, v[0][i], acc[r][i]))));
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (column) {
+#pragma unroll
+            for (int i = 0; i < VW; ++i) acc_s[(warp * R + r) * D + lane * VW + i] = acc[r][i];
+        }
+        if (lane == 0) { m_s[warp * R + r] = m[r]; l_s[warp * R + r] = l[r]; }
+    }
+    __syncthreads();
+    for (int e = tid; e < rows * D; e += ROW_WARPS * 32) {
+        const int r = e / D;
+        float top = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < ROW_WARPS; ++w) top = fmaxf(top, m_s[w * R + r]);
+        float sum = 0.0f, value = 0.0f;
+#pragma unroll
+        for (int w = 0; w < ROW_WARPS; ++w) {
+            const float mw = m_s[w * R + r];
+            if (mw == -INFINITY) continue;
+            const float f = expf(mw - top);
+            sum = fmaf(l_s[w * R + r], f, sum);
+            value = fmaf(acc_s[w * R * D + e], f, value);
+        }
+        const float o = value * (sum > 0.0f ? 1.0f / sum : 0.0f);
+        if (out_bf16) ((__nv_bfloat16*)p.out)[q_at + e] = from_f32<__nv_bfloat16>(o);
+        else ((float*)p.out)[q_at + e] = o;
+    }
+}
+
+template <typename KVT, int VW, int R>
+int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stream) {
+    static bool done[MAX_DEVICES] = {};
+    auto kernel = paged_attention_rows_kernel<KVT, VW, R>;
+    const int d = device_index();
+    constexpr int most = (R * VW * 32 * (ROW_WARPS + 1) + 2 * ROW_WARPS * R + ROW_WARPS * R * 32) * 4;
+    if (!done[d]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return check_launch("paged_attention_rows: shared memory");
+        done[d] = true;
+    }
+    const int group = p.num_heads / p.num_kv_heads, chunks = (group + R - 1) / R;
+    const long long blocks = (long long)p.tokens * p.num_kv_heads * chunks;
+    if (blocks > 0x7fffffffll) return fail(MLB_UNSUPPORTED_SIZE, "paged_attention_plain: %d tokens are more than one launch takes", p.tokens);
+    const size_t smem = (size_t)(R * p.head_dim * (ROW_WARPS + 1) + 2 * ROW_WARPS * R + ROW_WARPS * R * 32) * 4;
+    launch_kernel(kernel, (unsigned)blocks, ROW_WARPS * 32, smem, stream, p, q_bf16, out_bf16, chunks);
+    return check_launch("paged_attention_rows");
+}
+
+template <typename KVT>
+int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stream) {
+    // heads of a kv head together (at most four at head size 256, whose accumulators are long); one where there are few rows
+    const int group = p.tokens <= 2 * sm_count() / p.num_heads ? 1 : p.num_heads / p.num_kv_heads;
+    if (p.head_dim > 128) return group == 1 ? launch_rows<KVT, 8, 1>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 8, 4>(p, q_bf16, out_bf16, stream);
+    if (p.head_dim > 64) return group == 1 ? launch_rows<KVT, 4, 1>(p, q_bf16, out_bf16, stream)
+                                : group <= 4 ? launch_rows<KVT, 4, 4>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 4, 8>(p, q_bf16, out_bf16, stream);
+    return group == 1 ? launch_rows<KVT, 2, 1>(p, q_bf16, out_bf16, stream)
+           : group <= 4 ? launch_rows<KVT, 2, 4>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 2, 8>(p, q_bf16, out_bf16, stream);
+}
+
 }  // namespace
 
 MLB_EXPORT int mlb_paged_attention_plain(const void* q, int q_dtype, const void* pages, int kv_dtype, void* out,
@@ -135,6 +356,11 @@ MLB_EXPORT int mlb_paged_attention_plain(const void* q, int q_dtype, const void*
     if (tokens == 0) return MLB_OK;
     AttnParams p{q, pages, out, positions, token_seq, block_table, max_blocks, num_pages, page_size,
                  tokens, num_heads, num_kv_heads, head_dim, chunk, window, scale, error_flag};
+    const bool known = (q_dtype == MLB_F32 || q_dtype == MLB_BF16) && (out_dtype == MLB_F32 || (out_dtype == MLB_BF16 && q_dtype == MLB_BF16)) &&
+                       (kv_dtype == MLB_BF16 || (kv_dtype == MLB_F32 && q_dtype == MLB_F32 && out_dtype == MLB_F32));
+    if (known && head_dim % (head_dim > 128 ? 8 : 4) == 0 && (uintptr_t)pages % 16 == 0)
+        return kv_dtype == MLB_F32 ? launch_rows<float>(p, q_dtype == MLB_BF16, out_dtype == MLB_BF16, stream)
+                                   : launch_rows<__nv_bfloat16>(p, q_dtype == MLB_BF16, out_dtype == MLB_BF16, stream);
     const long long items = (long long)tokens * num_heads;
     const unsigned blocks = (unsigned)((items + WARPS - 1) / WARPS);
     if (q_dtype == MLB_F32 && kv_dtype == MLB_F32 && out_dtype == MLB_F32)
