@@ -13,9 +13,12 @@
 //   u      = splitmix64(seed + GOLDEN * (draw + 1)) >> 11, times 2^-53      in [0, 1)
 //   choose the first candidate, in index order, whose running weight sum exceeds u * total.
 // Ties at the top-k threshold go to the smaller index.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 using namespace mlb;
+namespace cg = cooperative_groups;
 
 MLB_DEFINE_LAST_ERROR()
 
@@ -221,6 +224,189 @@ __global__ void __launch_bounds__(THREADS) sample_rows_kernel(SampleParams p) {
     }
 }
 
+// The same selection with a cluster of CTAs per row, for large vocabularies.  One CTA a row reads its logits from memory six times
+// over (maximum, four digits of the threshold, weights) with one SM's bandwidth: 505 us for 41 rows of 151,936, top 50, where the
+// 25 MB need 4 us.  Here CTA r of the row's eight keeps its eighth in shared memory after one read, the digits are eleven bits
+// wide (three passes, and neighbouring logits fall into more bins, so that fewer atomics meet), and the CTAs' counts, sums and
+// picks meet through distributed shared memory: 85 us (150 with every bin summed by every CTA and no floor under the counting).  Threads own contiguous spans in index order, across the CTAs too,
+// so candidates are walked and ties are kept in the order that the one-CTA kernel has.
+constexpr int CLUSTER = 8, CLUSTER_THREADS = 512, WARPS = CLUSTER_THREADS / 32, BINS = 2048;
+constexpr int CLUSTER_MAX_SLICE = 52 * 1024;
+
+__global__ void __launch_bounds__(CLUSTER_THREADS) sample_rows_cluster_kernel(SampleParams p, int slice) {
+    pdl_prologue();
+    extern __shared__ float x[];                             // this CTA's logits
+    __shared__ float s_val[32];
+    __shared__ int s_idx[32];
+    __shared__ double s_dbl[32];
+    __shared__ int s_int[32];
+    __shared__ unsigned s_hist[2][BINS];                     // two: the next one is cleared while this one is filled
+    __shared__ float s_max[CLUSTER * WARPS];
+    __shared__ int s_flag, s_first, s_last, s_digit, s_left;
+    __shared__ struct { float best; int index, bad, eighth, equal, first, last; double sum; } meet;
+
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), row = blockIdx.x / CLUSTER, tid = threadIdx.x;
+    const float T = p.temperature ? p.temperature[row] : 0.0f;
+    int k = p.top_k ? p.top_k[row] : 0;
+    if (p.skip_greedy && (T == 0.0f || k == 1)) return;     // (the whole cluster)
+    const int V = p.vocab, from = min(rank * slice, V), count = min(slice, V - from);
+    const float* logits = p.logits + (size_t)row * p.ld + from;
+    if (tid == 0) { s_flag = 0; s_first = 0x7fffffff; s_last = -1; }
+    for (int i = tid; i < BINS; i += CLUSTER_THREADS) s_hist[0][i] = 0u;
+    __syncthreads();
+    float best = -INFINITY;
+    int best_i = 0x7fffffff;
+    bool bad = false;
+#pragma unroll 8
+    for (int i = tid; i < count; i += CLUSTER_THREADS) {
+        const float v = logits[i];
+        x[i] = v;
+        if (!isfinite(v)) bad = true;
+        if (v > best) { best = v; best_i = from + i; }
+    }
+    if (bad) atomicExch(&s_flag, 1);
+    block_argmax(best, best_i, s_val, s_idx);
+    __syncthreads();
+    if (tid == 0) { meet.best = best; meet.index = best_i; meet.bad = s_flag; }
+    cluster.sync();
+    int any_bad = 0;
+    best = -INFINITY;
+    for (int r = 0; r < CLUSTER; ++r) {                      // ranks in index order: the first maximum wins
+        const auto* other = cluster.map_shared_rank(&meet, r);
+        any_bad |= other->bad;
+        if (other->best > best) { best = other->best; best_i = other->index; }
+    }
+    if (any_bad || T == 0.0f || k == 1) {
+        if (rank == 0 && tid == 0) p.out[row] = any_bad ? -1 : best_i;
+        cluster.sync();
+        return;
+    }
+    if (k <= 0 || k > V) k = V;
+
+    // the key of the k-th largest logit, eleven, eleven and ten bits, and how many equal to it are kept
+    unsigned thr_key = 0u;
+    int keep_equal = 0x7fffffff;
+    if (k < V) {
+        // Nothing below the k-th largest of the warps' maxima (each a logit of its own) can be among the k largest: with few
+        // candidates wanted only a handful of logits is counted below.
+        unsigned floor_key = 0u;
+        if (k <= CLUSTER * WARPS) {
+            if (tid < CLUSTER * WARPS) s_max[tid] = cluster.map_shared_rank(s_val, tid / WARPS)[tid % WARPS];
+            __syncthreads();
+            if (tid < CLUSTER * WARPS) {
+                int larger = 0;
+                for (int j = 0; j < CLUSTER * WARPS; ++j) larger += s_max[j] > s_max[tid] || (s_max[j] == s_max[tid] && j < tid) ? 1 : 0;
+                if (larger == k - 1) s_digit = (int)sortable_key(s_max[tid]);
+            }
+            __syncthreads();
+            floor_key = (unsigned)s_digit;
+        }
+        int left = k;
+        for (int pass = 0; pass < 3; ++pass) {
+            const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0, bins = pass == 2 ? 1024 : BINS;
+            const unsigned mask = pass == 0 ? 0u : 0xffffffffu << (pass == 1 ? 21 : 10);
+            unsigned* hist = s_hist[pass & 1];
+            for (int i = tid; i < count; i += CLUSTER_THREADS) {
+                const unsigned key = sortable_key(x[i]);
+                if (key >= floor_key && (key & mask) == thr_key) atomicAdd(&hist[(key >> shift) & (unsigned)(bins - 1)], 1u);
+            }
+            if (pass < 2)
+                for (int i = tid; i < BINS; i += CLUSTER_THREADS) s_hist[1 - (pass & 1)][i] = 0u;
+            cluster.sync();                                  // all counted (and the other histogram was read before the last sync)
+            // CTA r adds up the r-th eighth of the bins, from the largest down, a thread each
+            const int each = bins / CLUSTER, bin = bins - 1 - (rank * each + tid);
+            int mine = 0;
+            if (tid < each) {
+#pragma unroll
+                for (int r = 0; r < CLUSTER; ++r) mine += (int)cluster.map_shared_rank(hist, r)[bin];
+            }
+            int all;
+            int before = block_exclusive_scan<int>(mine, s_int, all);
+            if (tid == 0) meet.eighth = all;
+            cluster.sync();
+            int in_front = 0;
+#pragma unroll
+            for (int r = 0; r < CLUSTER; ++r) {
+                const int n = cluster.map_shared_rank(&meet, r)->eighth;
+                if (r < rank) in_front += n;
+            }
+            before += in_front;
+            if (tid < each && before < left && before + mine >= left) {      // one thread of one CTA: it tells them all
+#pragma unroll
+                for (int r = 0; r < CLUSTER; ++r) { *cluster.map_shared_rank(&s_digit, r) = bin; *cluster.map_shared_rank(&s_left, r) = left - before; }
+            }
+            cluster.sync();
+            thr_key |= (unsigned)s_digit << shift;
+            left = s_left;
+        }
+        keep_equal = left;
+    }
+
+    // spans of an odd number of logits: neighbouring threads' first ones lie in different banks
+    const int span = ((slice + CLUSTER_THREADS - 1) / CLUSTER_THREADS) | 1;
+    const int begin = min(tid * span, count), end = min(begin + span, count);
+    int equal_before = 0;
+    if (k < V) {
+        int mine = 0, all;
+        for (int i = begin; i < end; ++i) mine += sortable_key(x[i]) == thr_key ? 1 : 0;
+        equal_before = block_exclusive_scan<int>(mine, s_int, all);
+        if (tid == 0) meet.equal = all;
+        cluster.sync();
+        for (int r = 0; r < rank; ++r) equal_before += cluster.map_shared_rank(&meet, r)->equal;
+    }
+    const float max_scaled = best / T;
+    auto candidate = [&](int i, int& equal) {
+        if (k == V) return true;
+        const unsigned key = sortable_key(x[i]);
+        return key > thr_key || (key == thr_key && equal++ < keep_equal);
+    };
+    double partial = 0.0;
+    int equal = equal_before;
+    for (int i = begin; i < end; ++i)
+        if (candidate(i, equal)) partial += exp((double)(x[i] / T - max_scaled));
+    double total;
+    double before = block_exclusive_scan<double>(partial, s_dbl, total);
+    if (tid == 0) meet.sum = total;
+    cluster.sync();
+    total = 0.0;
+    for (int r = 0; r < CLUSTER; ++r) {
+        const double sum = cluster.map_shared_rank(&meet, r)->sum;
+        if (r == rank) before += total;
+        total += sum;
+    }
+    const double target = uniform_from(p.seed[row], p.draw[row]) * total;
+    if (partial > 0.0) {
+        atomicMax(&s_last, tid);
+        if (before + partial > target) atomicMin(&s_first, tid);
+    }
+    __syncthreads();
+    if (tid == 0) { meet.first = s_first; meet.last = s_last; }
+    cluster.sync();
+    int owner_rank = -1, owner = -1;
+    for (int r = 0; r < CLUSTER && owner_rank < 0; ++r) {
+        const int first = cluster.map_shared_rank(&meet, r)->first;
+        if (first != 0x7fffffff) { owner_rank = r; owner = first; }
+    }
+    for (int r = CLUSTER - 1; r >= 0 && owner_rank < 0; --r) {      // rounding left the target at the very end
+        const int last = cluster.map_shared_rank(&meet, r)->last;
+        if (last >= 0) { owner_rank = r; owner = last; }
+    }
+    if (rank == owner_rank && tid == owner) {
+        double running = before;
+        int chosen = -1, last = -1;
+        equal = equal_before;
+        for (int i = begin; i < end && chosen < 0; ++i) {
+            if (!candidate(i, equal)) continue;
+            last = from + i;
+            running += exp((double)(x[i] / T - max_scaled));
+            if (running > target) chosen = last;
+        }
+        p.out[row] = chosen >= 0 ? chosen : last;
+    }
+    cluster.sync();                                          // nobody leaves while its `meet` is read
+}
+
 __global__ void __launch_bounds__(THREADS) argmax_rows_kernel(const float* __restrict__ logits, long long ld,
                                                               int vocab, int* __restrict__ out) {
     pdl_prologue();
@@ -352,6 +538,33 @@ MLB_EXPORT int mlb_sample_rows(const float* logits, long long ld, int rows, int 
         int status = check_launch("argmax_split");
         if (status != MLB_OK) return status;
         p.skip_greedy = 1;
+    }
+    // Eight CTAs a row where an eighth fits an SM's shared memory and is worth a CTA (the vocabulary that greedy selection splits
+    // too); else one, whose six reads of a short row come from L2.
+    const int slice = (vocab + CLUSTER - 1) / CLUSTER;
+    if (vocab >= SPLIT_MIN_VOCAB && slice <= CLUSTER_MAX_SLICE && rows <= 0x7fffffff / CLUSTER) {
+        static bool configured[MAX_DEVICES] = {};
+        const int d = device_index();
+        if (!configured[d]) {
+            if (cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CLUSTER_MAX_SLICE * 4 / 1024 * 1024) != cudaSuccess)
+                return check_launch("sample_rows: shared memory");
+            configured[d] = true;
+        }
+        cudaLaunchConfig_t config = {};
+        config.gridDim = rows * CLUSTER;
+        config.blockDim = CLUSTER_THREADS;
+        config.dynamicSmemBytes = (size_t)slice * 4;
+        config.stream = stream;
+        cudaLaunchAttribute attributes[2];
+        attributes[0].id = cudaLaunchAttributeClusterDimension;
+        attributes[0].val.clusterDim.x = CLUSTER;
+        attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+        attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attributes[1].val.programmaticStreamSerializationAllowed = 1;
+        config.attrs = attributes;
+        config.numAttrs = pdl_enabled() ? 2 : 1;
+        cudaLaunchKernelEx(&config, sample_rows_cluster_kernel, p, slice);
+        return check_launch("sample_rows_cluster");
     }
     launch_kernel(sample_rows_kernel, rows, THREADS, 0, stream, p);
     return check_launch("sample_rows");

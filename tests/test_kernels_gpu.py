@@ -679,6 +679,29 @@ def test_sampling_kernel_matches_the_plain_sampler(vocab):
     assert out.tolist() == want
 
 
+@pytest.mark.parametrize("vocab", [16384, 16387, 151936, 425984, 425985])
+def test_sampling_over_a_clusters_slices_matches_the_plain_sampler(vocab):
+    """The smallest vocabulary that eight CTAs share, a ragged one, a real one, the largest and one more (one CTA again): ties at
+    the threshold on both sides of a slice's edge, a row of few distinct values, one of a single value, one that is not finite."""
+    torch.manual_seed(vocab)
+    rows = 10
+    x = torch.randn(rows, vocab) * 2
+    edge = -(-vocab // 8)
+    for i in (3, edge - 1, edge, edge + 1, vocab - 1):
+        x[1, i] = x[2, i] = 30.0
+    x[3] = torch.round(x[3])
+    x[4] = 1.5
+    x[5, vocab // 2] = float("nan")
+    temps = [0.8, 0.7, 0.7, 1.0, 1.3, 0.8, 0.0, 0.9, 2.0, 0.5]
+    topk = [50, 3, 4, 1000, 0, 50, 0, vocab - 1, 0, 1]
+    seeds, draws = [11, 3, 4, 5, 6, 7, 8, 9, 1 << 40, 1], list(range(rows))
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    ops().sample_rows(x.to(DEV), torch.tensor(temps).to(DEV), torch.tensor(topk, dtype=torch.int32).to(DEV),
+                      torch.tensor(seeds, dtype=torch.int64).to(DEV), torch.tensor(draws, dtype=torch.int64).to(DEV), out)
+    want = [-1 if r == 5 else plain.sample_token(x[r].numpy(), temps[r], topk[r], seeds[r], draws[r]) for r in range(rows)]
+    assert out.tolist() == want
+
+
 def test_sampling_kernel_follows_the_distribution():
     logits = torch.tensor([[0.0, 1.0, 2.0, 0.5, -1.0]]).repeat(4000, 1)
     out = torch.empty(4000, dtype=torch.int32, device=DEV)
