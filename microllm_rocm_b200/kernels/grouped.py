@@ -13,6 +13,8 @@ import torch
 
 from . import build, ops
 from .build import KernelError
+from .device import sm_count
+from .gemm_bf16 import device_error_flag
 
 SOURCE = "grouped_gemm.cu"
 ops.register_signatures(SOURCE, {
@@ -29,12 +31,23 @@ ops.register_signatures(MMA_SOURCE, {
                         c_int, c_int, c_void_p, c_void_p],
 })
 
+# CTA pairs on the fifth-generation tensor cores: groups of many rows (csrc/grouped_tc2.cu)
+PAIR_SOURCE = "grouped_tc2.cu"
+ops.register_signatures(PAIR_SOURCE, {
+    "mlb_grouped_pair": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "mlb_gather_rows": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
+})
+
+# None: pair_pays decides; tests set it to True or False to send listed products to the pair kernel, or not
+USE_PAIRS = None
+
 # Tests set it to False to send bf16 products to the CUDA-core kernel and compare.
 USE_TENSOR_CORES = True
 
 
 def sources():
-    return [(SOURCE, {}), (MMA_SOURCE, {})]
+    return [(SOURCE, {}), (MMA_SOURCE, {}), (PAIR_SOURCE, {})]
 
 
 def mma_supported(a: torch.Tensor, weight: torch.Tensor, a_group_cols: int = 0) -> bool:
@@ -43,6 +56,44 @@ def mma_supported(a: torch.Tensor, weight: torch.Tensor, a_group_cols: int = 0) 
     return (USE_TENSOR_CORES and a.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.shape[2] % 8 == 0
             and a.stride(0) % 8 == 0 and weight.stride(1) % 8 == 0 and weight.stride(0) % 8 == 0 and a_group_cols % 8 == 0
             and a.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def pair_supported(a: torch.Tensor, weight: torch.Tensor) -> bool:
+    """The pair kernel reads its operands by TMA out of whole matrices: what the tensor-core kernel takes, the weights of the
+    groups one behind another."""
+    G, N, K = weight.shape
+    return mma_supported(a, weight) and G <= 1024 and weight.is_contiguous() and a.stride(1) == 1 and G * N < 1 << 31
+
+
+def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: int) -> bool:
+    """Tiles of 256 weight rows for pairs of SMs: worth it for large groups whatever their number, for groups of 16 rows and more where
+    every pair has a tile, and for small groups whose weights (`weight_bytes` a group) take long enough to read that the set-up of a
+    pair does not show.  Measured (gate/up + down, us, mma.sync against pairs): 64 groups of 1,408, width 2,048: 24 listed rows
+    46 + 27 / 44 + 30, 48 rows 69 + 43 / 65 + 39, 1,200 rows 181 + 101 / 128 + 64, 12,288 rows 616 + 379 / 184 + 112; 32 of 704: 256 rows 39 + 20 / 43 + 23,
+    512 rows 55 + 25 / 45 + 24; 16 of 512, width 1,024: 256 rows 18 + 17 / 35 + 19, 1,024 rows 23 + 15 / 26 + 16, 1,600 rows 39 + 15 / 27 + 16."""
+    if USE_PAIRS is not None:
+        return USE_PAIRS
+    active = min(groups, rows)
+    return rows >= 96 * groups or (rows >= 16 * groups and -(-weight_rows // 256) * active >= sms // 2) or active * weight_bytes >= 200 << 20
+
+
+def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_rows, dual, act, row_scale, alloc, error_flag):
+    G, w_rows, K = weight.shape
+    flag = error_flag if error_flag is not None else device_error_flag(a.device)
+    L = ops.lib(PAIR_SOURCE)
+    source = a
+    if a_rows is not None:                               # the pair kernel reads rows as they lie: in the order of the list
+        source = alloc((rows, K), a.dtype) if alloc is not None else torch.empty((rows, K), dtype=a.dtype, device=a.device)
+        build.check(L, L.mlb_gather_rows(a.data_ptr(), a.stride(0), a_rows.data_ptr(), int(a_row_div), group_offsets.data_ptr(), G,
+                                         source.data_ptr(), int(rows), K, ops._stream()))
+    # one tile for most groups: the mean and a quarter more
+    mean = rows / min(G, rows)
+    cap = 32 if mean <= 16 else min(256, max(64, -(-int(1.25 * mean) // 64) * 64))
+    sms = sm_count(a.device)
+    build.check(L, L.mlb_grouped_pair(
+        source.data_ptr(), source.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0), group_offsets.data_ptr(), ops._ptr(c_rows),
+        ops._ptr(row_scale), ops._ptr(a_rows) if row_scale is not None else None, 1 if out.dtype == torch.bfloat16 else 0, 1 if dual else 0,
+        int(act), outputs if dual else 0, int(rows), outputs, K, G, w_rows, cap, sms - sms % 2, flag.data_ptr(), ops._stream()))
 
 
 def row_tile_for(rows: int, groups: int, listed: bool, tensor_cores: bool) -> int:
@@ -57,7 +108,7 @@ def row_tile_for(rows: int, groups: int, listed: bool, tensor_cores: bool) -> in
 def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, rows: int, a_group_cols: int = 0,
                    c_group_cols: int = 0, group_offsets: Optional[torch.Tensor] = None, a_rows: Optional[torch.Tensor] = None,
                    c_rows: Optional[torch.Tensor] = None, a_row_div: int = 1, factor: Optional[torch.Tensor] = None,
-                   row_scale: Optional[torch.Tensor] = None, row_tile: int = 64) -> None:
+                   row_scale: Optional[torch.Tensor] = None, row_tile: int = 64, error_flag: Optional[torch.Tensor] = None) -> None:
     """weight [G, N, K]; a [*, lda] and out [*, ldc] are 2-D and row-major.
 
     group g multiplies the K columns of `a` that start at g * a_group_cols with weight[g] and writes N columns of
@@ -83,6 +134,11 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
             raise KernelError("grouped_linear: the factor matrix is narrower than the output")
     if row_scale is not None:
         ops._need(row_scale, "row_scale", torch.float32)
+    if (group_offsets is not None and a_rows is None and factor is None and row_scale is None and not a_group_cols and not c_group_cols
+            and pair_supported(a, weight) and pair_pays(rows, G, N, weight.stride(0) * 2, sm_count(a.device))):
+        _pair(a, weight, out, rows=rows, outputs=N, group_offsets=group_offsets, a_rows=None, a_row_div=1, c_rows=c_rows, dual=False, act=0,
+              row_scale=None, alloc=None, error_flag=error_flag)
+        return
     tensor_cores = mma_supported(a, weight, a_group_cols) and row_scale is None
     if row_tile == 128 and not tensor_cores:
         row_tile = 64
@@ -104,7 +160,8 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
 
 def grouped_silu_mul(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, rows: int, group_offsets: torch.Tensor,
                      a_rows: Optional[torch.Tensor] = None, a_row_div: int = 1, row_tile: int = 64, alloc=None,
-                     activation: str = "silu", limit: Optional[float] = None, row_scale: Optional[torch.Tensor] = None) -> None:
+                     activation: str = "silu", limit: Optional[float] = None, row_scale: Optional[torch.Tensor] = None,
+                     error_flag: Optional[torch.Tensor] = None) -> None:
     """weight [G, 2 * F, K]: per group F gate rows over F up rows; out[place] = silu(a gate^T) * (a up^T), [rows, F]; or,
     with `activation` "clamped_swish" and its `limit`, the clamped form (ops.activation_code).  `row_scale` (fp32, one number per
     entry that a_rows may name): both products are multiplied by row_scale[a_rows[place]] in front of the activation, which is a
@@ -124,6 +181,10 @@ def grouped_silu_mul(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *
         ops._need(group_offsets, "group_offsets", torch.int32, 1)
         if a_rows is not None:
             ops._need(a_rows, "a_rows", torch.int32, 1)
+        if pair_supported(a, weight) and pair_pays(rows, G, two_f, weight.stride(0) * 2, sm_count(a.device)):
+            _pair(a, weight, out, rows=rows, outputs=F, group_offsets=group_offsets, a_rows=a_rows, a_row_div=a_row_div, c_rows=None, dual=True,
+                  act=ops.activation_code(activation, limit), row_scale=row_scale, alloc=alloc, error_flag=error_flag)
+            return
         L = ops.lib(MMA_SOURCE)
         build.check(L, L.mlb_grouped_mma(
             a.data_ptr(), a.stride(0), 0, weight.data_ptr(), weight.stride(1), weight.stride(0), out.data_ptr(), out.stride(0), 0,

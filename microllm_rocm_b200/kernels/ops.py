@@ -130,6 +130,7 @@ def lagged_sources():
     out = [("attention_tc.cu", {"HEAD_DIM": 128, "MLB_LAG_WARP": w}) for w in (0, 1, 2, 5)]
     out += [("gemm_stream.cu", {"MLB_LAG_WARP": w}) for w in (0, 1, 3)]
     out += [("gemm_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
+    out += [("grouped_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
     out += [("attention_mma.cu", {"HEAD_DIM": 128, "MLB_LAG_WARP": w}) for w in (1, 4)]
     return out
 
@@ -169,7 +170,7 @@ def base_sources():
 def part_sources():
     """(source, defines) of the kernels that only some kinds of parts ask for (each part names its own in
     `kernel_sources`)."""
-    return [("residual.cu", {}), ("grouped_gemm.cu", {}), ("grouped_mma.cu", {}), ("latent.cu", {}), ("moe.cu", {}),
+    return [("residual.cu", {}), ("grouped_gemm.cu", {}), ("grouped_mma.cu", {}), ("grouped_tc2.cu", {}), ("latent.cu", {}), ("moe.cu", {}),
             ("layernorm.cu", {}), ("short_conv.cu", {}), ("state_space.cu", {}), ("attention_kv.cu", {}), ("delta_rule.cu", {}),
             ("linear_attention.cu", {}), ("post_norm.cu", {}), ("streams.cu", {})]
 

@@ -188,9 +188,10 @@ class RoutedExperts(FeedForward):
         act = buf("act", (P, ff), self.rt.dtype)
         grouped.grouped_silu_mul(x, self.w_gate_up, act, rows=P, group_offsets=offsets, a_rows=order, a_row_div=top,
                                  row_tile=row_tile, alloc=lambda shape, dtype: buf("gate_up", shape, dtype), activation=self.activation, limit=self.limit,
-                                 row_scale=weights.view(-1) if weigh_in else None)
+                                 row_scale=weights.view(-1) if weigh_in else None, error_flag=flag)
         y = buf("y", (P, W), torch.float32)
-        grouped.grouped_linear(act, self.w_down, y, rows=P, group_offsets=offsets, c_rows=order if dest is None else dest, row_tile=row_tile)
+        grouped.grouped_linear(act, self.w_down, y, rows=P, group_offsets=offsets, c_rows=order if dest is None else dest, row_tile=row_tile,
+                               error_flag=flag)
         if partials:
             return y.view(top, T, W) if top > 1 else y
         shared = self.shared.forward(x, ctx) if self.shared is not None else None

@@ -162,6 +162,54 @@ def test_gemm_f32_has_one_order_of_additions_for_every_number_of_rows(K, pad):
     assert (whole[:9].cpu() == want).float().mean() > 0.99
 
 
+# ------------------------------------------------------------------------------ grouped products of many rows
+@pytest.mark.parametrize("N,K,counts", [(72, 104, [0, 1, 31, 32, 33, 64, 65, 0]), (256, 64, [255, 256, 257, 300]), (264, 520, [700, 0, 0, 5]),
+                                        (40, 2048, [128, 129, 191, 193, 40, 20]), (1408, 128, [24]), (136, 72, [1, 2, 0, 3, 33, 1])])
+def test_grouped_pair_product_over_row_counts(N, K, counts):
+    """Rows on every side of the tiles' and the instruction's steps (32 columns; tiles of 64 .. 256), groups without rows, places behind
+    the list, ragged K and N: plain results in another row order, and the gated form with scales on the rows that go in."""
+    from microllm_rocm_b200.kernels import grouped
+    torch.manual_seed(N + K)
+    G, listed = len(counts), sum(counts)
+    rows = listed + 9                                    # (choices without an expert leave places behind the list)
+    offsets = torch.tensor(np.cumsum([0] + counts), dtype=torch.int32, device=DEV)
+    group = torch.repeat_interleave(torch.arange(G), torch.tensor(counts))
+    a = torch.randn(rows, K, device=DEV).bfloat16()
+    w = (torch.randn(G, N, K, device=DEV) * K ** -0.5).bfloat16()
+    assert grouped.pair_supported(a, w)
+    grouped.USE_PAIRS = True
+    try:
+        c_rows = torch.randperm(rows).to(torch.int32).to(DEV)
+        out = torch.full((rows, N), -7.0, device=DEV)
+        grouped.grouped_linear(a, w, out, rows=rows, group_offsets=offsets, c_rows=c_rows)
+        want = torch.einsum("rk,rnk->rn", a[:listed].double(), w.double()[group.to(DEV)])
+        got = out[c_rows.long()].double()
+        # exact products, K fp32 additions of terms of magnitude K^-1/2
+        assert float((got[:listed] - want).abs().max()) < 2e-7 * 6 * math.sqrt(K)
+        assert bool((got[listed:] == -7.0).all()), "a place behind the list was written"
+        F = N // 2
+        w2 = (torch.randn(G, 2 * F, K, device=DEV) * K ** -0.5).bfloat16()
+        order = torch.randperm(rows).to(torch.int32).to(DEV)
+        scale = torch.rand(rows, device=DEV) + 0.5
+        for activation, limit in (("silu", None), ("clamped_swish", 0.75)):
+            act = torch.full((rows, F), -7.0, device=DEV, dtype=torch.bfloat16)
+            grouped.grouped_silu_mul(a, w2, act, rows=rows, group_offsets=offsets, a_rows=order, activation=activation, limit=limit, row_scale=scale)
+            x = a[order.long()[:listed]].double() * scale[order.long()[:listed], None].double()
+            both = torch.einsum("rk,rnk->rn", x, w2.double()[group.to(DEV)])
+            g, u = both[:, :F], both[:, F:]
+            if activation == "silu":
+                want = g * torch.sigmoid(g) * u
+            else:
+                g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+                want = g * torch.sigmoid(1.702 * g) * (u + 1)
+            # half an ulp of bf16, and the sums' error through the activation
+            assert torch.allclose(act[:listed].double(), want, rtol=2 ** -8, atol=1e-4)
+            assert bool((act[listed:] == -7.0).all())
+    finally:
+        grouped.USE_PAIRS = None
+    torch.cuda.synchronize()
+
+
 # ------------------------------------------------------------------------------ paged cache helpers
 def paged_from_dense(k, v, page_size, num_pages, dtype, seed=0):
     """k, v: lists (one per sequence) of [n, NKV, D].  Returns pages and a block table with
@@ -435,6 +483,21 @@ def served_size_cases(flag):
         gemm_bf16.gemm_pair(x5, w5, out, dual_rows=8960, error_flag=flag)
         return out
     cases["pair_dual"] = pair_dual
+    from microllm_rocm_b200.kernels import grouped
+    counts = [300, 0, 190, 256, 1, 220, 513, 64]
+    offsets = torch.tensor(np.cumsum([0] + counts), dtype=torch.int32, device=DEV)
+    xg, wg, wd = rand(sum(counts), 1408), rand(8, 2048, 1408, scale=0.02), rand(8, 2 * 1408, 1408, scale=0.02)
+
+    def grouped_pair():
+        out = torch.empty(sum(counts), 2048, device=DEV)
+        grouped.grouped_linear(xg, wg, out, rows=sum(counts), group_offsets=offsets, error_flag=flag)
+        return out
+
+    def grouped_pair_dual():
+        out = torch.empty(sum(counts), 1408, dtype=torch.bfloat16, device=DEV)
+        grouped.grouped_silu_mul(xg, wd, out, rows=sum(counts), group_offsets=offsets, error_flag=flag)
+        return out
+    cases["grouped_pair"], cases["grouped_pair_dual"] = grouped_pair, grouped_pair_dual
     x6 = rand(8, 1536)
 
     def gemv():
@@ -494,7 +557,7 @@ def test_kernels_with_barriers_or_rings_give_the_same_bits_beside_a_memory_hog(k
 def held_back_builds():
     from microllm_rocm_b200.kernels import ops as o
     uses = {"attention_tc.cu": ["prompt"], "gemm_stream.cu": ["stream_partials", "stream_many_tiles", "stream_silu"],
-            "gemm_tc2.cu": ["pair", "pair_dual"], "attention_mma.cu": ["decode_ring"]}
+            "gemm_tc2.cu": ["pair", "pair_dual"], "grouped_tc2.cu": ["grouped_pair", "grouped_pair_dual"], "attention_mma.cu": ["decode_ring"]}
     return [(source, tuple(sorted(defines.items())), case) for source, defines in o.lagged_sources() for case in uses[source]]
 
 
