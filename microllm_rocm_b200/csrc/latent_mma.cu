@@ -12,6 +12,10 @@
 //   values   P[16 x 32] goes to shared memory as bf16; each warp owns a quarter of the R output columns and adds
 //            P V for them (V = the first R columns of the same cache rows, fetched with ldmatrix.trans)
 // A sink (one learned number per head) enters the denominator once, with no value.
+// In prompts of many rows a CTA holds GROUPS = 2 such groups of four warps with 16 rows each: they share the ring of keys, which is
+// most of a CTA's shared memory, so that four groups and not two fit a multiprocessor and cover each other's barriers (a
+// tile is a serial path of scores, softmax and values with four of them).  A row's bits stay the same: a tile that only the other
+// group's rows see adds nothing.  2,048 tokens of 16 heads, 512 + 64 wide: 632 us with one group, 426 with two.
 // With `splits` > 1 a work item's key tiles are divided among that many CTAs, which leave unnormalised partial
 // outputs with their maximum and sum in a workspace; latent_merge_kernel puts them together (and adds the sink).
 #include "common.cuh"
@@ -69,32 +73,42 @@ constexpr int KW = (KS + 3) / 4;          // of which a warp takes every fourth:
 constexpr int SP = BN + 4;                // pitch of a row of partial scores, in floats
 
 template <int STAGES>
-struct Smem {
+struct Ring {
     __nv_bfloat16 k[STAGES][BN][KP];
+};
+struct Group {
     __nv_bfloat16 p[BM][PP];
     float part[4][BM][SP];                // each warp's partial scores of the tile
     float red_max[4][BM];
     float red_sum[4][BM];
 };
+template <int STAGES, int GROUPS> constexpr size_t smem_bytes() { return sizeof(Ring<STAGES>) + GROUPS * sizeof(Group); }
+static_assert(sizeof(Ring<2>) % 16 == 0 && sizeof(Group) % 16 == 0, "a group's tiles are read in 16-byte pieces");
 
-template <int STAGES>
-__global__ void __launch_bounds__(128)
+template <int STAGES, int GROUPS>
+__global__ void __launch_bounds__(128 * GROUPS, GROUPS == 1 ? 1 : 2)
 latent_mma_kernel(Params p) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem<STAGES>& s = *reinterpret_cast<Smem<STAGES>*>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int seq = p.work[2 * blockIdx.x], first_row = p.work[2 * blockIdx.x + 1];
+    Ring<STAGES>& ring = *reinterpret_cast<Ring<STAGES>*>(smem_raw);
+    const int tid = threadIdx.x, group = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31;
+    Group& s = reinterpret_cast<Group*>(smem_raw + sizeof(Ring<STAGES>))[group];
+    auto meet = [&] {                                                      // the four warps of a group
+        if (GROUPS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+    };
+    const int seq = p.work[2 * blockIdx.x], cta_row = p.work[2 * blockIdx.x + 1], first_row = cta_row + BM * group;
     const int split = blockIdx.y;
     const int H = p.heads;
     const int seq_start = p.seq_starts[seq], n_new = p.seq_starts[seq + 1] - seq_start;
     const int pos0 = p.seq_pos0[seq];
-    const int rows = min(BM, n_new * H - first_row);                       // rows of this tile that exist
+    const int cta_rows = min(BM * GROUPS, n_new * H - cta_row);            // rows of this tile that exist,
+    const int rows = min(BM, n_new * H - first_row);                       // and of this group (none: it only helps with the keys)
     const size_t row_base = (size_t)seq_start * H + first_row;             // global (token, head) row of the tile's first row
     const int* table = p.block_table + (size_t)seq * p.max_blocks;
 
     // what the tile's rows may see: from the first row's lower edge to the last row's own position
-    const int pos_first = pos0 + first_row / H, pos_last = pos0 + (first_row + rows - 1) / H;
+    const int pos_first = pos0 + cta_row / H, pos_last = pos0 + (cta_row + cta_rows - 1) / H;
     const int lo_tile = (p.window > 0 && pos_first - p.window + 1 > 0) ? pos_first - p.window + 1 : 0;
     const int tile_first = lo_tile / BN, tile_count_all = pos_last / BN - tile_first + 1;
     const int t_begin = tile_first + (int)((long long)tile_count_all * split / p.splits);
@@ -118,9 +132,10 @@ latent_mma_kernel(Params p) {
             qa[i][3] = in && g + 8 < rows ? *reinterpret_cast<const unsigned*>(q1 + col + 8) : 0u;
         }
     }
-    // Four threads share a cache row: each looks the row's page up ONCE per tile and copies every fourth 16-byte piece.
+    // Four threads a group share a cache row: each looks the row's page up ONCE per tile and copies its share of the 16-byte pieces.
     auto load_keys = [&](int stage, int tile) {
-        const int row = tid >> 2;
+        constexpr int SHARE = 4 * GROUPS;
+        const int row = tid / SHARE;
         const int kp = tile * BN + row;
         bool ok = kp >= lo_tile && kp <= pos_last;
         const __nv_bfloat16* src = p.pages;
@@ -135,8 +150,8 @@ latent_mma_kernel(Params p) {
             }
         }
 #pragma unroll
-        for (int piece = tid & 3; piece < DK / 8; piece += 4)
-            cp_async16(&s.k[stage][row][piece * 8], ok ? src + piece * 8 : p.pages, ok);
+        for (int piece = tid % SHARE; piece < DK / 8; piece += SHARE)
+            cp_async16(&ring.k[stage][row][piece * 8], ok ? src + piece * 8 : p.pages, ok);
     };
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) {
@@ -181,8 +196,8 @@ latent_mma_kernel(Params p) {
             const int ks = warp + 4 * i;
             if (ks < KS) {                                  // the same for the whole warp
                 unsigned b0[4], b1[4];
-                ldmatrix_x4(b0, &s.k[stage][(lane & 7) + 8 * (lane >> 4)][ks * 16 + 8 * ((lane >> 3) & 1)]);
-                ldmatrix_x4(b1, &s.k[stage][16 + (lane & 7) + 8 * (lane >> 4)][ks * 16 + 8 * ((lane >> 3) & 1)]);
+                ldmatrix_x4(b0, &ring.k[stage][(lane & 7) + 8 * (lane >> 4)][ks * 16 + 8 * ((lane >> 3) & 1)]);
+                ldmatrix_x4(b1, &ring.k[stage][16 + (lane & 7) + 8 * (lane >> 4)][ks * 16 + 8 * ((lane >> 3) & 1)]);
                 mma_bf16(sp[0], qa[i], b0[0], b0[1]);
                 mma_bf16(sp[1], qa[i], b0[2], b0[3]);
                 mma_bf16(sp[2], qa[i], b1[0], b1[1]);
@@ -194,7 +209,7 @@ latent_mma_kernel(Params p) {
             *reinterpret_cast<float2*>(&s.part[warp][lane >> 2][j * 8 + 2 * (lane & 3)]) = make_float2(sp[j][0], sp[j][1]);
             *reinterpret_cast<float2*>(&s.part[warp][(lane >> 2) + 8][j * 8 + 2 * (lane & 3)]) = make_float2(sp[j][2], sp[j][3]);
         }
-        __syncthreads();
+        meet();
         // ---- from here on warp w owns keys 8 w .. 8 w + 7 of the tile: their scores are the four warps' partial sums, in order
         float sc[4];
 #pragma unroll
@@ -223,7 +238,7 @@ latent_mma_kernel(Params p) {
             part_max[h] = v;
         }
         if ((lane & 3) == 0) { s.red_max[warp][lane >> 2] = part_max[0]; s.red_max[warp][(lane >> 2) + 8] = part_max[1]; }
-        __syncthreads();
+        meet();
         float corr[2], part_sum[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -240,7 +255,7 @@ latent_mma_kernel(Params p) {
             part_sum[h] = v;
         }
         if ((lane & 3) == 0) { s.red_sum[warp][lane >> 2] = part_sum[0]; s.red_sum[warp][(lane >> 2) + 8] = part_sum[1]; }
-        __syncthreads();
+        meet();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = (lane >> 2) + 8 * h;
@@ -256,7 +271,7 @@ latent_mma_kernel(Params p) {
 #pragma unroll
             for (int j = 0; j < NT; j += 2) {
                 unsigned v[4];
-                ldmatrix_x4_trans(v, &s.k[stage][ks * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][warp * WR + j * 8 + 8 * (lane >> 4)]);
+                ldmatrix_x4_trans(v, &ring.k[stage][ks * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][warp * WR + j * 8 + 8 * (lane >> 4)]);
                 mma_bf16(acc[j], a, v[0], v[1]);
                 if (j + 1 < NT) mma_bf16(acc[j + 1], a, v[2], v[3]);
             }
@@ -340,16 +355,16 @@ latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
     }
 }
 
-template <int STAGES>
+template <int STAGES, int GROUPS>
 int launch_attention(const Params& p, int num_work, cudaStream_t stream) {
     static bool configured[MAX_DEVICES] = {false};
-    const size_t smem = sizeof(Smem<STAGES>);
+    const size_t smem = smem_bytes<STAGES, GROUPS>();
     if (!configured[device_index()]) {
-        if (cudaFuncSetAttribute(latent_mma_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(latent_mma_kernel<STAGES, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return fail(MLB_UNSUPPORTED_SIZE, "latent_attention_mma: %zu bytes of shared memory per CTA are not available", smem);
         configured[device_index()] = true;
     }
-    launch_kernel(latent_mma_kernel<STAGES>, dim3(num_work, p.splits), 128, smem, stream, p);
+    launch_kernel(latent_mma_kernel<STAGES, GROUPS>, dim3(num_work, p.splits), 128 * GROUPS, smem, stream, p);
     return check_launch("latent_attention_mma");
 }
 
@@ -358,22 +373,24 @@ int launch_attention(const Params& p, int num_work, cudaStream_t stream) {
 MLB_EXPORT int mlb_latent_mma_widths(int which) { return which == 0 ? R : DR; }
 
 // q [T*H, R+DR] bf16, pages [num_pages, page_size, R+DR] bf16, out [T*H, R] bf16.  work: num_work (sequence, first row)
-// pairs, each a tile of up to 16 (token, head) rows of one sequence.  splits > 1 needs part_o [splits, T*H, R] and
+// pairs, each a tile of up to 16 * groups (token, head) rows of one sequence; groups is 1, or 2 where splits is 1.  splits > 1 needs part_o [splits, T*H, R] and
 // part_ml [splits, T*H, 2] fp32.
 MLB_EXPORT int mlb_latent_attention_mma(const void* q, const void* pages, void* out, const float* sink, const int* seq_starts,
                                         const int* seq_pos0, const int* block_table, const int* work, int num_work,
                                         float* part_o, float* part_ml, int max_blocks, int num_pages, int page_size,
-                                        int heads, int window, int splits, int total_rows, float scale, int* error_flag,
+                                        int heads, int window, int splits, int groups, int total_rows, float scale, int* error_flag,
                                         cudaStream_t stream) {
     if (num_work < 0 || heads <= 0 || splits < 1 || splits > MAX_SPLITS || total_rows < 0 || page_size <= 0 || num_pages <= 0 || max_blocks <= 0 || window < 0)
         return fail(MLB_INVALID_ARGUMENT, "latent_attention_mma: bad sizes");
+    if (groups != 1 && (groups != 2 || splits != 1)) return fail(MLB_INVALID_ARGUMENT, "latent_attention_mma: %d groups a CTA", groups);
     if (splits > 1 && (!part_o || !part_ml)) return fail(MLB_INVALID_ARGUMENT, "latent_attention_mma: split keys need a workspace");
     if (num_work == 0) return MLB_OK;
     Params p{(const __nv_bfloat16*)q, (const __nv_bfloat16*)pages, (__nv_bfloat16*)out, sink, seq_starts, seq_pos0, block_table, work,
              part_o, part_ml, max_blocks, num_pages, page_size, heads, window, splits, total_rows, scale, error_flag};
     // shared keys: few tiles per CTA, all of them in flight at once (if four stages fit this device's shared memory)
-    const bool deep = splits > 1 && sizeof(Smem<4>) <= 200 * 1024;
-    int status = deep ? launch_attention<4>(p, num_work, stream) : launch_attention<2>(p, num_work, stream);
+    const bool deep = splits > 1 && smem_bytes<4, 1>() <= 200 * 1024;
+    int status = deep ? launch_attention<4, 1>(p, num_work, stream)
+               : groups == 2 ? launch_attention<2, 2>(p, num_work, stream) : launch_attention<2, 1>(p, num_work, stream);
     if (status != MLB_OK || splits == 1) return status;
     launch_kernel(latent_merge_kernel, total_rows, 128, 0, stream, (const float*)part_o, (const float*)part_ml, sink,
                   (__nv_bfloat16*)out, splits, total_rows, heads);

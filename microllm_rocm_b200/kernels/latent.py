@@ -29,9 +29,9 @@ MMA_SOURCE = "latent_mma.cu"
 ops.register_signatures(MMA_SOURCE, {
     "mlb_latent_mma_widths": [c_int],
     "mlb_latent_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
+                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
 })
-ROWS_PER_TILE = 16                  # (token, head) rows of one sequence that a CTA of the tensor-core kernel owns
+ROWS_PER_TILE = 16                  # (token, head) rows of one sequence that a group of warps of the tensor-core kernel owns
 KEYS_PER_TILE = 32
 MIN_KEY_TILES_PER_SPLIT = 4         # a CTA that shares a work item's keys streams 128 of them at least
 MAX_SPLITS = 64
@@ -54,25 +54,29 @@ def key_splits(num_work: int, max_seq_len: int, sms: int) -> int:
 
 
 def _plan(ctx, heads: int):
-    """Work items of a step ((sequence, first row) per 16 rows of a sequence's new (token, head) rows; long causal
-    ranges first) and the key split, shared by every layer with this many heads."""
+    """Work items of a step ((sequence, first row) per 16 rows of a sequence's new (token, head) rows, or 32; long causal
+    ranges first), the key split and the groups of 16 rows a CTA holds, shared by every layer with this many heads.  Two
+    groups where four a multiprocessor have work, and the keys are not split."""
     from .device import sm_count
     key = ("latent_mma", heads)
     plan = ctx.extras.get(key)
     if plan is not None:
         return plan
     starts = ctx.seq_starts_host
+    device = ctx.positions.device
+    sms = sm_count(device)
+    rows = [(starts[a + 1] - starts[a]) * heads for a in range(ctx.num_seqs)]
+    tiles = sum(-(-n // ROWS_PER_TILE) for n in rows)
+    splits = key_splits(tiles, ctx.max_seq_len, sms) if ctx.decode_only or tiles <= 32 else 1
+    groups = 2 if splits == 1 and not ctx.decode_only and tiles >= 4 * sms else 1
     work = []
     for a in range(ctx.num_seqs):
-        rows = (starts[a + 1] - starts[a]) * heads
         pos0 = ctx.seq_pos0_host[a] if ctx.seq_pos0_host else 0
-        work += [(pos0 + first // heads, a, first) for first in range(0, rows, ROWS_PER_TILE)]
+        work += [(pos0 + first // heads, a, first) for first in range(0, rows[a], groups * ROWS_PER_TILE)]
     if not ctx.decode_only:
         work.sort(key=lambda item: -item[0])
-    device = ctx.positions.device
     work_dev = ops.upload([x for _, a, first in work for x in (a, first)], "int32", device)
-    splits = key_splits(len(work), ctx.max_seq_len, sm_count(device)) if ctx.decode_only or len(work) <= 32 else 1
-    plan = ctx.extras[key] = (work_dev, len(work), splits)
+    plan = ctx.extras[key] = (work_dev, len(work), splits, groups)
     return plan
 
 
@@ -104,7 +108,7 @@ def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Opt
     num_pages, page_size, width = pages.shape
     if width != rank + rot_dim or q.shape[1] != heads * width or tuple(out.shape) != (T, heads * rank):
         raise KernelError("latent.attention: shapes do not agree")
-    work, num_work, splits = _plan(ctx, heads)
+    work, num_work, splits, groups = _plan(ctx, heads)
     part_o = part_ml = None
     if splits > 1:
         part_o = ctx.buffer("latent.part_o", (splits, T * heads, rank), torch.float32)
@@ -113,7 +117,7 @@ def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Opt
     build.check(L, L.mlb_latent_attention_mma(
         q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(),
         block_table.data_ptr(), work.data_ptr(), num_work, ops._ptr(part_o), ops._ptr(part_ml), block_table.shape[1], num_pages,
-        page_size, heads, int(window or 0), splits, T * heads, float(scale), ops._ptr(ctx.error_flag), ops._stream()))
+        page_size, heads, int(window or 0), splits, groups, T * heads, float(scale), ops._ptr(ctx.error_flag), ops._stream()))
 
 
 def sources():
