@@ -6,7 +6,9 @@ There is no CPU path and no silent fallback: a missing compiler or extension rai
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -32,7 +34,14 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _current_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
+_launch_on = threading.local()
+
+
 def _stream() -> int:
+    """Where this thread's launches go: the current stream, or the side stream inside on_side_stream()."""
+    side = getattr(_launch_on, "side", None)
+    if side is not None:
+        return side
     if _raw_stream is not None and _current_device is not None:
         return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
@@ -664,6 +673,20 @@ def join(side: int) -> None:
     """The current stream waits for everything queued on the side stream."""
     L = lib("basic.cu")
     build.check(L, L.mlb_stream_join(side, _stream()))
+
+
+@contextlib.contextmanager
+def on_side_stream():
+    """This library's launches inside go to the device's second stream, which continues from where the current one stands; the
+    caller joins (`join(side)`, side being what this yields) before anything reads what they write, and lets go of none of their
+    tensors before that.  Only for work that launches kernels of this library and nothing through the tensor framework."""
+    side = side_stream()
+    fork(side)
+    _launch_on.side = side
+    try:
+        yield side
+    finally:
+        _launch_on.side = None
 
 
 def stream_synchronize() -> None:

@@ -4,7 +4,7 @@ reference: src/model/model.cpp:757-794; activation src/ops/ops.cpp:760-785) or t
 `activation="clamped_swish"` with `limit` L: g = min(gate(x), L), u = clamp(up(x), -L, L), down(g * sigmoid(1.702 g) * (u + 1))."""
 from __future__ import annotations
 
-from typing import Dict
+from typing import Dict, Optional
 
 import torch
 
@@ -60,6 +60,14 @@ class SwiGLU(FeedForward):
 
     def own_tensors(self):
         return [self.w_gate_up, self.w_down]
+
+    def streams_weights(self, x: torch.Tensor, ctx: Optional[StepContext]) -> bool:
+        """Whether both products of these tokens run on this library's weight-streaming kernels, whose scratch is the step's: then
+        forward may be issued on the device's second stream (the library product's workspace belongs to one stream)."""
+        if ctx is None or x.dtype != torch.bfloat16 or self.w_down.dtype != torch.bfloat16:
+            return False
+        act = scratch(ctx, "swiglu.act", (x.shape[0], self.inter), self.rt.dtype, x.device)
+        return all(gemm_bf16.gemv_preferred(a, w) or gemm_bf16.stream_preferred(a, w) for a, w in ((x, self.w_gate_up), (act, self.w_down)))
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         # fp32 path: everything f32.  bf16 path: gate/up leave the product as bf16, the

@@ -27,10 +27,15 @@ from typing import Dict, Optional
 
 import torch
 
-from ..kernels import gemm_bf16, grouped, moe
+from ..kernels import gemm_bf16, grouped, moe, ops
 from ..kernels.linear import linear
 from ..kernels.ops import CLAMPED_ACTIVATION
 from .base import FEED_FORWARDS, FeedForward, Runtime, StepContext, WeightSpec, make, register_feed_forward, scratch
+
+
+# Steps up to which the shared expert runs beside the router (a decode step of 8 requests, 64 experts of 1,408 and a shared one of
+# 2,816, eight layers: 1.71 ms a step one after the other, 1.58 side by side)
+SIDE_MAX_TOKENS = 32
 
 
 @register_feed_forward("routed_experts")
@@ -167,6 +172,12 @@ class RoutedExperts(FeedForward):
         dev, P = x.device, x.shape[0] * self.top
         flag = ctx.error_flag if ctx is not None else None
         buf = lambda role, shape, dtype: scratch(ctx, "routed." + role, shape, dtype, dev)
+        # Few tokens: the shared expert's weights stream while the router, the choice and the sorting of the pairs, each a few round
+        # trips long, pass on the main stream.  Many tokens fill the device on their own.
+        shared = side = None
+        if self.shared is not None and T <= SIDE_MAX_TOKENS and getattr(self.shared, "streams_weights", None) and self.shared.streams_weights(x, ctx):
+            with ops.on_side_stream() as side:
+                shared = self.shared.forward(x, ctx)
         ids = buf("ids", (T, top), torch.int32)
         weights = buf("weights", (T, top), torch.float32)
         gate = buf("shared_gate", (T,), torch.float32) if self.has_gate else None
@@ -194,7 +205,10 @@ class RoutedExperts(FeedForward):
                                error_flag=flag)
         if partials:
             return y.view(top, T, W) if top > 1 else y
-        shared = self.shared.forward(x, ctx) if self.shared is not None else None
+        if side is not None:
+            ops.join(side)
+        elif self.shared is not None:
+            shared = self.shared.forward(x, ctx)
         out = buf("out", (T, W), torch.float32)
         if self.identity:
             moe.combine(y, weights, out, shared=shared, gate=gate, col_scale=out_scale, ids=ids, experts=E, x=x)

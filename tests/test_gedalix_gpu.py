@@ -370,3 +370,55 @@ def test_greedy_generation_through_the_scheduler(folders, dtype):
             else:       # bf16 may leave the fp32 choice at a near tie: every pick must be a near maximum of the plain logits
                 assert float(ref.max() - ref[token]) <= 0.05 * float(ref.abs().max())
             seq.append(token)
+
+
+# ------------------------------------------------------------------------------------------- two streams in a step
+def test_the_shared_expert_beside_the_router_changes_no_bits():
+    """Steps of few tokens run the shared expert on the device's second stream: the same logits, step by step and in captured
+    decode steps, as with everything on one."""
+    import copy
+
+    from microllm_rocm_b200.config.gedalix import PRESETS, GedalixConfig
+    from microllm_rocm_b200.engine.decode_graph import DecodeGraphPool
+    from microllm_rocm_b200.engine.loading import random_engine
+    from microllm_rocm_b200.engine.step import StepEntry
+    from microllm_rocm_b200.parts import routed
+    from microllm_rocm_b200.sampling import GenerationConfig
+    raw = copy.deepcopy(PRESETS["gedalix-small"])
+    raw["layers"], raw["max_positions"] = raw["layers"][:3], 256
+    config = GedalixConfig.from_dict(raw)
+    greedy = GenerationConfig(max_new_tokens=30, temperature=0.0)
+
+    def run(limit):
+        kept, routed.SIDE_MAX_TOKENS = routed.SIDE_MAX_TOKENS, limit
+        try:
+            engine = random_engine(config, seed=3, max_tokens=1024, max_requests=16, draw_on_device=True)
+            out = []
+            for batch in (1, 8, 13):
+                ids = [f"{batch}.{i}" for i in range(batch)]
+                for rid in ids:
+                    engine.cache.add(rid)
+                out.append(engine.step([StepEntry(rid, [7 + i, 11, 13 * i], [2]) for i, rid in enumerate(ids)]).clone())
+                out.append(engine.step([StepEntry(rid, [100 + i], [0]) for i, rid in enumerate(ids)]).clone())
+                graph = DecodeGraphPool(engine).get(ids, headroom_tokens=30)
+                logits = {}
+                graph.ctx.tensor_sink = lambda name, t: logits.__setitem__(name, t)
+                state = ([5] * batch, [4] * batch, [greedy] * batch, [0] * batch)
+                for rid in ids:
+                    engine.cache.reserve(rid, 30)
+                graph.load(ids, *state)
+                graph.capture()
+                graph.load(ids, *state)
+                for _ in range(20):
+                    graph.replay()
+                    out.append(logits["logits"][:batch].clone())
+                    graph.read_tokens()
+                for rid in ids:
+                    engine.cache.release(rid)
+            engine.check_device_errors()
+            return out
+        finally:
+            routed.SIDE_MAX_TOKENS = kept
+
+    one, two = run(0), run(32)
+    assert all(torch.equal(a, b) for a, b in zip(one, two))
