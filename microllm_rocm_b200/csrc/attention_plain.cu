@@ -125,7 +125,7 @@ paged_attention_plain_kernel(AttnParams p) {
 // belongs to warp t % ROW_WARPS, so that one decoded token's keys are read from many places at once; each warp keeps its own
 // running maximum, sum and accumulator per row, and they meet in the order of the warps at the end.  Scores: eight lanes a key,
 // 16 bytes each, so that a warp's load takes whole 128-byte lines of four keys (a lane per key would touch 32 lines, and
-// did: 390 us for two decoded tokens of 12 heads behind 300 keys, 730 us for a prompt of 333; now 16 and 77); a lane
+// did: 390 us for two decoded tokens of 12 heads behind 300 keys, 730 us for a prompt of 333; now 14 and 77); a lane
 // works on eight keys beside one another, and seven shuffles a row leave lane l with the score of key l.  Values: a lane per
 // VW neighbouring columns, VW * 32 >= head size.  What a row's bits are does not depend on R: few rows (two CTAs an SM at
 // most) get a CTA each, which then waits for memory only, so more of a tile is asked for at once (six heads together: 35 us
@@ -217,16 +217,32 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(row + v_offset * sizeof(KVT) + b));
             }
         }
-#pragma unroll (R == 1 ? 4 : 1)
-        for (int piece = c; piece < pieces; piece += 8) {
-            float4 k[8];
+        if (R == 1 && pieces <= 32) {                          // all of the lane's pieces of its eight keys at once
+            float4 k[4][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) k[j] = load4(pages + key_at[j] + piece * 4);
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float4 q = *reinterpret_cast<const float4*>(q_s + r * D + piece * 4);
+                for (int j = 0; j < 8; ++j)
+                    if (c + 8 * i < pieces) k[i][j] = load4(pages + key_at[j] + (c + 8 * i) * 4);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) dot[r][j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, fmaf(q.x, k[j].x, dot[r][j]))));
+            for (int i = 0; i < 4; ++i)
+                if (c + 8 * i < pieces) {
+                    const float4 q = *reinterpret_cast<const float4*>(q_s + (c + 8 * i) * 4);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        dot[0][j] = fmaf(q.w, k[i][j].w, fmaf(q.z, k[i][j].z, fmaf(q.y, k[i][j].y, fmaf(q.x, k[i][j].x, dot[0][j]))));
+                }
+        } else {
+            for (int piece = c; piece < pieces; piece += 8) {
+                float4 k[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) k[j] = load4(pages + key_at[j] + piece * 4);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float4 q = *reinterpret_cast<const float4*>(q_s + r * D + piece * 4);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) dot[r][j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, fmaf(q.x, k[j].x, dot[r][j]))));
+                }
             }
         }
         __syncwarp();                                          // every lane is done with the last tile's probabilities
@@ -261,11 +277,12 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
         }
         __syncwarp();
         const unsigned seen = __ballot_sync(0xffffffffu, valid);
-#pragma unroll (R == 1 ? 4 : 2)
-        for (int j0 = 0; j0 < 32; j0 += 4) {
-            float v[4][VW];
+        constexpr int BATCH = R == 1 ? 16 : 4;                 // keys whose values are asked for together
+#pragma unroll (R == 1 ? 1 : 2)
+        for (int j0 = 0; j0 < 32; j0 += BATCH) {
+            float v[BATCH][VW];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < BATCH; ++j) {
                 const long long at = __shfl_sync(0xffffffffu, k_off, j0 + j);
                 if (column && ((seen >> (j0 + j)) & 1u)) {
                     load_columns<KVT, VW>(pages + at + v_offset + lane * VW, v[j]);
@@ -275,10 +292,14 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
                 }
             }
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float4 w = *reinterpret_cast<const float4*>(p_s + r * 32 + j0);
+            for (int b = 0; b < BATCH; b += 4) {
 #pragma unroll
-                for (int i = 0; i < VW; ++i) acc[r][i] = fmaf(w.w, v[3][i], fmaf(w.z, v[2][i], fmaf(w.y, v[1][i], fmaf(w.x, v[0][i], acc[r][i]))));
+                for (int r = 0; r < R; ++r) {
+                    const float4 w = *reinterpret_cast<const float4*>(p_s + r * 32 + j0 + b);
+#pragma unroll
+                    for (int i = 0; i < VW; ++i)
+                        acc[r][i] = fmaf(w.w, v[b + 3][i], fmaf(w.z, v[b + 2][i], fmaf(w.y, v[b + 1][i], fmaf(w.x, v[b][i], acc[r][i]))));
+                }
             }
         }
     }
