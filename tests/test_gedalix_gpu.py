@@ -372,6 +372,28 @@ def test_greedy_generation_through_the_scheduler(folders, dtype):
             seq.append(token)
 
 
+@pytest.mark.parametrize("top, width", [(1, 96), (2, 2048), (3, 100), (4, 1028), (6, 2048), (8, 64), (9, 64), (6, 70)])
+@pytest.mark.parametrize("partials, gated, scaled", [(0, False, False), (1, True, True), (3, True, False)])
+def test_the_experts_results_are_summed_over_tops_and_widths(top, width, partials, gated, scaled):
+    """Four columns a thread (up to eight choices, widths that are multiples of four) and column by column (the others)."""
+    from microllm_rocm_b200.kernels import moe
+    torch.manual_seed(top * width)
+    T = 9
+    y, w = torch.randn(T * top, width, device=DEV), torch.rand(T, top, device=DEV)
+    shared = torch.randn(max(1, partials), T, width, device=DEV)
+    gate, scale = torch.rand(T, device=DEV), torch.rand(width, device=DEV)
+    out = torch.empty(T, width, device=DEV)
+    moe.combine(y, w, out, shared=(shared if partials > 1 else shared[0]) if partials else None, gate=gate if gated else None,
+                col_scale=scale if scaled else None)
+    want = (y.double().view(T, top, width) * w.double()[:, :, None]).sum(1)
+    if partials:
+        want = want + shared.double().sum(0) * (gate.double()[:, None] if gated else 1.0)
+    if scaled:
+        want = want * scale.double()
+    # at most top + partials + 2 roundings of terms of a few units
+    assert float((out.double() - want).abs().max()) < (top + partials + 2) * 2 ** -24 * 32
+
+
 # ------------------------------------------------------------------------------------------- two streams in a step
 def test_the_shared_expert_beside_the_router_changes_no_bits():
     """Steps of few tokens run the shared expert on the device's second stream: the same logits, step by step and in captured
