@@ -406,10 +406,16 @@ MLB_EXPORT int mlb_scatter_int(int* dst, int dst_len, const int* dst_index, cons
 // Two kernels of a step that do not depend on each other (the attention of the prompt portions and the attention
 // of the decoded tokens beside them) may run side by side: the first goes to a second stream that starts where
 // the main stream stands (fork) and the main stream waits for it before it goes on (join).  One stream and one
-// event of each kind per device, made at first use.
+// event of each kind per device and host thread, made at first use: a thread that captures a step must not find another one's launches
+// on its second stream, nor its events recorded over.
 namespace {
-struct SideStream { cudaStream_t stream; cudaEvent_t forked, joined; bool made; };
-SideStream side_streams[MAX_DEVICES] = {};
+struct SideStream {
+    cudaStream_t stream; cudaEvent_t forked, joined; bool made;
+    ~SideStream() {                                           // the thread ends: what it queued still runs, the handles go back
+        if (made) { cudaEventDestroy(forked); cudaEventDestroy(joined); cudaStreamDestroy(stream); }
+    }
+};
+thread_local SideStream side_streams[MAX_DEVICES] = {};
 
 SideStream* side_stream_of_device() {
     SideStream& s = side_streams[device_index()];

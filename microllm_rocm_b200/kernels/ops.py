@@ -644,14 +644,15 @@ def scatter_int(dst: torch.Tensor, dst_index: torch.Tensor, src: torch.Tensor, s
                                      src_index.data_ptr(), dst_index.shape[0], _stream()))
 
 
-_side_streams = {}
+_side_streams = threading.local()           # device -> handle, a stream for each thread
 
 
 def side_stream() -> int:
-    """This device's second stream, for work of a step that is independent of what the main stream does meanwhile
+    """This device's second stream (of this thread), for work of a step that is independent of what the main stream does meanwhile
     (see fork / join)."""
     device = _current_device() if _current_device is not None else torch.cuda.current_device()
-    handle = _side_streams.get(device)
+    handles = _side_streams.__dict__
+    handle = handles.get(device)
     if handle is None:
         L = lib("basic.cu")
         L.mlb_side_stream.restype = c_void_p
@@ -659,7 +660,7 @@ def side_stream() -> int:
         handle = L.mlb_side_stream()
         if not handle:
             raise KernelError("the device's second stream could not be made")
-        _side_streams[device] = handle
+        handles[device] = handle
     return handle
 
 
