@@ -89,3 +89,13 @@ def test_captured_batch_sizes():
         [1, 2, 4, 8, 8, 12, 16, 48, 64, 96, 256, 257, 300]
     assert captured_batch(5, 6) == 6 and captured_batch(6, 6) == 6 and captured_batch(3, 3) == 3      # never more rows than request slots... but never fewer than the requests
     assert list(BATCH_SIZES) == sorted(BATCH_SIZES)
+
+
+@pytest.mark.parametrize("rows, groups, weight_rows, weight_mb, pays", [
+    (12288, 64, 2816, 11, True), (48, 64, 2816, 11, True), (12, 64, 2816, 11, False),      # large experts: from a handful of tokens on
+    (512, 32, 1408, 5.5, True), (496, 32, 1408, 5.5, False),                                # 16 rows a group, a tile for every pair
+    (1024, 16, 1024, 2, False), (1536, 16, 1024, 2, True),                                  # too few tiles for the pairs, until the groups are large
+])
+def test_which_grouped_products_go_to_pairs(rows, groups, weight_rows, weight_mb, pays):
+    from microllm_rocm_b200.kernels import grouped
+    assert grouped.pair_pays(rows, groups, weight_rows, int(weight_mb * (1 << 20)), 148) is pays
