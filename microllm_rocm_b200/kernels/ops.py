@@ -139,9 +139,14 @@ def lagged_sources():
     out = [("attention_tc.cu", {"HEAD_DIM": 128, "MLB_LAG_WARP": w}) for w in (0, 1, 2, 5)]
     out += [("gemm_stream.cu", {"MLB_LAG_WARP": w}) for w in (0, 1, 3)]
     out += [("gemm_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
-    out += [("grouped_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
     out += [("attention_mma.cu", {"HEAD_DIM": 128, "MLB_LAG_WARP": w}) for w in (1, 4)]
     return out
+
+
+def lagged_group_sources():
+    """The same of the grouped product on CTA pairs: a list of its own, since callers look the sources of lagged_sources() up in tables
+    of theirs."""
+    return [("grouped_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
 
 
 def lib(source: str, defines=None) -> ctypes.CDLL:

@@ -557,11 +557,17 @@ def test_kernels_with_barriers_or_rings_give_the_same_bits_beside_a_memory_hog(k
 def held_back_builds():
     from microllm_rocm_b200.kernels import ops as o
     uses = {"attention_tc.cu": ["prompt"], "gemm_stream.cu": ["stream_partials", "stream_many_tiles", "stream_silu"],
-            "gemm_tc2.cu": ["pair", "pair_dual"], "grouped_tc2.cu": ["grouped_pair", "grouped_pair_dual"], "attention_mma.cu": ["decode_ring"]}
+            "gemm_tc2.cu": ["pair", "pair_dual"], "attention_mma.cu": ["decode_ring"]}
     return [(source, tuple(sorted(defines.items())), case) for source, defines in o.lagged_sources() for case in uses[source]]
 
 
-@pytest.mark.parametrize("source,defines,case", held_back_builds())
+def held_back_group_builds():
+    from microllm_rocm_b200.kernels import ops as o
+    return [(source, tuple(sorted(defines.items())), case) for source, defines in o.lagged_group_sources()
+            for case in ("grouped_pair", "grouped_pair_dual")]
+
+
+@pytest.mark.parametrize("source,defines,case", held_back_builds() + held_back_group_builds())
 def test_a_held_back_warp_changes_nothing(source, defines, case):
     """Every kernel whose warps have roles of their own (copy, MMA issue, epilogue or softmax) and meet at mbarriers is
     built once more per role with that role's warp sleeping 3 us at every turn of its loop (-DMLB_LAG_WARP, and

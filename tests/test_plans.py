@@ -99,3 +99,10 @@ def test_captured_batch_sizes():
 def test_which_grouped_products_go_to_pairs(rows, groups, weight_rows, weight_mb, pays):
     from microllm_rocm_b200.kernels import grouped
     assert grouped.pair_pays(rows, groups, weight_rows, int(weight_mb * (1 << 20)), 148) is pays
+
+
+def test_the_held_back_builds_of_the_first_kernels_keep_their_list():
+    """Callers index tables of their own by these sources: a further kernel gets a list beside it."""
+    from microllm_rocm_b200.kernels import ops
+    assert {source for source, _ in ops.lagged_sources()} == {"attention_tc.cu", "gemm_stream.cu", "gemm_tc2.cu", "attention_mma.cu"}
+    assert {source for source, _ in ops.lagged_group_sources()} == {"grouped_tc2.cu"}
