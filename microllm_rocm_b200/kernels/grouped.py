@@ -79,6 +79,7 @@ def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: 
 
 def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_rows, dual, act, row_scale, alloc, error_flag):
     G, w_rows, K = weight.shape
+    out_bf16 = 1 if ops.dtype_tag(out) == ops.BF16 else 0                # (fp32 or bf16: other types are refused, as on the other routes)
     flag = error_flag if error_flag is not None else device_error_flag(a.device)
     L = ops.lib(PAIR_SOURCE)
     source = a
@@ -92,7 +93,7 @@ def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_
     sms = sm_count(a.device)
     build.check(L, L.mlb_grouped_pair(
         source.data_ptr(), source.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0), group_offsets.data_ptr(), ops._ptr(c_rows),
-        ops._ptr(row_scale), ops._ptr(a_rows) if row_scale is not None else None, 1 if out.dtype == torch.bfloat16 else 0, 1 if dual else 0,
+        ops._ptr(row_scale), ops._ptr(a_rows) if row_scale is not None else None, out_bf16, 1 if dual else 0,
         int(act), outputs if dual else 0, int(rows), outputs, K, G, w_rows, cap, sms - sms % 2, flag.data_ptr(), ops._stream()))
 
 

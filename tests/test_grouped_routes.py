@@ -1,0 +1,61 @@
+"""What the grouped products hand to their launchers, on the CPU: the launchers are stand-ins that note their arguments, so a call
+that would write or read out of range on a device shows as an argument."""
+import pytest
+import torch
+
+from microllm_rocm_b200.kernels import grouped, ops
+from microllm_rocm_b200.kernels.build import KernelError
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """[(launcher, {argument name: value})] of the calls made."""
+    import re
+
+    from microllm_rocm_b200.kernels import build
+    made = []
+
+    class Library:
+        def __init__(self, source):
+            text = open(f"{build.CSRC}/{source}").read()
+            self.names = {fn: [p.strip().split()[-1].lstrip("*") for p in params.split(",")]
+                          for fn, params in re.findall(r"MLB_EXPORT\s+int\s+(\w+)\s*\(([^)]*)\)", text, re.S)}
+
+        def __getattr__(self, fn):
+            def launcher(*args):
+                assert len(args) == len(self.names[fn])
+                made.append((fn, dict(zip(self.names[fn], args))))
+                return 0
+            return launcher
+
+    monkeypatch.setattr(ops, "lib", lambda source, defines=None: Library(source))
+    monkeypatch.setattr(ops, "_need", lambda *args, **kwargs: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(grouped, "sm_count", lambda device: 148)
+    return made
+
+
+ROUTES = {"pair": (True, True), "mma": (False, True), "plain": (False, False)}       # USE_PAIRS, USE_TENSOR_CORES
+
+
+def use(monkeypatch, route):
+    pairs, tensor_cores = ROUTES[route]
+    monkeypatch.setattr(grouped, "USE_PAIRS", pairs)
+    monkeypatch.setattr(grouped, "USE_TENSOR_CORES", tensor_cores)
+
+
+def operands(rows=24, G=3, N=32, K=64):
+    a, w = torch.zeros(rows, K, dtype=torch.bfloat16), torch.zeros(G, N, K, dtype=torch.bfloat16)
+    return a, w, torch.tensor([0, 8, 8, rows], dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+
+
+@pytest.mark.parametrize("route", sorted(ROUTES))
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int32, torch.float64])
+def test_outputs_of_other_types_are_refused_on_every_route(calls, monkeypatch, route, dtype):
+    use(monkeypatch, route)
+    a, w, offsets, flag = operands()
+    with pytest.raises(KernelError, match="dtype"):
+        grouped.grouped_linear(a, w, torch.zeros(24, 32, dtype=dtype), rows=24, group_offsets=offsets, error_flag=flag)
+    with pytest.raises(KernelError, match="dtype"):
+        grouped.grouped_silu_mul(a, w, torch.zeros(24, 16, dtype=dtype), rows=24, group_offsets=offsets, error_flag=flag)
+    assert not [fn for fn, _ in calls if fn in ("mlb_grouped_pair", "mlb_grouped_mma", "mlb_gather_rows")]
