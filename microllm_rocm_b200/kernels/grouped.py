@@ -87,6 +87,10 @@ def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_
         source = alloc((rows, K), a.dtype) if alloc is not None else torch.empty((rows, K), dtype=a.dtype, device=a.device)
         build.check(L, L.mlb_gather_rows(a.data_ptr(), a.stride(0), a_rows.data_ptr(), int(a_row_div), group_offsets.data_ptr(), G,
                                          source.data_ptr(), int(rows), K, ops._stream()))
+    # the copies take whole boxes of rows, a tile's last ones with rows of the next group: up to the end of the matrix and no further
+    rows = min(int(rows), source.shape[0])
+    if rows == 0:
+        return
     # one tile for most groups: the mean and a quarter more
     mean = rows / min(G, rows)
     cap = 32 if mean <= 16 else min(256, max(64, -(-int(1.25 * mean) // 64) * 64))
@@ -94,7 +98,7 @@ def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_
     build.check(L, L.mlb_grouped_pair(
         source.data_ptr(), source.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0), group_offsets.data_ptr(), ops._ptr(c_rows),
         ops._ptr(row_scale), ops._ptr(a_rows) if row_scale is not None else None, out_bf16, 1 if dual else 0,
-        int(act), outputs if dual else 0, int(rows), outputs, K, G, w_rows, cap, sms - sms % 2, flag.data_ptr(), ops._stream()))
+        int(act), outputs if dual else 0, rows, outputs, K, G, w_rows, cap, sms - sms % 2, flag.data_ptr(), ops._stream()))
 
 
 def row_tile_for(rows: int, groups: int, listed: bool, tensor_cores: bool) -> int:

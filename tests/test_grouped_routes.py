@@ -59,3 +59,17 @@ def test_outputs_of_other_types_are_refused_on_every_route(calls, monkeypatch, r
     with pytest.raises(KernelError, match="dtype"):
         grouped.grouped_silu_mul(a, w, torch.zeros(24, 16, dtype=dtype), rows=24, group_offsets=offsets, error_flag=flag)
     assert not [fn for fn, _ in calls if fn in ("mlb_grouped_pair", "mlb_grouped_mma", "mlb_gather_rows")]
+
+
+@pytest.mark.parametrize("rows, held", [(64, 24), (24, 24), (20, 24), (0, 24)])
+def test_the_pair_kernel_reads_no_row_behind_the_matrix(calls, monkeypatch, rows, held):
+    """`rows` may be more than the list holds, and than `a` has: the kernel's copies take whole boxes of rows up to the number it is
+    given, so that number stays within the matrix they come from."""
+    use(monkeypatch, "pair")
+    a, w, offsets, flag = operands(held)
+    order = torch.zeros(rows, dtype=torch.int32)
+    grouped.grouped_linear(a, w, torch.zeros(rows, 32), rows=rows, group_offsets=offsets, error_flag=flag)
+    grouped.grouped_silu_mul(a, w, torch.zeros(rows, 16), rows=rows, group_offsets=offsets, error_flag=flag)
+    grouped.grouped_silu_mul(a, w, torch.zeros(rows, 16), rows=rows, group_offsets=offsets, a_rows=order, error_flag=flag)
+    given = [args["M"] for fn, args in calls if fn == "mlb_grouped_pair"]
+    assert given == ([min(rows, held), min(rows, held), rows] if rows else [])          # with a list the rows are gathered first, all of them
