@@ -50,7 +50,7 @@ constexpr int MAX_GROUPS = 1024;
 struct GroupedParams {
     void* out;                 // fp32 or bf16, rows of pitch ldo
     const int* offsets;        // [G + 1]
-    const int* c_rows;         // the row written for a place (null: the place itself)
+    const int* c_rows;         // the row written for a place (null: the place itself; negative: none)
     const float* row_scale;    // dual: both products times row_scale[scale_rows[place]] in front of the activation (null: 1)
     const int* scale_rows;
     int* error_flag;
@@ -335,7 +335,8 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 // lane j: the row that place c + j is written to, and its scale
                 const int place = t.row0 + min(c + lane, t.rows - 1);
                 const int to = p.c_rows ? p.c_rows[place] : place;
-                const float scale = p.row_scale ? p.row_scale[p.scale_rows ? p.scale_rows[place] : place] : 1.0f;
+                const int scaled = p.scale_rows ? p.scale_rows[place] : place;
+                const float scale = p.row_scale && scaled >= 0 ? p.row_scale[scaled] : 1.0f;       // (a negative one: a row of zeros)
                 uint32_t raw[32];
                 if (ok) {
                     tmem_ld32_nowait(lane_addr + (uint32_t)c, raw);
@@ -367,8 +368,9 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const int here = ok && out_col < p.N ? t.rows - c - first_col : 0;      // places of these 16 that exist
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const size_t o = (size_t)__shfl_sync(0xffffffffu, to, first_col + j) * p.ldo + out_col;
-                        if (j < here) {
+                        const int row = __shfl_sync(0xffffffffu, to, first_col + j);
+                        const size_t o = (size_t)row * p.ldo + out_col;
+                        if (j < here && row >= 0) {
                             if (p.out_bf16) ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(g[j]);
                             else ((float*)p.out)[o] = g[j];
                         }
@@ -379,7 +381,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 for (int j = 0; j < 32; ++j) {                         // (plain stores: nothing to set side by side, and no address kept for later)
                     if (c + j >= t.rows) break;                        // (uniform)
                     const int row = __shfl_sync(0xffffffffu, to, j);
-                    if (out_col >= p.N) continue;
+                    if (out_col >= p.N || row < 0) continue;
                     if (p.out_bf16) ((__nv_bfloat16*)p.out)[(size_t)row * p.ldo + out_col] = __float2bfloat16_rn(__uint_as_float(raw[j]));
                     else ((float*)p.out)[(size_t)row * p.ldo + out_col] = __uint_as_float(raw[j]);
                 }
@@ -397,7 +399,8 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
 }
 
-// rows of A in the order of the list: out[place] = A[a_rows[place] / div], 16 bytes a thread
+// rows of A in the order of the list: out[place] = A[a_rows[place] / div], 16 bytes a thread; a negative row is one of zeros, as in
+// grouped_mma.cu
 __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ a, long long lda, const int* __restrict__ a_rows, int div,
                                                           const int* __restrict__ offsets, int G, uint4* __restrict__ out, int rows, int pieces) {
     pdl_prologue();
@@ -405,7 +408,8 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restric
     const long long total = (long long)listed * pieces;
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
         const int place = (int)(i / pieces), piece = (int)(i % pieces);
-        out[i] = a[(size_t)(a_rows[place] / div) * lda + piece];
+        const int row = a_rows[place] / div;
+        out[i] = row >= 0 ? a[(size_t)row * lda + piece] : make_uint4(0u, 0u, 0u, 0u);
     }
 }
 

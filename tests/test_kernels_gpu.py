@@ -210,6 +210,38 @@ def test_grouped_pair_product_over_row_counts(N, K, counts):
     torch.cuda.synchronize()
 
 
+def test_grouped_pair_product_of_rows_that_are_not_there():
+    """A negative row to read is a row of zeros, a negative row to write is not written: on pairs as on mma.sync."""
+    from microllm_rocm_b200.kernels import grouped
+    torch.manual_seed(5)
+    counts, N, K, top = [40, 0, 33, 70], 72, 64, 3
+    rows, G = sum(counts), len(counts)
+    offsets = torch.tensor(np.cumsum([0] + counts), dtype=torch.int32, device=DEV)
+    # small whole numbers: every sum is exact, so both kernels have the same bits
+    a = torch.randint(-2, 3, (rows, K), device=DEV).bfloat16()
+    w = torch.randint(-1, 2, (G, 2 * N, K), device=DEV).bfloat16()
+    c_rows = torch.randperm(rows).to(torch.int32)
+    c_rows[::7] = -1
+    a_rows = torch.randint(0, rows * top, (rows,), dtype=torch.int32)
+    a_rows[3::5] = -top
+    results = []
+    for pairs in (True, False):
+        grouped.USE_PAIRS = pairs
+        try:
+            out = torch.full((rows, 2 * N), -7.0, device=DEV)
+            grouped.grouped_linear(a, w, out, rows=rows, group_offsets=offsets, c_rows=c_rows.to(DEV))
+            act = torch.full((rows, N), -7.0, device=DEV)
+            grouped.grouped_silu_mul(a, w, act, rows=rows, group_offsets=offsets, a_rows=a_rows.to(DEV), a_row_div=top)
+            results.append((out, act))
+        finally:
+            grouped.USE_PAIRS = None
+    (out, act), (out2, act2) = results
+    assert torch.equal(out, out2) and torch.equal(act, act2)
+    kept = set(c_rows.tolist()) - {-1}
+    assert all(bool((out[r] == -7.0).all()) == (r not in kept) for r in range(rows))
+    assert bool((act[3::5] == 0).all()) and not bool((act[4::5] == 0).all())
+
+
 # ------------------------------------------------------------------------------ paged cache helpers
 def paged_from_dense(k, v, page_size, num_pages, dtype, seed=0):
     """k, v: lists (one per sequence) of [n, NKV, D].  Returns pages and a block table with
