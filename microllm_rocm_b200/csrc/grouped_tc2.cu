@@ -457,12 +457,14 @@ MLB_EXPORT int mlb_grouped_pair(const void* a, long long lda, const void* w, voi
     if (K % 8 != 0 || lda % 8 != 0 || lda < K || ((uintptr_t)a & 15) || ((uintptr_t)w & 15))
         return fail(MLB_UNSUPPORTED_SIZE, "grouped_pair: K=%d and the pitch %lld must be multiples of 8, the operands 16-byte aligned", K, lda);
     if (dual && (up_offset < 0 || up_offset + N > w_rows)) return fail(MLB_INVALID_ARGUMENT, "grouped_pair: up rows outside the weight");
+    if (act < 0 || act == 1) return fail(MLB_INVALID_ARGUMENT, "grouped_pair: unknown activation %d", act);
+    if (row_scale && !dual) return fail(MLB_INVALID_ARGUMENT, "grouped_pair: a factor per row goes with the two-block product");
     if (tok_cap != 32 && (tok_cap < 64 || tok_cap > 256 || tok_cap % 64 != 0)) return fail(MLB_INVALID_ARGUMENT, "grouped_pair: tiles of %d rows", tok_cap);
     if ((long long)G * w_rows >= (1ll << 31)) return fail(MLB_UNSUPPORTED_SIZE, "grouped_pair: too many weight rows");
     if (!offsets || sm_count < 2 || sm_count % 2 != 0) return fail(MLB_INVALID_ARGUMENT, "grouped_pair: bad arguments");
     if (M == 0) return MLB_OK;
     GroupedParams p{};
-    p.out = out; p.offsets = offsets; p.c_rows = c_rows; p.row_scale = dual ? row_scale : nullptr; p.scale_rows = scale_rows; p.error_flag = error_flag;
+    p.out = out; p.offsets = offsets; p.c_rows = c_rows; p.row_scale = row_scale; p.scale_rows = scale_rows; p.error_flag = error_flag;
     p.ldo = ldo; p.M = M; p.N = N; p.G = G; p.w_rows = w_rows; p.up_offset = up_offset; p.tok_cap = tok_cap;
     p.k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
     p.n_tiles = (N + (dual ? PAIR_W / 2 : PAIR_W) - 1) / (dual ? PAIR_W / 2 : PAIR_W);

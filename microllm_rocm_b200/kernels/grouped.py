@@ -77,8 +77,10 @@ def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: 
     return rows >= 96 * groups or (rows >= 16 * groups and -(-weight_rows // 256) * active >= sms // 2) or active * weight_bytes >= 200 << 20
 
 
-def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_rows, dual, act, row_scale, alloc, error_flag):
+def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_rows, dual, act, row_scale, row_tile, alloc, error_flag):
     G, w_rows, K = weight.shape
+    if rows < 0 or a_row_div <= 0 or row_tile not in (16, 64, 128):      # (refused by the launchers of the other routes)
+        raise KernelError(f"grouped product: bad sizes, {rows} rows, divisor {a_row_div}, row tile {row_tile}")
     out_bf16 = 1 if ops.dtype_tag(out) == ops.BF16 else 0                # (fp32 or bf16: other types are refused, as on the other routes)
     flag = error_flag if error_flag is not None else device_error_flag(a.device)
     L = ops.lib(PAIR_SOURCE)
@@ -141,8 +143,8 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
         ops._need(row_scale, "row_scale", torch.float32)
     if (group_offsets is not None and a_rows is None and factor is None and row_scale is None and not a_group_cols and not c_group_cols
             and pair_supported(a, weight) and pair_pays(rows, G, N, weight.stride(0) * 2, sm_count(a.device))):
-        _pair(a, weight, out, rows=rows, outputs=N, group_offsets=group_offsets, a_rows=None, a_row_div=1, c_rows=c_rows, dual=False, act=0,
-              row_scale=None, alloc=None, error_flag=error_flag)
+        _pair(a, weight, out, rows=rows, outputs=N, group_offsets=group_offsets, a_rows=None, a_row_div=a_row_div, c_rows=c_rows, dual=False,
+              act=0, row_scale=None, row_tile=row_tile, alloc=None, error_flag=error_flag)
         return
     tensor_cores = mma_supported(a, weight, a_group_cols) and row_scale is None
     if row_tile == 128 and not tensor_cores:
@@ -188,7 +190,7 @@ def grouped_silu_mul(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *
             ops._need(a_rows, "a_rows", torch.int32, 1)
         if pair_supported(a, weight) and pair_pays(rows, G, two_f, weight.stride(0) * 2, sm_count(a.device)):
             _pair(a, weight, out, rows=rows, outputs=F, group_offsets=group_offsets, a_rows=a_rows, a_row_div=a_row_div, c_rows=None, dual=True,
-                  act=ops.activation_code(activation, limit), row_scale=row_scale, alloc=alloc, error_flag=error_flag)
+                  act=ops.activation_code(activation, limit), row_scale=row_scale, row_tile=row_tile, alloc=alloc, error_flag=error_flag)
             return
         L = ops.lib(MMA_SOURCE)
         build.check(L, L.mlb_grouped_mma(

@@ -73,3 +73,30 @@ def test_the_pair_kernel_reads_no_row_behind_the_matrix(calls, monkeypatch, rows
     grouped.grouped_silu_mul(a, w, torch.zeros(rows, 16), rows=rows, group_offsets=offsets, a_rows=order, error_flag=flag)
     given = [args["M"] for fn, args in calls if fn == "mlb_grouped_pair"]
     assert given == ([min(rows, held), min(rows, held), rows] if rows else [])          # with a list the rows are gathered first, all of them
+
+
+def test_the_pair_route_refuses_what_the_others_refuse(calls, monkeypatch):
+    use(monkeypatch, "pair")
+    a, w, offsets, flag = operands()
+    for bad in ({"row_tile": 32}, {"a_row_div": 0}, {"a_row_div": -2}, {"rows": -1}):
+        out = {"rows": 24, "group_offsets": offsets, "error_flag": flag, **bad}
+        with pytest.raises(KernelError):
+            grouped.grouped_linear(a, w, torch.zeros(24, 32), **out)
+        with pytest.raises(KernelError):
+            grouped.grouped_silu_mul(a, w, torch.zeros(24, 16), **out)
+    assert not calls
+
+
+def test_the_pair_launcher_refuses_unknown_activations():
+    """The library itself, which answers before it touches a device."""
+    L = ops.lib(grouped.PAIR_SOURCE)
+    matrix = torch.zeros(64, 64, dtype=torch.bfloat16)
+    list_of = torch.zeros(2, dtype=torch.int32)
+    at = matrix.data_ptr()
+
+    def status(act, dual, row_scale):
+        return L.mlb_grouped_pair(at, 64, at, at, 64, list_of.data_ptr(), None, row_scale, None, 1, dual, act, 16 if dual else 0, 0, 16, 64, 1,
+                                  64, 64, 148, None, 0)
+    assert status(0, 1, None) == 0 and status(0, 0, None) == 0 and status(0x3f400000, 1, at) == 0       # (no rows: nothing to do)
+    for refused in ((1, 1, None), (-1, 1, None), (0, 0, at)):
+        assert status(*refused) != 0
