@@ -337,6 +337,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 const int to = p.c_rows ? p.c_rows[place] : place;
                 const int scaled = p.scale_rows ? p.scale_rows[place] : place;
                 const float scale = p.row_scale && scaled >= 0 ? p.row_scale[scaled] : 1.0f;       // (a negative one: a row of zeros)
+                const unsigned there = __ballot_sync(0xffffffffu, to >= 0);       // (a test of each row behind its shuffle: down 127 us, so 108)
                 uint32_t raw[32];
                 if (ok) {
                     tmem_ld32_nowait(lane_addr + (uint32_t)c, raw);
@@ -370,7 +371,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     for (int j = 0; j < 16; ++j) {
                         const int row = __shfl_sync(0xffffffffu, to, first_col + j);
                         const size_t o = (size_t)row * p.ldo + out_col;
-                        if (j < here && row >= 0) {
+                        if (j < here && ((there >> (first_col + j)) & 1u)) {
                             if (p.out_bf16) ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(g[j]);
                             else ((float*)p.out)[o] = g[j];
                         }
@@ -381,7 +382,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 for (int j = 0; j < 32; ++j) {                         // (plain stores: nothing to set side by side, and no address kept for later)
                     if (c + j >= t.rows) break;                        // (uniform)
                     const int row = __shfl_sync(0xffffffffu, to, j);
-                    if (out_col >= p.N || row < 0) continue;
+                    if (out_col >= p.N || !((there >> j) & 1u)) continue;
                     if (p.out_bf16) ((__nv_bfloat16*)p.out)[(size_t)row * p.ldo + out_col] = __float2bfloat16_rn(__uint_as_float(raw[j]));
                     else ((float*)p.out)[(size_t)row * p.ldo + out_col] = __uint_as_float(raw[j]);
                 }
