@@ -145,26 +145,40 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t addr, uint32_t (&r)[32
 }
 __device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// a / y for y in [1, inf], rounded as a division is, without a branch (the values a thread holds are then divided side by side and
-// not one behind another): the reciprocal refined by one Newton step, the quotient corrected by its remainder (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
+// a / y, rounded as a division is, for y in [1, QUOTIENT_MAX] and |a| <= QUOTIENT_MAX, without a branch (the values a thread holds are
+// then divided side by side and not one behind another): the reciprocal refined by one Newton step, the quotient corrected by its
+// remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  Above 2^126 the
+// reciprocal would be flushed to zero.  Of all fp32 gates within the limits, g / (1 + e^-g) and 1 / (1 + e^(-1.702 g)) have the bits of
+// the division, every one compared on a B200.
+constexpr float QUOTIENT_MAX = 0x1p125f;
 __device__ __forceinline__ float quotient(float a, float y) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-    const float refined = fmaf(r, fmaf(-y, r, 1.0f), r);
-    r = y < INFINITY ? refined : 0.0f;
-    const float q = a * r, corrected = fmaf(fmaf(-y, q, a), r, q);
-    return y < INFINITY && fabsf(q) < INFINITY ? corrected : q;
+    r = fmaf(r, fmaf(-y, r, 1.0f), r);
+    const float q = a * r;
+    return fmaf(-fmaf(y, q, -a), r, q);               // (this sign of the remainder keeps the sign of a zero)
 }
-// act 0: silu(g) * u; larger values are the bits of the clamped form's limit L: g = min(g, L), u = clamp(u, -L, L), g sigmoid(1.702 g) (u + 1)
+// g <- the gated values.  silu(g) * u, or the clamped form with its limit L: g = min(g, L), u = clamp(u, -L, L), g sigmoid(1.702 g) (u + 1);
+// grouped_mma.cu's bits.  A warp with a gate beyond the quotient's range (about -87 and -51, or not finite) divides one by one.
 template <bool CLAMPED>
-__device__ __forceinline__ float gated_value(float g, float u, float limit) {
-    if (CLAMPED) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return g * quotient(1.0f, 1.0f + expf(-1.702f * g)) * (u + 1.0f);
+__device__ __forceinline__ void gated_values(float (&g)[16], const float (&u)[16], float limit) {
+    float y[16];
+    bool near = true;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        if (CLAMPED) g[j] = fminf(g[j], limit);
+        y[j] = 1.0f + expf(CLAMPED ? -1.702f * g[j] : -g[j]);
+        near = near && y[j] <= QUOTIENT_MAX && fabsf(g[j]) <= QUOTIENT_MAX;
     }
-    return quotient(g, 1.0f + expf(-g)) * u;
+    if (__all_sync(0xffffffffu, near)) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) y[j] = quotient(CLAMPED ? 1.0f : g[j], y[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) y[j] = (CLAMPED ? 1.0f : g[j]) / y[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) g[j] = CLAMPED ? g[j] * y[j] * (fminf(fmaxf(u[j], -limit), limit) + 1.0f) : y[j] * u[j];
 }
 
 // The tiles of the list, walked in increasing order by every role of a pair.
@@ -359,13 +373,8 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         g[j] = upper ? theirs : mine;
                         u[j] = upper ? mine : theirs;
                     }
-                    if (p.act > 1) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) g[j] = gated_value<true>(g[j], u[j], __int_as_float(p.act));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) g[j] = gated_value<false>(g[j], u[j], 0.0f);
-                    }
+                    if (p.act > 1) gated_values<true>(g, u, __int_as_float(p.act));
+                    else gated_values<false>(g, u, 0.0f);
                     const int here = ok && out_col < p.N ? t.rows - c - first_col : 0;      // places of these 16 that exist
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {

@@ -242,6 +242,62 @@ def test_grouped_pair_product_of_rows_that_are_not_there():
     assert bool((act[3::5] == 0).all()) and not bool((act[4::5] == 0).all())
 
 
+def both_grouped_routes(run):
+    """The results of `run()` on CTA pairs and on mma.sync."""
+    from microllm_rocm_b200.kernels import grouped
+    out = []
+    for pairs in (True, False):
+        grouped.USE_PAIRS = pairs
+        try:
+            out.append(run())
+        finally:
+            grouped.USE_PAIRS = None
+    return out
+
+
+@pytest.mark.parametrize("activation,limit", [("silu", None), ("clamped_swish", 0.75), ("clamped_swish", 60.0)])
+def test_grouped_pair_activation_has_the_bits_of_a_division(activation, limit):
+    """Gates given as they are (one product of one and the row's scale): far out on both sides, where the exponential's sum passes the
+    largest power of two that has a reciprocal and then the largest number, zeros, subnormal, infinite and not-a-number ones.  They
+    come in order, so that runs of sixteen hold near gates only, far ones only, and both.  The mma.sync kernel divides; fp32 results,
+    compared as bits."""
+    from microllm_rocm_b200.kernels import grouped
+    near = torch.randn(4000)
+    near[1000:1008] = torch.tensor([0.0, -0.0, 1e-45, -1e-45, 1e-38, -1e-38, 1e-30, -1e-30])
+    far = [math.inf, -math.inf, math.nan, 3e38, -3e38, 5e37, -5e37]
+    gates = torch.cat([near, torch.linspace(-130, 130, 60000), torch.linspace(-89, -86, 4000), torch.linspace(-53, -50, 4000), torch.tensor(far)]).to(DEV)
+    rows, K, F = gates.shape[0], 8, 16
+    a, w = torch.zeros(rows, K, device=DEV).bfloat16(), torch.zeros(1, 2 * F, K, device=DEV).bfloat16()
+    a[:, 0] = w[0, :, 0] = 1
+    offsets, order = torch.tensor([0, rows], dtype=torch.int32, device=DEV), torch.arange(rows, dtype=torch.int32, device=DEV)
+
+    def run():
+        out = torch.empty(rows, F, device=DEV)
+        grouped.grouped_silu_mul(a, w, out, rows=rows, group_offsets=offsets, a_rows=order, row_scale=gates, activation=activation, limit=limit,
+                                 row_tile=128)
+        return out
+    pairs, divided = both_grouped_routes(run)
+    other = (pairs.view(torch.int32) != divided.view(torch.int32)) & ~(pairs.isnan() & divided.isnan())
+    assert not bool(other.any()), gates[other[:, 0]][:8].tolist()
+
+
+@pytest.mark.parametrize("G,N,K,rows", [(8, 256, 2048, 1600), (4, 72, 104, 400), (3, 40, 520, 70), (8, 1408, 1024, 600)])
+def test_grouped_pair_products_have_the_bits_of_the_mma_kernel(G, N, K, rows):
+    from microllm_rocm_b200.kernels import grouped
+    torch.manual_seed(rows)
+    a, w = torch.randn(rows, K, device=DEV).bfloat16(), (torch.randn(G, 2 * N, K, device=DEV) * K ** -0.5).bfloat16()
+    counts = torch.bincount(torch.randint(0, G, (rows,)), minlength=G)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]).to(torch.int32).to(DEV)
+
+    def run():
+        out, act = torch.empty(rows, 2 * N, device=DEV), torch.empty(rows, N, dtype=torch.bfloat16, device=DEV)
+        grouped.grouped_linear(a, w, out, rows=rows, group_offsets=offsets)
+        grouped.grouped_silu_mul(a, w, act, rows=rows, group_offsets=offsets)
+        return out, act
+    pairs, mma = both_grouped_routes(run)
+    assert torch.equal(pairs[0], mma[0]) and torch.equal(pairs[1], mma[1])
+
+
 # ------------------------------------------------------------------------------ paged cache helpers
 def paged_from_dense(k, v, page_size, num_pages, dtype, seed=0):
     """k, v: lists (one per sequence) of [n, NKV, D].  Returns pages and a block table with
