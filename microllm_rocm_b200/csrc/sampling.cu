@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS) sample_rows_cluster_kernel(Sa
     __shared__ double s_dbl[32];
     __shared__ int s_int[32];
     __shared__ unsigned s_hist[2][BINS];                     // two: the next one is cleared while this one is filled
-    __shared__ float s_max[CLUSTER * WARPS];
+    __shared__ unsigned s_max[CLUSTER * WARPS];
     __shared__ int s_flag, s_first, s_last, s_digit, s_left;
     __shared__ struct { float best; int index, bad, eighth, equal, first, last; double sum; } meet;
 
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS) sample_rows_cluster_kernel(Sa
     if (p.skip_greedy && (T == 0.0f || k == 1)) return;     // (the whole cluster)
     const int V = p.vocab, from = min(rank * slice, V), count = min(slice, V - from);
     const float* logits = p.logits + (size_t)row * p.ld + from;
-    if (tid == 0) { s_flag = 0; s_first = 0x7fffffff; s_last = -1; }
+    if (tid == 0) { s_flag = 0; s_first = 0x7fffffff; s_last = -1; s_digit = 0; s_left = 0; }
     for (int i = tid; i < BINS; i += CLUSTER_THREADS) s_hist[0][i] = 0u;
     __syncthreads();
     float best = -INFINITY;
@@ -289,15 +289,16 @@ __global__ void __launch_bounds__(CLUSTER_THREADS) sample_rows_cluster_kernel(Sa
     int keep_equal = 0x7fffffff;
     if (k < V) {
         // Nothing below the k-th largest of the warps' maxima (each a logit of its own) can be among the k largest: with few
-        // candidates wanted only a handful of logits is counted below.
+        // candidates wanted only a handful of logits is counted below.  Ranked by the key, as the counting is: -0 and +0 are
+        // equal numbers with different keys, and a floor taken between them as numbers could lie above the k-th largest key.
         unsigned floor_key = 0u;
         if (k <= CLUSTER * WARPS) {
-            if (tid < CLUSTER * WARPS) s_max[tid] = cluster.map_shared_rank(s_val, tid / WARPS)[tid % WARPS];
+            if (tid < CLUSTER * WARPS) s_max[tid] = sortable_key(cluster.map_shared_rank(s_val, tid / WARPS)[tid % WARPS]);
             __syncthreads();
             if (tid < CLUSTER * WARPS) {
                 int larger = 0;
                 for (int j = 0; j < CLUSTER * WARPS; ++j) larger += s_max[j] > s_max[tid] || (s_max[j] == s_max[tid] && j < tid) ? 1 : 0;
-                if (larger == k - 1) s_digit = (int)sortable_key(s_max[tid]);
+                if (larger == k - 1) s_digit = (int)s_max[tid];
             }
             __syncthreads();
             floor_key = (unsigned)s_digit;

@@ -859,6 +859,41 @@ def test_sampling_over_a_clusters_slices_matches_the_plain_sampler(vocab):
     assert out.tolist() == want
 
 
+@pytest.mark.parametrize("vocab", [1000, 16384])
+def test_sampling_among_zeros_of_both_signs(vocab):
+    """The threshold lies among zeros, where the kernels' order (by the key's bits) has -0 below +0: one CTA and a cluster of eight,
+    zeros in one warp's span and in several, few candidates and more than there are warps."""
+    torch.manual_seed(3)
+    rows = []
+    for spots in ([(0, -0.0), (40, 0.0)], [(0, 0.0), (40, -0.0)], [(0, -0.0), (40, 0.0), (400, -0.0), (700, 0.0), (vocab - 1, -0.0)],
+                  [(1, -0.0), (33, 0.0), (34, -0.0)]):
+        x = -torch.rand(vocab) - 1.0
+        for i, v in spots:
+            x[i] = v
+        rows.append(x)
+    rows.append(torch.where(torch.rand(vocab) < 0.5, 0.0, -0.0))
+    rows.append(torch.full((vocab,), -0.0))
+    x = torch.stack(rows)
+
+    def kept_of(row, k):                                  # larger keys first, then the smaller index
+        bits = row.view(torch.int32).long() & 0xffffffff
+        key = torch.where(bits >= 1 << 31, 0xffffffff - bits, bits + (1 << 31))
+        order = sorted(range(vocab), key=lambda i: (-int(key[i]), i))
+        return sorted(order[:k])
+
+    for top_k in ([2, 2, 4, 2, 100, 3], [1, 3, 2, 3, 129, 128], [5, 2, 3, 4, vocab - 1, 1]):
+        kept = [kept_of(row, k) for row, k in zip(x, top_k)]
+        for draw in range(6):
+            out = torch.full((len(rows),), -77, dtype=torch.int32, device=DEV)
+            seeds = [17 + r for r in range(len(rows))]
+            ops().sample_rows(x.to(DEV), torch.full((len(rows),), 0.7, device=DEV), torch.tensor(top_k, dtype=torch.int32).to(DEV),
+                              torch.tensor(seeds).to(DEV), torch.full((len(rows),), draw, dtype=torch.int64, device=DEV), out)
+            for r, token in enumerate(out.tolist()):
+                # the plain sampler over the kept logits alone
+                want = kept[r][plain.sample_token(x[r][kept[r]].numpy(), 0.7, 0, seeds[r], draw)] if top_k[r] != 1 else int(np.argmax(x[r].numpy()))
+                assert token == want, (r, top_k[r], draw)
+
+
 def test_sampling_kernel_follows_the_distribution():
     logits = torch.tensor([[0.0, 1.0, 2.0, 0.5, -1.0]]).repeat(4000, 1)
     out = torch.empty(4000, dtype=torch.int32, device=DEV)
