@@ -14,8 +14,10 @@
 // A sink (one learned number per head) enters the denominator once, with no value.
 // In prompts of many rows a CTA holds GROUPS = 2 such groups of four warps with 16 rows each: they share the ring of keys, which is
 // most of a CTA's shared memory, so that four groups and not two fit a multiprocessor and cover each other's barriers (a
-// tile is a serial path of scores, softmax and values with four of them).  A row's bits stay the same: a tile that only the other
-// group's rows see adds nothing.  2,048 tokens of 16 heads, 512 + 64 wide: 632 us with one group, 426 with two.
+// tile is a serial path of scores, softmax and values with four of them).  A row's bits stay the same, whatever the other group's keys
+// hold: a group takes zeros for the values of keys that none of its own rows sees, as a CTA of one group stages them, and a tile of
+// such keys adds nothing (passing it over costs more in registers than it saves).  2,048 tokens of 16 heads, 512 + 64 wide: 632 us with
+// one group, 434 with two (426 without the zeros), which are held to 128 registers a thread for four groups a multiprocessor and spill 180 bytes (one group: 205).
 // With `splits` > 1 a work item's key tiles are divided among that many CTAs, which leave unnormalised partial
 // outputs with their maximum and sum in a workspace; latent_merge_kernel puts them together (and adds the sink).
 #include "common.cuh"
@@ -57,8 +59,7 @@ __device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], const void* p) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
-__device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], const void* p) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+__device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], unsigned a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
@@ -81,8 +82,12 @@ struct Group {
     float part[4][BM][SP];                // each warp's partial scores of the tile
     float red_max[4][BM];
     float red_sum[4][BM];
+    int lo, span, pad[2];                 // what the group's rows see: keys lo .. lo + span
 };
-template <int STAGES, int GROUPS> constexpr size_t smem_bytes() { return sizeof(Ring<STAGES>) + GROUPS * sizeof(Group); }
+constexpr int ZERO_COLS = WR + 8;         // two groups: the values of a key that one of them does not see (read two n-tiles at a time)
+template <int STAGES, int GROUPS> constexpr size_t smem_bytes() {
+    return sizeof(Ring<STAGES>) + GROUPS * sizeof(Group) + (GROUPS > 1 ? ZERO_COLS * sizeof(__nv_bfloat16) : 0);
+}
 static_assert(sizeof(Ring<2>) % 16 == 0 && sizeof(Group) % 16 == 0, "a group's tiles are read in 16-byte pieces");
 
 template <int STAGES, int GROUPS>
@@ -99,7 +104,7 @@ latent_mma_kernel(Params p) {
     };
     const int seq = p.work[2 * blockIdx.x], cta_row = p.work[2 * blockIdx.x + 1], first_row = cta_row + BM * group;
     const int split = blockIdx.y;
-    const int H = p.heads;
+    const int H = p.heads, splits = GROUPS > 1 ? 1 : p.splits;             // (two groups do not split the keys)
     const int seq_start = p.seq_starts[seq], n_new = p.seq_starts[seq + 1] - seq_start;
     const int pos0 = p.seq_pos0[seq];
     const int cta_rows = min(BM * GROUPS, n_new * H - cta_row);            // rows of this tile that exist,
@@ -110,9 +115,20 @@ latent_mma_kernel(Params p) {
     // what the tile's rows may see: from the first row's lower edge to the last row's own position
     const int pos_first = pos0 + cta_row / H, pos_last = pos0 + (cta_row + cta_rows - 1) / H;
     const int lo_tile = (p.window > 0 && pos_first - p.window + 1 > 0) ? pos_first - p.window + 1 : 0;
+    constexpr unsigned ZEROS = sizeof(Ring<STAGES>) + GROUPS * sizeof(Group);
+    const unsigned smem_base = (unsigned)__cvta_generic_to_shared(smem_raw);
+    if (GROUPS > 1) {
+        // of these keys, what the group's own rows may see (none: no key); read behind the loop's first barrier, as the zeros are
+        if ((tid & 127) == 0) {
+            const int own_first = pos0 + first_row / H;
+            s.lo = rows <= 0 ? 0x3fffffff : (p.window > 0 && own_first - p.window + 1 > 0) ? own_first - p.window + 1 : 0;
+            s.span = rows <= 0 ? 0 : pos0 + (first_row + rows - 1) / H - s.lo;
+        }
+        for (int i = tid; i < ZERO_COLS; i += 128 * GROUPS) reinterpret_cast<__nv_bfloat16*>(smem_raw + ZEROS)[i] = __float2bfloat16_rn(0.0f);
+    }
     const int tile_first = lo_tile / BN, tile_count_all = pos_last / BN - tile_first + 1;
-    const int t_begin = tile_first + (int)((long long)tile_count_all * split / p.splits);
-    const int t_end = tile_first + (int)((long long)tile_count_all * (split + 1) / p.splits);
+    const int t_begin = tile_first + (int)((long long)tile_count_all * split / splits);
+    const int t_end = tile_first + (int)((long long)tile_count_all * (split + 1) / splits);
 
     // Q never touches shared memory: warp w multiplies the 16-wide steps w, w + 4, ... of the contraction for ALL 32 keys
     // of a tile, so it needs only those columns of Q, and keeps them as A fragments for the whole kernel
@@ -168,7 +184,7 @@ latent_mma_kernel(Params p) {
         const bool exists = r < rows;
         row_pos[h] = exists ? pos0 + (first_row + r) / H : -1;             // -1: sees nothing
         row_lo[h] = (p.window > 0 && row_pos[h] - p.window + 1 > 0) ? row_pos[h] - p.window + 1 : 0;
-        const bool own_sink = p.sink != nullptr && p.splits == 1 && exists;
+        const bool own_sink = p.sink != nullptr && splits == 1 && exists;
         m_run[h] = own_sink ? p.sink[(first_row + r) % H] : -INFINITY;
         l_run[h] = own_sink ? 1.0f : 0.0f;
     }
@@ -237,6 +253,15 @@ latent_mma_kernel(Params p) {
             v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
             part_max[h] = v;
         }
+        // Lane l names the place of the values of key l % 16 of each sixteen: a row of zeros for a key that only the other group sees.
+        // (Worked out here, a meeting ahead of its use: beside the loads 12 us more.)
+        unsigned value_row[BN / 16];
+#pragma unroll
+        for (int ks = 0; ks < BN / 16; ++ks) {
+            const int key = ks * 16 + (lane & 15);
+            value_row[ks] = smem_base + (unsigned)(((stage * BN + key) * KP + warp * WR) * 2) + 16 * (lane >> 4);
+            if (GROUPS > 1 && (unsigned)(tile * BN + key - s.lo) > (unsigned)s.span) value_row[ks] = smem_base + ZEROS + 16 * (lane >> 4);
+        }
         if ((lane & 3) == 0) { s.red_max[warp][lane >> 2] = part_max[0]; s.red_max[warp][(lane >> 2) + 8] = part_max[1]; }
         meet();
         float corr[2], part_sum[2];
@@ -271,7 +296,7 @@ latent_mma_kernel(Params p) {
 #pragma unroll
             for (int j = 0; j < NT; j += 2) {
                 unsigned v[4];
-                ldmatrix_x4_trans(v, &ring.k[stage][ks * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][warp * WR + j * 8 + 8 * (lane >> 4)]);
+                ldmatrix_x4_trans(v, value_row[ks] + 16 * j);
                 mma_bf16(acc[j], a, v[0], v[1]);
                 if (j + 1 < NT) mma_bf16(acc[j + 1], a, v[2], v[3]);
             }
@@ -284,7 +309,7 @@ latent_mma_kernel(Params p) {
         const int r = (lane >> 2) + 8 * h;
         if (r >= rows) continue;
         const size_t g = row_base + r;
-        if (p.splits == 1) {
+        if (splits == 1) {
             const float inv = l_run[h] > 0.0f ? 1.0f / l_run[h] : 0.0f;
 #pragma unroll
             for (int j = 0; j < NT; ++j) {

@@ -35,6 +35,7 @@ ROWS_PER_TILE = 16                  # (token, head) rows of one sequence that a 
 KEYS_PER_TILE = 32
 MIN_KEY_TILES_PER_SPLIT = 4         # a CTA that shares a work item's keys streams 128 of them at least
 MAX_SPLITS = 64
+GROUPS = None                       # 1 or 2: tests set the groups of rows a CTA holds (where the keys are not split); None: _plan decides
 USE_TENSOR_CORES = True             # tests set it to False to run the plain kernel on the same inputs
 
 
@@ -69,6 +70,8 @@ def _plan(ctx, heads: int):
     tiles = sum(-(-n // ROWS_PER_TILE) for n in rows)
     splits = key_splits(tiles, ctx.max_seq_len, sms) if ctx.decode_only or tiles <= 32 else 1
     groups = 2 if splits == 1 and not ctx.decode_only and tiles >= 4 * sms else 1
+    if GROUPS is not None and splits == 1:
+        groups = GROUPS
     work = []
     for a in range(ctx.num_seqs):
         pos0 = ctx.seq_pos0_host[a] if ctx.seq_pos0_host else 0

@@ -444,3 +444,106 @@ def test_the_shared_expert_beside_the_router_changes_no_bits():
 
     one, two = run(0), run(32)
     assert all(torch.equal(a, b) for a, b in zip(one, two))
+
+
+# ------------------------------------------------------------------------------- two groups of rows a CTA (latent_mma.cu)
+def latent_step(seqs, heads, rank, rot, window, sink, seed=0, page_size=16):
+    """A step's queries, cache and context.  seqs: (new tokens, tokens in front) each; the cache's pages are shuffled."""
+    from microllm_rocm_b200.parts.base import StepContext
+    g = torch.Generator().manual_seed(seed)
+    width, T = rank + rot, sum(n for n, _ in seqs)
+    q = (torch.randn(T, heads * width, generator=g) * 0.3).bfloat16().to(DEV)
+    blocks = [-(-(n + p) // page_size) for n, p in seqs]
+    order = torch.randperm(sum(blocks) + 3, generator=g)
+    table = torch.full((len(seqs), max(blocks)), -1, dtype=torch.int32)
+    at = 0
+    for a, b in enumerate(blocks):
+        table[a, :b] = order[at:at + b]
+        at += b
+    pages = torch.randn(sum(blocks) + 3, page_size, width, generator=g).bfloat16().to(DEV)
+    starts = [0]
+    for n, _ in seqs:
+        starts.append(starts[-1] + n)
+    on = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    positions = [p + i for n, p in seqs for i in range(n)]
+
+    def context():
+        return StepContext(num_tokens=T, num_seqs=len(seqs), token_ids=on(positions), positions=on(positions),
+                           token_seq=on([a for a, (n, _) in enumerate(seqs) for _ in range(n)]), seq_starts=on(starts), seq_pos0=on([p for _, p in seqs]),
+                           seq_lens=on([n + p for n, p in seqs]), block_tables={}, state_slots=None, logit_rows=None,
+                           error_flag=torch.zeros(1, dtype=torch.int32, device=DEV), seq_starts_host=starts, seq_pos0_host=[p for _, p in seqs],
+                           max_new_tokens=max(n for n, _ in seqs), max_seq_len=max(n + p for n, p in seqs))
+    sinks = torch.randn(heads, generator=g).to(DEV) if sink else None
+
+    def run(groups, pages=pages):
+        from microllm_rocm_b200.kernels import latent
+        ctx, out = context(), torch.full((T, heads * rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+        latent.GROUPS = groups
+        try:
+            latent.attention(q, pages, out, sinks, ctx, table.to(DEV), heads, rank, rot, width ** -0.5, window)
+        finally:
+            latent.GROUPS = None
+        assert int(ctx.error_flag.item()) == 0
+        assert groups is None or next(iter(ctx.extras.values()))[3] == groups
+        return out
+
+    def want():
+        """In float64, with the largest value a row of the result may be made of."""
+        out, most = torch.empty(T, heads, rank, dtype=torch.float64, device=DEV), torch.empty(T, 1, 1, dtype=torch.float64, device=DEV)
+        for a, (n, p) in enumerate(seqs):
+            keys = pages.double()[table[a, :blocks[a]].long().to(DEV)].reshape(-1, width)[:n + p]
+            query = q.double()[starts[a]:starts[a + 1]].view(n, heads, width)
+            scores = torch.einsum("nhw,kw->nhk", query, keys) * width ** -0.5
+            i, k = torch.arange(p, p + n, device=DEV)[:, None], torch.arange(n + p, device=DEV)[None]
+            seen = (k <= i) & (k > i - (window or 1 << 30))
+            scores = scores.masked_fill(~seen[:, None, :], -math.inf)
+            if sinks is not None:
+                scores = torch.cat([scores, sinks.double()[None, :, None].expand(n, -1, 1)], -1)
+            weights = torch.softmax(scores, -1)[..., :n + p]
+            out[starts[a]:starts[a + 1]] = weights @ keys[:, :rank]
+            most[starts[a]:starts[a + 1]] = keys[:, :rank].abs().max()
+        return out.reshape(T, -1), most.reshape(T, 1)
+    return run, want, pages, table
+
+
+# new tokens and tokens in front: 31, 30, 32, 17, 1 and 16 rows in the last pair of groups, a second group without rows, later portions
+GROUP_STEPS = {16: [(2, 0), (41, 0), (70, 33), (1, 5)], 5: [(19, 0), (38, 3), (13, 100), (3, 64), (45, 31)], 3: [(11, 7), (53, 0), (75, 40)],
+               40: [(4, 0), (9, 60)], 31: [(1, 0), (33, 90)]}
+
+
+@pytest.mark.parametrize("heads", sorted(GROUP_STEPS))
+@pytest.mark.parametrize("window, sink, rank, rot", [(None, False, 256, 32), (None, True, 512, 64), (7, True, 256, 32), (40, False, 512, 64), (33, True, 256, 32)])
+def test_two_groups_of_latent_rows_give_the_bits_of_one(heads, window, sink, rank, rot):
+    """A row's bits do not follow which rows share its CTA; both against float64."""
+    run, want, _, _ = latent_step(GROUP_STEPS[heads], heads, rank, rot, window, sink, seed=heads)
+    one, two = run(1), run(2)
+    assert torch.equal(one, two)
+    ref, most = want()
+    # weights are rounded to bf16 (and their sum is of the unrounded ones), the result too: half an ulp each, of the largest value
+    # at most; fp32 sums besides
+    assert bool(((one.double() - ref).abs() <= 2 ** -7.9 * most).all()), float(((one.double() - ref).abs() / most).max())
+
+
+@pytest.mark.parametrize("window", [None, 20])
+def test_keys_that_only_the_other_group_sees_do_not_reach_a_row(window):
+    """Cache rows that are not finite: what a row does not see does not touch it.  16 heads, so that a group is one token's."""
+    heads, rank, rot = 16, 256, 32
+    seqs = [(64, 0), (37, 50)]
+    run, _, pages, table = latent_step(seqs, heads, rank, rot, window, True)
+    clean = run(2)
+    for a, position in ((0, 1), (0, 32), (0, 63), (1, 51), (1, 86), (1, 31)):
+        spoiled = pages.clone()
+        spoiled[int(table[a, position // 16]), position % 16] = float("nan")
+        one, two = run(1, spoiled), run(2, spoiled)
+        assert torch.equal(one.view(torch.int16), two.view(torch.int16)), (a, position)
+        start, (n, p) = (0, 64)[a], seqs[a]
+        for i in range(n):
+            sees = p + i >= position and (window is None or p + i - window < position)
+            assert bool(torch.isnan(two[start + i].float()).any()) == sees, (a, position, i)
+            if not sees:
+                assert torch.equal(two[start + i], clean[start + i])
+
+
+def test_a_step_of_many_latent_rows_holds_two_groups_a_cta():
+    run, want, _, _ = latent_step([(640, 0), (33, 7)], 16, 256, 32, None, True)
+    assert torch.equal(run(None), run(2)) and torch.equal(run(1), run(2))
