@@ -686,13 +686,17 @@ def on_side_stream():
     """This library's launches inside go to the device's second stream, which continues from where the current one stands; the
     caller joins (`join(side)`, side being what this yields) before anything reads what they write, and lets go of none of their
     tensors before that.  Only for work that launches kernels of this library and nothing through the tensor framework."""
-    side = side_stream()
+    side, outer = side_stream(), getattr(_launch_on, "side", None)
     fork(side)
     _launch_on.side = side
     try:
         yield side
+    except BaseException:
+        _launch_on.side = outer
+        join(side)                                   # whoever catches this lets go of the tensors, and may be capturing
+        raise
     finally:
-        _launch_on.side = None
+        _launch_on.side = outer
 
 
 def stream_synchronize() -> None:
