@@ -547,3 +547,125 @@ def test_keys_that_only_the_other_group_sees_do_not_reach_a_row(window):
 def test_a_step_of_many_latent_rows_holds_two_groups_a_cta():
     run, want, _, _ = latent_step([(640, 0), (33, 7)], 16, 256, 32, None, True)
     assert torch.equal(run(None), run(2)) and torch.equal(run(1), run(2))
+
+
+# ---------------------------------------------------------------------- rows in registers, and partial results asked for together
+@pytest.mark.parametrize("width", [1, 255, 256, 257, 1023, 1024, 1025, 2047, 2048, 2049, 3000])
+@pytest.mark.parametrize("partials, scaled, out_dtype", [(1, True, torch.float32), (2, False, torch.bfloat16), (3, True, torch.bfloat16),
+                                                         (4, True, torch.float32), (5, False, torch.float32), (8, True, torch.float32)])
+def test_scaled_add_norm_over_widths_and_partial_results(width, partials, scaled, out_dtype):
+    """Four columns a thread, eight, and any number; whole and partial rounds of three further partial results."""
+    from microllm_rocm_b200.kernels import ops
+    torch.manual_seed(width * 10 + partials)
+    rows, eps = 5, 1e-5
+    x, delta = torch.randn(rows, width, device=DEV), torch.randn(partials, rows, width, device=DEV)
+    scale = torch.randn(width, device=DEV) if scaled else None
+    weight = torch.randn(width, device=DEV)
+    d = delta[0].clone()                                  # the order of additions: one partial result after the other
+    for k in range(1, partials):
+        d += delta[k]
+    want_x = x.double() + d.double() * (scale.double() if scaled else 1.0)
+    res, out = x.clone(), torch.empty(rows, width, dtype=out_dtype, device=DEV)
+    ops.add_scaled_rmsnorm(res, delta if partials > 1 else delta[0], scale, weight, eps, out)
+    # fp32 sums in that order are exact here; then one fused multiply-add: half an ulp of the result
+    assert bool(((res.double() - want_x).abs() <= 2 ** -24 * want_x.abs() * 1.0001 + 1e-38).all())
+    want = plain.rms(res.double(), eps) * weight.double()
+    # the sum of squares (a few dozen additions a thread and across threads), root, quotient and two products: well within 16 ulps
+    rel = 2 ** -8 if out_dtype == torch.bfloat16 else 16 * 2 ** -24
+    assert bool(((out.double() - want).abs() <= rel * want.abs() + 1e-30).all()), float(((out.double() - want).abs() / want.abs()).max())
+
+
+@pytest.mark.parametrize("experts", [1, 31, 32, 127, 128, 129, 200, 256])
+@pytest.mark.parametrize("partials, gated", [(1, True), (1, False), (4, True), (5, True), (6, False)])
+def test_router_choice_over_numbers_of_experts_and_partial_results(experts, partials, gated):
+    """The gate's column travels with the logits, four columns a lane and four partial results at a time: on both sides of a lane's
+    and of a round's end."""
+    from microllm_rocm_b200.kernels import moe
+    torch.manual_seed(experts + partials)
+    T, top = 7, min(6, experts)
+    gate_col = experts + 2 if gated else -1               # (with padding in front of it)
+    logits = torch.randn(partials, T, experts + 5, device=DEV)
+    bias = torch.randn(experts, device=DEV)
+    ids, weights = torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    gate = torch.full((T,), -9.0, device=DEV) if gated else None
+    moe.select(logits if partials > 1 else logits[0], experts, bias, top, ids, weights, gate_col, gate)
+    z = logits[0].clone()
+    for k in range(1, partials):                          # the order of additions
+        z += logits[k]
+    chosen = torch.topk(z[:, :experts] + bias, top, dim=-1)
+    assert torch.equal(ids.long(), chosen.indices)
+    # softmax of numbers of a few units: exponential, sum of six and a quotient
+    assert torch.allclose(weights.double(), torch.softmax(chosen.values.double(), -1), rtol=2e-6, atol=0)
+    if gated:
+        assert torch.allclose(gate.double(), torch.sigmoid(z[:, gate_col].double()), rtol=1e-6, atol=0)
+
+
+def test_the_second_stream_is_used_up_to_its_limit_and_not_beyond(monkeypatch):
+    """What test_the_shared_expert_beside_the_router_changes_no_bits compares are two ways and not one twice."""
+    import copy
+    import contextlib
+
+    from microllm_rocm_b200.config.gedalix import PRESETS, GedalixConfig
+    from microllm_rocm_b200.engine.loading import random_engine
+    from microllm_rocm_b200.engine.step import StepEntry
+    from microllm_rocm_b200.kernels import ops
+    from microllm_rocm_b200.parts import routed
+    raw = copy.deepcopy(PRESETS["gedalix-small"])
+    raw["layers"], raw["max_positions"] = raw["layers"][:3], 256
+    engine = random_engine(GedalixConfig.from_dict(raw), seed=3, max_tokens=1024, max_requests=64, draw_on_device=True)
+    engine.model.replay_layers = False                    # (a recorded layer is issued again without this function)
+    entered, real = [], ops.on_side_stream
+
+    @contextlib.contextmanager
+    def counted():
+        entered.append(ops._stream())
+        with real() as side:
+            yield side
+    monkeypatch.setattr(ops, "on_side_stream", counted)
+    routed_layers = sum(isinstance(b.feed_forward, routed.RoutedExperts) for b in engine.model.blocks)
+    assert routed_layers > 0
+    for tokens, limit, uses in ((1, 32, True), (8, 32, True), (32, 32, True), (33, 32, False), (8, 0, False), (8, 8, True), (9, 8, False)):
+        monkeypatch.setattr(routed, "SIDE_MAX_TOKENS", limit)
+        entered.clear()
+        ids = [f"{tokens}.{limit}.{i}" for i in range(tokens)]
+        for rid in ids:
+            engine.cache.add(rid)
+        engine.step([StepEntry(rid, [5 + i], [0]) for i, rid in enumerate(ids)])
+        for rid in ids:
+            engine.cache.release(rid)
+        assert bool(entered) == uses and (not uses or len(entered) >= routed_layers), (tokens, limit, entered)
+    engine.check_device_errors()
+
+
+def test_every_host_thread_has_a_second_stream_of_its_own():
+    """Two threads fork, launch and join side by side, each on its own stream and events."""
+    import threading
+
+    from microllm_rocm_b200.kernels import ops
+    n, failures, handles = 1 << 20, [], {}
+    barrier = threading.Barrier(2)
+
+    def work(name):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                x, one = torch.zeros(n, device=DEV), torch.ones(n, device=DEV)
+                handles[name] = ops.side_stream()
+                barrier.wait(timeout=30)
+                for i in range(50):
+                    with ops.on_side_stream() as side:
+                        assert side == handles[name] and ops._stream() == side
+                        ops.add_inplace(x, one)
+                    ops.join(side)
+                    ops.add_inplace(x, one)               # behind the join: on the thread's own stream
+                stream.synchronize()
+                assert bool((x == 100).all())
+        except BaseException as e:                        # noqa: BLE001  (reported by the test's thread)
+            failures.append((name, repr(e)))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+    assert len(set(handles.values())) == 2 and ops.side_stream() not in handles.values()
