@@ -16,6 +16,8 @@
 //
 //   paged_attention_rows_kernel    head sizes that are multiples of 4 (beyond 128: of 8)
 //   paged_attention_plain_kernel   the others, whose rows have no such pieces: a warp per (token, head)
+#include <type_traits>
+
 #include "common.cuh"
 
 using namespace mlb;
@@ -122,15 +124,17 @@ paged_attention_plain_kernel(AttnParams p) {
 }
 
 // A CTA per query token and up to R query heads of one kv head, which share every key and value read.  Tile t of 32 keys
-// belongs to warp t % ROW_WARPS, so that one decoded token's keys are read from many places at once; each warp keeps its own
-// running maximum, sum and accumulator per row, and they meet in the order of the warps at the end.  Scores: eight lanes a key,
+// belongs to share t % SHARES, so that one decoded token's keys are read from many places at once; each share has its own
+// running maximum, sum and accumulator per row, and they meet in the order of the shares at the end.  Scores: eight lanes a key,
 // 16 bytes each, so that a warp's load takes whole 128-byte lines of four keys (a lane per key would touch 32 lines, and
-// did: 390 us for two decoded tokens of 12 heads behind 300 keys, 730 us for a prompt of 333; now 14 and 77); a lane
+// did: 390 us for two decoded tokens of 12 heads behind 300 keys, 730 us for a prompt of 333; now 14 and 67); a lane
 // works on eight keys beside one another, and seven shuffles a row leave lane l with the score of key l.  Values: a lane per
-// VW neighbouring columns, VW * 32 >= head size.  What a row's bits are does not depend on R: few rows (two CTAs an SM at
-// most) get a CTA each, which then waits for memory only, so more of a tile is asked for at once (six heads together: 35 us
-// for the two decoded tokens).
-constexpr int ROW_WARPS = 8;
+// VW neighbouring columns, VW * 32 >= head size.
+// What a row's bits are depends neither on R nor on how many of the CTA's WIDE warps share the work: a warp takes one share after
+// the other.  Few rows (R 1, WIDE 8): a CTA a head, which waits for memory only, so all of a tile is asked for at once
+// (FEW; six heads together: 35 us for the two decoded tokens).  Many rows fill the device with four warps each; eight would mostly
+// idle where the keys are few (launch_rows has the measurements).
+constexpr int SHARES = 8;
 
 template <typename KVT> __device__ __forceinline__ float4 load4(const KVT* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -151,17 +155,17 @@ template <typename KVT, int VW> __device__ __forceinline__ void load_columns(con
     }
 }
 
-template <typename KVT, int VW, int R>
-__global__ void __launch_bounds__(ROW_WARPS * 32)
+template <typename KVT, int VW, int R, int WIDE, bool FEW>
+__global__ void __launch_bounds__(WIDE * 32)
 paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) {
     pdl_prologue();
     extern __shared__ __align__(16) float shared[];
     const int D = p.head_dim;
     float* q_s = shared;                                       // [R][D]
-    float* acc_s = q_s + R * D;                                // [ROW_WARPS][R][D]
-    float* m_s = acc_s + ROW_WARPS * R * D;                    // [ROW_WARPS][R]
-    float* l_s = m_s + ROW_WARPS * R;
-    float* p_s = l_s + ROW_WARPS * R + (threadIdx.x >> 5) * (R * 32);        // this warp's probabilities of a tile
+    float* acc_s = q_s + R * D;                                // [SHARES][R][D]
+    float* m_s = acc_s + SHARES * R * D;                       // [SHARES][R]
+    float* l_s = m_s + SHARES * R;
+    float* p_s = l_s + SHARES * R + (threadIdx.x >> 5) * (R * 32);        // this warp's probabilities of a tile
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.num_heads / p.num_kv_heads;
     const int chunk = blockIdx.x % chunks, kvh = (blockIdx.x / chunks) % p.num_kv_heads, t = blockIdx.x / (chunks * p.num_kv_heads);
@@ -169,17 +173,10 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
     const int pos = p.positions[t], seq = p.token_seq[t];
     const int lo = first_visible_key(pos, p.window, p.chunk);
     const size_t q_at = ((size_t)t * p.num_heads + h0) * D;
-    for (int e = tid; e < R * D; e += ROW_WARPS * 32)
+    for (int e = tid; e < R * D; e += WIDE * 32)
         q_s[e] = e >= rows * D ? 0.0f : q_bf16 ? to_f32(((const __nv_bfloat16*)p.q)[q_at + e]) : ((const float*)p.q)[q_at + e];
     __syncthreads();
 
-    float acc[R][VW], m[R], l[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        m[r] = -INFINITY; l[r] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < VW; ++i) acc[r][i] = 0.0f;
-    }
     const size_t page_stride = (size_t)2 * p.num_kv_heads * p.page_size * D;
     const size_t v_offset = (size_t)p.num_kv_heads * p.page_size * D;
     const int* table = p.block_table + (size_t)seq * p.max_blocks;
@@ -188,138 +185,147 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
     const bool column = lane * VW < D;
 
     const int first = lo / 32, last = pos / 32;
-    for (int tile = first + (warp - first % ROW_WARPS + ROW_WARPS) % ROW_WARPS; tile <= last; tile += ROW_WARPS) {
-        const int kp = tile * 32 + lane;
-        bool valid = kp >= lo && kp <= pos;
-        long long k_off = 0;                                   // (a key that is not visible is read from the pool's first row)
-        if (valid) {
-            const int block = kp / p.page_size;
-            const int page = block < p.max_blocks ? table[block] : -1;
-            if (page < 0 || page >= p.num_pages) {
-                if (p.error_flag) atomicExch(p.error_flag, 2);
-                valid = false;
-            } else {
-                k_off = (long long)((size_t)page * page_stride + ((size_t)kvh * p.page_size + kp % p.page_size) * D);
-            }
-        }
-        float dot[R][8];
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) dot[r][j] = 0.0f;
-        long long key_at[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) key_at[j] = __shfl_sync(0xffffffffu, k_off, key_group * 8 + j);
-        if (R == 1 && valid) {                                 // this lane's key and value, all lines of them
-            const char* row = (const char*)(pages + k_off);
-            for (int b = 0; b < D * (int)sizeof(KVT); b += 128) {
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(row + v_offset * sizeof(KVT) + b));
-            }
-        }
-        if (R == 1 && pieces <= 32) {                          // all of the lane's pieces of its eight keys at once
-            float4 k[4][8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (c + 8 * i < pieces) k[i][j] = load4(pages + key_at[j] + (c + 8 * i) * 4);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (c + 8 * i < pieces) {
-                    const float4 q = *reinterpret_cast<const float4*>(q_s + (c + 8 * i) * 4);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        dot[0][j] = fmaf(q.w, k[i][j].w, fmaf(q.z, k[i][j].z, fmaf(q.y, k[i][j].y, fmaf(q.x, k[i][j].x, dot[0][j]))));
-                }
-        } else {
-            for (int piece = c; piece < pieces; piece += 8) {
-                float4 k[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) k[j] = load4(pages + key_at[j] + piece * 4);
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float4 q = *reinterpret_cast<const float4*>(q_s + r * D + piece * 4);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) dot[r][j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, fmaf(q.x, k[j].x, dot[r][j]))));
-                }
-            }
-        }
-        __syncwarp();                                          // every lane is done with the last tile's probabilities
+    for (int share = warp; share < SHARES; share += WIDE) {
+        float acc[R][VW], m[R], l[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            // lane c of a key group ends up with the sum over the group's lanes of dot[r][c]
-            float a4[4], a2[2];
+            m[r] = -INFINITY; l[r] = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float keep = c & 4 ? dot[r][j + 4] : dot[r][j], give = c & 4 ? dot[r][j] : dot[r][j + 4];
-                a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const float keep = c & 2 ? a4[j + 2] : a4[j], give = c & 2 ? a4[j] : a4[j + 2];
-                a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
-            }
-            const float keep = c & 1 ? a2[1] : a2[0], give = c & 1 ? a2[0] : a2[1];
-            const float full = keep + __shfl_xor_sync(0xffffffffu, give, 1);
-            const float s = valid ? full * p.scale : -INFINITY;
-            const float m_new = fmaxf(m[r], warp_max(s));
-            float prob = 0.0f;
-            if (m_new != -INFINITY) {                          // else: no readable key in this tile yet
-                prob = valid ? expf(s - m_new) : 0.0f;
-                const float corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
-                l[r] = l[r] * corr + warp_sum(prob);
-                m[r] = m_new;
-#pragma unroll
-                for (int i = 0; i < VW; ++i) acc[r][i] *= corr;
-            }
-            p_s[r * 32 + lane] = prob;
+            for (int i = 0; i < VW; ++i) acc[r][i] = 0.0f;
         }
-        __syncwarp();
-        const unsigned seen = __ballot_sync(0xffffffffu, valid);
-        constexpr int BATCH = R == 1 ? 16 : 4;                 // keys whose values are asked for together
-#pragma unroll (R == 1 ? 1 : 2)
-        for (int j0 = 0; j0 < 32; j0 += BATCH) {
-            float v[BATCH][VW];
-#pragma unroll
-            for (int j = 0; j < BATCH; ++j) {
-                const long long at = __shfl_sync(0xffffffffu, k_off, j0 + j);
-                if (column && ((seen >> (j0 + j)) & 1u)) {
-                    load_columns<KVT, VW>(pages + at + v_offset + lane * VW, v[j]);
+        for (int tile = first + (share - first % SHARES + SHARES) % SHARES; tile <= last; tile += SHARES) {
+            const int kp = tile * 32 + lane;
+            bool valid = kp >= lo && kp <= pos;
+            long long k_off = 0;                                   // (a key that is not visible is read from the pool's first row)
+            if (valid) {
+                const int block = kp / p.page_size;
+                const int page = block < p.max_blocks ? table[block] : -1;
+                if (page < 0 || page >= p.num_pages) {
+                    if (p.error_flag) atomicExch(p.error_flag, 2);
+                    valid = false;
                 } else {
-#pragma unroll
-                    for (int i = 0; i < VW; ++i) v[j][i] = 0.0f;
+                    k_off = (long long)((size_t)page * page_stride + ((size_t)kvh * p.page_size + kp % p.page_size) * D);
                 }
             }
+            float dot[R][8];
 #pragma unroll
-            for (int b = 0; b < BATCH; b += 4) {
+            for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float4 w = *reinterpret_cast<const float4*>(p_s + r * 32 + j0 + b);
+                for (int j = 0; j < 8; ++j) dot[r][j] = 0.0f;
+            long long key_at[8];
 #pragma unroll
-                    for (int i = 0; i < VW; ++i)
-                        acc[r][i] = fmaf(w.w, v[b + 3][i], fmaf(w.z, v[b + 2][i], fmaf(w.y, v[b + 1][i], fmaf(w.x, v[b][i], acc[r][i]))));
+            for (int j = 0; j < 8; ++j) key_at[j] = __shfl_sync(0xffffffffu, k_off, key_group * 8 + j);
+            if (FEW && valid) {                                    // this lane's key and value, all lines of them
+                const char* row = (const char*)(pages + k_off);
+                for (int b = 0; b < D * (int)sizeof(KVT); b += 128) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(row + v_offset * sizeof(KVT) + b));
+                }
+            }
+            if (FEW && pieces <= 32) {                             // all of the lane's pieces of its eight keys at once
+                float4 k[4][8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (c + 8 * i < pieces) k[i][j] = load4(pages + key_at[j] + (c + 8 * i) * 4);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (c + 8 * i < pieces) {
+                        const float4 q = *reinterpret_cast<const float4*>(q_s + (c + 8 * i) * 4);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            dot[0][j] = fmaf(q.w, k[i][j].w, fmaf(q.z, k[i][j].z, fmaf(q.y, k[i][j].y, fmaf(q.x, k[i][j].x, dot[0][j]))));
+                    }
+            } else {
+                for (int piece = c; piece < pieces; piece += 8) {
+                    float4 k[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) k[j] = load4(pages + key_at[j] + piece * 4);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float4 q = *reinterpret_cast<const float4*>(q_s + r * D + piece * 4);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) dot[r][j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, fmaf(q.x, k[j].x, dot[r][j]))));
+                    }
+                }
+            }
+            __syncwarp();                                          // every lane is done with the last tile's probabilities
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                // lane c of a key group ends up with the sum over the group's lanes of dot[r][c]
+                float a4[4], a2[2];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float keep = c & 4 ? dot[r][j + 4] : dot[r][j], give = c & 4 ? dot[r][j] : dot[r][j + 4];
+                    a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float keep = c & 2 ? a4[j + 2] : a4[j], give = c & 2 ? a4[j] : a4[j + 2];
+                    a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+                }
+                const float keep = c & 1 ? a2[1] : a2[0], give = c & 1 ? a2[0] : a2[1];
+                const float full = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+                const float s = valid ? full * p.scale : -INFINITY;
+                const float m_new = fmaxf(m[r], warp_max(s));
+                float prob = 0.0f;
+                if (m_new != -INFINITY) {                          // else: no readable key in this tile yet
+                    prob = valid ? expf(s - m_new) : 0.0f;
+                    const float corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
+                    l[r] = l[r] * corr + warp_sum(prob);
+                    m[r] = m_new;
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) acc[r][i] *= corr;
+                }
+                p_s[r * 32 + lane] = prob;
+            }
+            __syncwarp();
+            const unsigned seen = __ballot_sync(0xffffffffu, valid);
+            constexpr int BATCH = FEW ? 16 : 4;                    // keys whose values are asked for together
+#pragma unroll (FEW ? 1 : 2)
+            for (int j0 = 0; j0 < 32; j0 += BATCH) {
+                float v[BATCH][VW];
+#pragma unroll
+                for (int j = 0; j < BATCH; ++j) {
+                    const long long at = __shfl_sync(0xffffffffu, k_off, j0 + j);
+                    if (column && ((seen >> (j0 + j)) & 1u)) {
+                        load_columns<KVT, VW>(pages + at + v_offset + lane * VW, v[j]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < VW; ++i) v[j][i] = 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int b = 0; b < BATCH; b += 4) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float4 w = *reinterpret_cast<const float4*>(p_s + r * 32 + j0 + b);
+#pragma unroll
+                        for (int i = 0; i < VW; ++i)
+                            acc[r][i] = fmaf(w.w, v[b + 3][i], fmaf(w.z, v[b + 2][i], fmaf(w.y, v[b + 1][i], fmaf(w.x, v[b][i], acc[r][i]))));
+                    }
                 }
             }
         }
-    }
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if (column) {
+        for (int r = 0; r < R; ++r) {
+            if (column && m[r] != -INFINITY) {                     // (a share without keys is not read)
 #pragma unroll
-            for (int i = 0; i < VW; ++i) acc_s[(warp * R + r) * D + lane * VW + i] = acc[r][i];
+                for (int i = 0; i < VW; ++i) acc_s[(share * R + r) * D + lane * VW + i] = acc[r][i];
+            }
+            if (lane == 0) { m_s[share * R + r] = m[r]; l_s[share * R + r] = l[r]; }
         }
-        if (lane == 0) { m_s[warp * R + r] = m[r]; l_s[warp * R + r] = l[r]; }
     }
     __syncthreads();
-    for (int e = tid; e < rows * D; e += ROW_WARPS * 32) {
+    for (int e = tid; e < rows * D; e += WIDE * 32) {
         const int r = e / D;
         float top = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < ROW_WARPS; ++w) top = fmaxf(top, m_s[w * R + r]);
+        for (int w = 0; w < SHARES; ++w) top = fmaxf(top, m_s[w * R + r]);
         float sum = 0.0f, value = 0.0f;
 #pragma unroll
-        for (int w = 0; w < ROW_WARPS; ++w) {
+        for (int w = 0; w < SHARES; ++w) {
             const float mw = m_s[w * R + r];
             if (mw == -INFINITY) continue;
             const float f = expf(mw - top);
@@ -332,12 +338,12 @@ paged_attention_rows_kernel(AttnParams p, int q_bf16, int out_bf16, int chunks) 
     }
 }
 
-template <typename KVT, int VW, int R>
+template <typename KVT, int VW, int R, int WIDE, bool FEW>
 int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stream) {
     static bool done[MAX_DEVICES] = {};
-    auto kernel = paged_attention_rows_kernel<KVT, VW, R>;
+    auto kernel = paged_attention_rows_kernel<KVT, VW, R, WIDE, FEW>;
     const int d = device_index();
-    constexpr int most = (R * VW * 32 * (ROW_WARPS + 1) + 2 * ROW_WARPS * R + ROW_WARPS * R * 32) * 4;
+    constexpr int most = (R * VW * 32 * (SHARES + 1) + 2 * SHARES * R + WIDE * R * 32) * 4;
     if (!done[d]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return check_launch("paged_attention_rows: shared memory");
         done[d] = true;
@@ -345,20 +351,42 @@ int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stre
     const int group = p.num_heads / p.num_kv_heads, chunks = (group + R - 1) / R;
     const long long blocks = (long long)p.tokens * p.num_kv_heads * chunks;
     if (blocks > 0x7fffffffll) return fail(MLB_UNSUPPORTED_SIZE, "paged_attention_plain: %d tokens are more than one launch takes", p.tokens);
-    const size_t smem = (size_t)(R * p.head_dim * (ROW_WARPS + 1) + 2 * ROW_WARPS * R + ROW_WARPS * R * 32) * 4;
-    launch_kernel(kernel, (unsigned)blocks, ROW_WARPS * 32, smem, stream, p, q_bf16, out_bf16, chunks);
+    const size_t smem = (size_t)(R * p.head_dim * (SHARES + 1) + 2 * SHARES * R + WIDE * R * 32) * 4;
+    launch_kernel(kernel, (unsigned)blocks, WIDE * 32, smem, stream, p, q_bf16, out_bf16, chunks);
     return check_launch("paged_attention_rows");
+}
+
+// Heads of a kv head together (at most four at head size 256, whose accumulators are long); one where there are few rows.
+// Four warps a CTA instead of eight where the CTAs are many, two where besides no row has more than two tiles (the table's width).
+// Measured on 148 SMs, us, fp32; heads / kv heads x head size, tokens of a prompt or (sequences x keys), eight warps -> four (-> two):
+// 12/2x128: 64 11.9 -> 12.6, 333 73 -> 67, 300 x 20 49 -> 32 -> 30; 8/2x256: 333 75 -> 53; 14/2x64: 333 59 -> 53.  One head a kv head, where
+// eight warps ask for all of a tile at once: 16/16x128: 30 x 300 63 -> 81, 64 34 -> 13, 333 243 -> 121, 300 x 20 203 -> 117 -> 74, 300 x 300
+// 465 -> 428; 4/4x256: 333 105 -> 72, 300 x 300 226 -> 257 (eight warps spill 136 bytes at head sizes beyond 128, and still read best
+// where rows are few: 17 for one token behind 300 keys).  Two to four heads of up to 64 columns: 8/4x64: 1,500 470 -> 522, 300 x 20
+// 31 -> 19 -> 16 (four warps' CTAs leave less of L1 for keys that are read again): four only where the table holds few keys.
+template <typename KVT, int VW>
+int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stream) {
+    const int group = p.num_heads / p.num_kv_heads, sms = sm_count();
+    const long long ctas = (long long)p.tokens * p.num_kv_heads * (VW == 8 ? (group + 3) / 4 : (group + 7) / 8);
+    const long long keys = (long long)p.max_blocks * p.page_size;         // of a row at most
+    if (p.tokens <= 2 * sms / p.num_heads || (group == 1 && ctas < 4 * sms)) return launch_rows<KVT, VW, 1, 8, true>(p, q_bf16, out_bf16, stream);
+    const int wide = ctas < 2 * sms ? 8 : keys <= 64 ? 2 : VW > 2 || group == 1 || group > 4 || keys <= 128 ? 4 : 8;
+    auto go = [&](auto r) {
+        constexpr int R = decltype(r)::value;
+        if (wide == 2) return launch_rows<KVT, VW, R, 2, false>(p, q_bf16, out_bf16, stream);
+        if (wide == 4) return launch_rows<KVT, VW, R, 4, false>(p, q_bf16, out_bf16, stream);
+        return launch_rows<KVT, VW, R, 8, false>(p, q_bf16, out_bf16, stream);
+    };
+    if (group == 1) return go(std::integral_constant<int, 1>());
+    if constexpr (VW < 8)
+        if (group > 4) return go(std::integral_constant<int, 8>());
+    return go(std::integral_constant<int, 4>());
 }
 
 template <typename KVT>
 int launch_rows(const AttnParams& p, int q_bf16, int out_bf16, cudaStream_t stream) {
-    // heads of a kv head together (at most four at head size 256, whose accumulators are long); one where there are few rows
-    const int group = p.tokens <= 2 * sm_count() / p.num_heads ? 1 : p.num_heads / p.num_kv_heads;
-    if (p.head_dim > 128) return group == 1 ? launch_rows<KVT, 8, 1>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 8, 4>(p, q_bf16, out_bf16, stream);
-    if (p.head_dim > 64) return group == 1 ? launch_rows<KVT, 4, 1>(p, q_bf16, out_bf16, stream)
-                                : group <= 4 ? launch_rows<KVT, 4, 4>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 4, 8>(p, q_bf16, out_bf16, stream);
-    return group == 1 ? launch_rows<KVT, 2, 1>(p, q_bf16, out_bf16, stream)
-           : group <= 4 ? launch_rows<KVT, 2, 4>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 2, 8>(p, q_bf16, out_bf16, stream);
+    if (p.head_dim > 128) return launch_rows<KVT, 8>(p, q_bf16, out_bf16, stream);
+    return p.head_dim > 64 ? launch_rows<KVT, 4>(p, q_bf16, out_bf16, stream) : launch_rows<KVT, 2>(p, q_bf16, out_bf16, stream);
 }
 
 }  // namespace

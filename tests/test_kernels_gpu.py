@@ -418,6 +418,30 @@ def test_plain_attention_over_head_sizes_groups_and_cuts(dtype, nh, nkv, d, wind
     assert torch.equal(alone[0], got[3])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,d", [(6, 6, 20), (8, 8, 96), (3, 3, 136), (8, 4, 36), (12, 2, 100), (14, 2, 36), (8, 2, 200)])
+def test_plain_attention_of_many_tokens_has_the_bits_of_few(dtype, nh, nkv, d):
+    """Heads one by one and together, eight warps a CTA and four, tables of few keys and of many: a token's bits are the same in a step of
+    several hundred tokens (short sequences, then one long one) as alone."""
+    torch.manual_seed(nh + d)
+    for lens in ([20] * 300, [90] * 5, [330]):
+        news = [1] * 300 if len(lens) == 300 else lens
+        ks, vs = ([torch.randn(n, nkv, d) for n in lens] for _ in range(2))
+        qs = [torch.randn(n, nh, d) for n in news]
+        if dtype == torch.bfloat16:
+            ks, vs, qs = ([x.to(dtype).float() for x in y] for y in (ks, vs, qs))
+        pos0 = [l - n for l, n in zip(lens, news)]
+        got = run_attention(qs, ks, vs, pos0, nh, nkv, d, None, dtype, page_size=24, num_pages=320)
+        at = 0
+        for i in range(0, len(lens), 97):
+            n = news[i]
+            alone = run_attention([qs[i][n - 1:]], ks[i:i + 1], vs[i:i + 1], [lens[i] - 1], nh, nkv, d, None, dtype, page_size=24)
+            at = sum(news[:i + 1]) - 1
+            assert torch.equal(got[at], alone[0]), i
+        want = plain_attention_rows(qs[-1], ks[-1], vs[-1], pos0[-1], None).reshape(-1, nh * d)
+        assert torch.allclose(got[-news[-1]:], want, **tol(dtype))
+
+
 @pytest.mark.parametrize("nh,nkv,d", [(12, 2, 128), (4, 4, 64), (6, 1, 64)])
 def test_decode_step_of_long_and_short_sequences_shares_one_key_split(nh, nkv, d):
     """One decode step for sequences of 1,500, 20, 300 and 1 cached tokens: the number of CTAs that share a
