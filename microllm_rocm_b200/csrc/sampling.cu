@@ -540,10 +540,14 @@ MLB_EXPORT int mlb_sample_rows(const float* logits, long long ld, int rows, int 
         if (status != MLB_OK) return status;
         p.skip_greedy = 1;
     }
-    // Eight CTAs a row where an eighth fits an SM's shared memory and is worth a CTA (the vocabulary that greedy selection splits
-    // too); else one, whose six reads of a short row come from L2.
+    // Eight CTAs a row where an eighth fits an SM's shared memory and the rows leave room for them; else one, whose six reads of a
+    // row come from L2 and which two of an SM run at once.  Rows up to which the cluster is the faster one, us of one CTA / cluster, top
+    // 50 (148 SMs): vocabulary 16,384: 32 rows 44 / 28, 48 rows 44 / 48; 24,000: 32 45 / 33, 48 46 / 50; 32,000: 64 86 / 58, 96 78 / 82; 50,000: 64 69 / 60,
+    // 80 68 / 81; 151,936: 41 156 / 74, 64 226 / 86, 112 158 / 151, 128 160 / 167, 256 328 / 349; 250,000: 64 227 / 200, 80 227 / 246.
+    // (Greedy rows among them leave at once in both.)
     const int slice = (vocab + CLUSTER - 1) / CLUSTER;
-    if (vocab >= SPLIT_MIN_VOCAB && slice <= CLUSTER_MAX_SLICE && rows <= 0x7fffffff / CLUSTER) {
+    const int most_rows = vocab < 30000 ? 32 : 64;
+    if (vocab >= SPLIT_MIN_VOCAB && slice <= CLUSTER_MAX_SLICE && rows <= most_rows) {
         static bool configured[MAX_DEVICES] = {};
         const int d = device_index();
         if (!configured[d]) {

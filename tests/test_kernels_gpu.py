@@ -918,6 +918,23 @@ def test_sampling_among_zeros_of_both_signs(vocab):
                 assert token == want, (r, top_k[r], draw)
 
 
+@pytest.mark.parametrize("vocab, limit", [(16384, 32), (29999, 32), (30000, 64)])
+def test_sampling_of_many_rows_gives_the_tokens_of_few(vocab, limit):
+    """Up to `limit` rows a cluster of CTAs works on each, beyond it one CTA: the same tokens on both sides."""
+    torch.manual_seed(vocab)
+    n = limit + 3
+    x = (torch.randn(n, vocab) * 3).to(DEV)
+    args = (torch.full((n,), 0.8, device=DEV), torch.tensor([(0, 50, 1, 700)[r % 4] for r in range(n)], dtype=torch.int32, device=DEV),
+            torch.arange(n, device=DEV), torch.arange(n, device=DEV) * 3)
+
+    def sampled(a, b):
+        out = torch.full((b - a,), -77, dtype=torch.int32, device=DEV)
+        ops().sample_rows(x[a:b].contiguous(), *(t[a:b].contiguous() for t in args), out)
+        return out.tolist()
+    many = sampled(0, n)
+    assert sampled(0, limit) == many[:limit] and sampled(limit, n) == many[limit:] and sampled(0, limit + 1) == many[:limit + 1]
+
+
 def test_sampling_kernel_follows_the_distribution():
     logits = torch.tensor([[0.0, 1.0, 2.0, 0.5, -1.0]]).repeat(4000, 1)
     out = torch.empty(4000, dtype=torch.int32, device=DEV)
