@@ -190,7 +190,8 @@ MLB_EXPORT int mlb_add_scaled_rmsnorm(float* residual, const float* delta, int n
     auto* b = (__nv_bfloat16*)out;
     if (out_dtype != MLB_F32 && out_dtype != MLB_BF16) return fail(MLB_INVALID_ARGUMENT, "add_scaled_rmsnorm: unknown output dtype %d", out_dtype);
     const bool wide = out_dtype == MLB_F32;
-    if (width <= 4 * ROW_THREADS) wide ? go(add_scaled_rmsnorm_kernel<float, 4>, f) : go(add_scaled_rmsnorm_kernel<__nv_bfloat16, 4>, b);
+    if (width <= ROW_THREADS) wide ? go(add_scaled_rmsnorm_kernel<float, 1>, f) : go(add_scaled_rmsnorm_kernel<__nv_bfloat16, 1>, b);
+    else if (width <= 4 * ROW_THREADS) wide ? go(add_scaled_rmsnorm_kernel<float, 4>, f) : go(add_scaled_rmsnorm_kernel<__nv_bfloat16, 4>, b);
     else if (width <= 8 * ROW_THREADS) wide ? go(add_scaled_rmsnorm_kernel<float, 8>, f) : go(add_scaled_rmsnorm_kernel<__nv_bfloat16, 8>, b);
     else wide ? go(add_scaled_rmsnorm_kernel<float, 0>, f) : go(add_scaled_rmsnorm_kernel<__nv_bfloat16, 0>, b);
     return check_launch("add_scaled_rmsnorm");
