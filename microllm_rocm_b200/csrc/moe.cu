@@ -46,34 +46,37 @@ moe_select_kernel(const float* __restrict__ logits, long long ld, int n_partials
     float* z = logits_s + (size_t)warp * experts * (min(scoring, 2) + 1);
     float* score = z + experts;                         // scoring 1 to 3 only
     const float* row = logits + (size_t)t * ld;
-    // the logits and, behind them, the gate's: four columns a lane and four partial results of each asked for at a time
-    const int columns = experts + (gate_col >= 0 && gate_out ? 1 : 0);
-    for (int e0 = 0; e0 < columns; e0 += 128) {
-        float v[4];
-        const float* at[4];
+    // the logits, and in the first round the gate's in lane 31's fifth place: four columns a lane and four partial results of each asked
+    // for at a time
+    const bool gated = gate_col >= 0 && gate_out;
+    for (int e0 = 0; e0 < experts; e0 += 128) {
+        const bool gate_here = gated && e0 == 0 && lane == 31;
+        float v[5];
+        const float* at[5];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 5; ++j) {
             const int e = e0 + lane + 32 * j;
-            at[j] = row + (e < experts ? e : e < columns ? gate_col : 0);
-            v[j] = *at[j];
+            at[j] = row + (j == 4 ? (gate_here ? gate_col : 0) : min(e, experts - 1));
+            v[j] = j < 4 || gate_here ? *at[j] : 0.0f;
         }
         for (int k0 = 1; k0 < n_partials; k0 += 4) {
-            float part[4][4];
+            float part[4][5];
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[k][j] = k0 + k < n_partials && e0 + lane + 32 * j < columns ? at[j][(size_t)(k0 + k) * partial_stride] : 0.0f;
+                for (int j = 0; j < 5; ++j)
+                    part[k][j] = k0 + k < n_partials && (j < 4 ? e0 + lane + 32 * j < experts : gate_here) ? at[j][(size_t)(k0 + k) * partial_stride] : 0.0f;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] += part[k][j];
+                for (int j = 0; j < 5; ++j) v[j] += part[k][j];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int e = e0 + lane + 32 * j;
             if (e < experts) z[e] = scoring >= 1 ? v[j] : v[j] + (bias ? bias[e] : 0.0f);
-            else if (e < columns) gate_out[t] = 1.0f / (1.0f + expf(-v[j]));
         }
+        if (gate_here) gate_out[t] = 1.0f / (1.0f + expf(-v[4]));
     }
     if (scoring >= 2) {
         for (int e = lane; e < experts; e += 32) {      // (every lane turns its own elements)
