@@ -54,10 +54,19 @@ def key_splits(num_work: int, max_seq_len: int, sms: int) -> int:
     return max(1, min((2 * sms) // max(1, num_work), key_tiles // MIN_KEY_TILES_PER_SPLIT, MAX_SPLITS))
 
 
+def two_groups_pay(tiles: int, mean_keys: float, most_keys: int, sms: int) -> bool:
+    """Whether a CTA holds two groups of 16 rows, which share a ring of keys: from five tiles of 16 rows a multiprocessor on, and from four
+    where the tiles see about as many keys.  The CTAs are half as many, and with four tiles a multiprocessor all of them run at
+    once: the longest then sets the time.  Measured (512 + 64 wide, 148 SMs, us, one group / two): 16 heads, a prompt of 592 tokens
+    (592 tiles) 59 / 71, 640 69 / 73, 704 84 / 81, 740 92 / 83, 2,048 577 / 434; 592 tokens behind 1,500 288 / 235, 20 times 32 behind
+    2,000 471 / 382; 3 times 200 29 / 30; 4 heads, 2,500 tokens (625 tiles) 220 / 261, 3,000 334 / 315."""
+    return tiles >= 5 * sms or (tiles >= 4 * sms and mean_keys >= 0.7 * most_keys)
+
+
 def _plan(ctx, heads: int):
     """Work items of a step ((sequence, first row) per 16 rows of a sequence's new (token, head) rows, or 32; long causal
-    ranges first), the key split and the groups of 16 rows a CTA holds, shared by every layer with this many heads.  Two
-    groups where four a multiprocessor have work, and the keys are not split."""
+    ranges first), the key split and the groups of 16 rows a CTA holds (two_groups_pay; one where the keys are split), shared by every
+    layer with this many heads."""
     from .device import sm_count
     key = ("latent_mma", heads)
     plan = ctx.extras.get(key)
@@ -69,13 +78,15 @@ def _plan(ctx, heads: int):
     rows = [(starts[a + 1] - starts[a]) * heads for a in range(ctx.num_seqs)]
     tiles = sum(-(-n // ROWS_PER_TILE) for n in rows)
     splits = key_splits(tiles, ctx.max_seq_len, sms) if ctx.decode_only or tiles <= 32 else 1
-    groups = 2 if splits == 1 and not ctx.decode_only and tiles >= 4 * sms else 1
+    front = ctx.seq_pos0_host or [0] * ctx.num_seqs
+    new = [starts[a + 1] - starts[a] for a in range(ctx.num_seqs)]
+    mean = sum(n * (p + 0.5 * (n + 1)) for n, p in zip(new, front)) / max(1, sum(new))           # keys that a new token sees
+    groups = 2 if splits == 1 and not ctx.decode_only and two_groups_pay(tiles, mean, max((n + p for n, p in zip(new, front)), default=0), sms) else 1
     if GROUPS is not None and splits == 1:
         groups = GROUPS
     work = []
     for a in range(ctx.num_seqs):
-        pos0 = ctx.seq_pos0_host[a] if ctx.seq_pos0_host else 0
-        work += [(pos0 + first // heads, a, first) for first in range(0, rows[a], groups * ROWS_PER_TILE)]
+        work += [(front[a] + first // heads, a, first) for first in range(0, rows[a], groups * ROWS_PER_TILE)]
     if not ctx.decode_only:
         work.sort(key=lambda item: -item[0])
     work_dev = ops.upload([x for _, a, first in work for x in (a, first)], "int32", device)

@@ -106,3 +106,12 @@ def test_the_held_back_builds_of_the_first_kernels_keep_their_list():
     from microllm_rocm_b200.kernels import ops
     assert {source for source, _ in ops.lagged_sources()} == {"attention_tc.cu", "gemm_stream.cu", "gemm_tc2.cu", "attention_mma.cu"}
     assert {source for source, _ in ops.lagged_group_sources()} == {"grouped_tc2.cu"}
+
+
+@pytest.mark.parametrize("tiles, mean, most, pays", [
+    (592, 296, 592, False), (640, 320, 640, False), (740, 370, 740, True), (739, 370, 740, False), (2048, 1024, 2048, True),      # one prompt
+    (592, 1796, 2092, True), (640, 2016, 2032, True), (591, 1796, 2092, False), (600, 100, 200, False),      # behind many keys; short prompts
+])
+def test_when_two_groups_of_latent_rows_share_their_keys(tiles, mean, most, pays):
+    from microllm_rocm_b200.kernels import latent
+    assert latent.two_groups_pay(tiles, mean, most, 148) is pays
