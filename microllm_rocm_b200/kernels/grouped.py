@@ -65,16 +65,30 @@ def pair_supported(a: torch.Tensor, weight: torch.Tensor) -> bool:
     return mma_supported(a, weight) and G <= 1024 and weight.is_contiguous() and a.stride(1) == 1 and G * N < 1 << 31
 
 
-def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: int) -> bool:
-    """Tiles of 256 weight rows for pairs of SMs: worth it for large groups whatever their number, for groups of 16 rows and more where
-    every pair has a tile, and for small groups whose weights (`weight_bytes` a group) take long enough to read that the set-up of a
-    pair does not show.  Measured (gate/up + down, us, mma.sync against pairs): 64 groups of 1,408, width 2,048: 24 listed rows
-    46 + 27 / 44 + 30, 48 rows 69 + 43 / 65 + 39, 1,200 rows 181 + 101 / 128 + 64, 12,288 rows 616 + 379 / 184 + 112; 32 of 704: 256 rows 39 + 20 / 43 + 23,
-    512 rows 55 + 25 / 45 + 24; 16 of 512, width 1,024: 256 rows 18 + 17 / 35 + 19, 1,024 rows 23 + 15 / 26 + 16, 1,600 rows 39 + 15 / 27 + 16."""
+def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: int, dual: bool = True) -> bool:
+    """Whether a listed product goes to pairs of SMs with tiles of 256 weight rows (`weight_bytes` a group; `dual`: the gated form).  Against
+    it stand the set-up of a pair (5 us, and 2 for the gathering), waves of tiles that a last one leaves half empty, and an epilogue that
+    short sums do not hide.  Measured (148 SMs, us, mma.sync / pairs):
+      * Groups of more than 16 rows, where mma.sync takes 64 rows a tile: every pair needs a tile.  32 of 768 rows, width 1,024: gate/up
+        of 512 23 / 21, down 16 / 12; sums of 256 lose (64 groups of 48 rows 15.5 / 16.5).
+      * From 96 rows on (128 a tile) few tiles are enough, but sums below 1,024 need work to amortize: gate/up from 0.8 GFLOP on, plain
+        from 2.  600 rows, width 2,048: gate/up of 704 44 / 28, down 17.2 / 19.2; 8 groups of 192 rows, 512 x 1,024: 15.1 / 17.9;
+        64 groups of 192 of 1,408, width 2,048: 616 / 170 and 379 / 108; sums of 256 lose (16 x 600 rows 25.6 / 29.0).
+      * Up to 16 rows both stream the weights, 16 rows a tile on mma.sync: pairs where the weights in use are large and fill their
+        waves of tiles.  48 rows for 64 groups of 1,408, width 2,048: 69 + 43 / 65 + 39; 12 rows for 32 of 1,408, width 4,096: gate/up 49 / 54; 512 rows for 64 of 704: 71 / 79 (384 tiles
+        in six waves of 74); 48 rows for 16 groups of 1,408, width 4,096: 73 / 78 (176 tiles in three waves); 512 for 32 of 704, width 2,048:
+        55 / 45."""
     if USE_PAIRS is not None:
         return USE_PAIRS
-    active = min(groups, rows)
-    return rows >= 96 * groups or (rows >= 16 * groups and -(-weight_rows // 256) * active >= sms // 2) or active * weight_bytes >= 200 << 20
+    active, pairs = min(groups, rows), sms // 2
+    tiles, total = active * -(-weight_rows // 256), active * weight_bytes
+    k = weight_bytes // (2 * weight_rows)
+    if rows >= 96 * groups:
+        return k >= 1024 or (k >= 512 and 2 * rows * weight_rows * k >= (0.8e9 if dual else 2e9))
+    if rows > 16 * groups:
+        return tiles >= pairs and k >= 512
+    filled = active * weight_rows / (256 * pairs * max(1, -(-tiles // pairs)))
+    return (total >= 150 << 20 and filled >= 0.75) if rows >= 16 * groups else (total >= (300 if dual else 250) << 20 and filled >= 0.85)
 
 
 def _pair(a, weight, out, *, rows, outputs, group_offsets, a_rows, a_row_div, c_rows, dual, act, row_scale, row_tile, alloc, error_flag):
@@ -142,7 +156,7 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
     if row_scale is not None:
         ops._need(row_scale, "row_scale", torch.float32)
     if (group_offsets is not None and a_rows is None and factor is None and row_scale is None and not a_group_cols and not c_group_cols
-            and pair_supported(a, weight) and pair_pays(rows, G, N, weight.stride(0) * 2, sm_count(a.device))):
+            and pair_supported(a, weight) and pair_pays(rows, G, N, weight.stride(0) * 2, sm_count(a.device), dual=False)):
         _pair(a, weight, out, rows=rows, outputs=N, group_offsets=group_offsets, a_rows=None, a_row_div=a_row_div, c_rows=c_rows, dual=False,
               act=0, row_scale=None, row_tile=row_tile, alloc=None, error_flag=error_flag)
         return

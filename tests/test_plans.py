@@ -115,3 +115,16 @@ def test_the_held_back_builds_of_the_first_kernels_keep_their_list():
 def test_when_two_groups_of_latent_rows_share_their_keys(tiles, mean, most, pays):
     from microllm_rocm_b200.kernels import latent
     assert latent.two_groups_pay(tiles, mean, most, 148) is pays
+
+
+@pytest.mark.parametrize("rows, groups, weight_rows, k, dual, pays", [
+    (600, 1, 2048, 704, False, False), (600, 1, 1408, 2048, True, True), (96, 1, 1408, 2048, True, True),      # one group of many rows
+    (1536, 8, 1024, 512, False, False), (3072, 16, 1024, 512, False, True), (1536, 8, 1024, 512, True, True),      # the work that shorter sums take
+    (9600, 16, 512, 256, True, False), (12288, 64, 512, 256, True, False), (3072, 64, 512, 256, True, False),      # sums that do not hide the epilogue
+    (768, 32, 1024, 1024, True, True), (384, 16, 1024, 1024, True, False), (385, 24, 1024, 512, True, True), (384, 24, 1024, 512, True, False),
+    (48, 64, 2816, 2048, True, True), (512, 64, 1408, 2048, True, False), (48, 16, 2816, 4096, True, False), (12, 32, 2816, 4096, True, False),
+    (48, 64, 2048, 1408, False, True), (44, 64, 2048, 1408, False, False), (512, 32, 1408, 2048, True, True), (128, 8, 2816, 4096, True, False), (0, 64, 2816, 2048, True, False), (1, 1, 8, 8, False, False),
+])
+def test_which_grouped_products_go_to_pairs_by_form_and_length_of_sums(rows, groups, weight_rows, k, dual, pays):
+    from microllm_rocm_b200.kernels import grouped
+    assert grouped.pair_pays(rows, groups, weight_rows, weight_rows * k * 2, 148, dual) is pays
