@@ -293,6 +293,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 tmem_ld32_nowait(lane_addr + (uint32_t)c, raw);
                 if (p.dual) tmem_ld32_nowait(lane_addr + (uint32_t)(p.tok_tile + c), raw_u);
                 tmem_wait();
+                if (!p.dual) {                       // nothing to evaluate: each value leaves as it comes (kept for later as below: fp32 51 -> 63 us
+                    if (f >= p.N) continue;          // at 2,048 tokens, 1,536 -> 8,960, bf16 51 -> 53.5)
+                    const int here = min(32, p.M - tok0 - c);
+                    const size_t at = (size_t)(tok0 + c) * p.ldo + f;
+                    if (p.out_bf16) {
+                        __nv_bfloat16* o = (__nv_bfloat16*)p.out + at;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j, o += p.ldo) {
+                            if (j >= here) break;
+                            *o = __float2bfloat16_rn(__uint_as_float(raw[j]) + bias);
+                        }
+                    } else if (!p.accumulate) {
+                        float* o = (float*)p.out + at;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j, o += p.ldo) {
+                            if (j >= here) break;
+                            *o = __uint_as_float(raw[j]) + bias;
+                        }
+                    } else {
+                        float* o = (float*)p.out + at;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j, o += p.ldo) {
+                            if (j >= here) break;
+                            *o += __uint_as_float(raw[j]) + bias;
+                        }
+                    }
+                    continue;
+                }
                 // Values first, all 32 side by side, then the stores, and the activation chosen outside the loop: with a branch per value
                 // they stood one behind another and the epilogue held the pair's products up (gate/up of 2,048 tokens at 1,536 -> 8,960:
                 // 94.2 us, now 88.5; 512 tokens at 3,584 -> 18,944: 117.5 and 115.2).
@@ -303,12 +331,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 } else if (p.dual == 2) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) r[j] = gated_value<1>(__uint_as_float(raw[j]), __uint_as_float(raw_u[j]), 0.0f);
-                } else if (p.dual == 1) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = gated_value<0>(__uint_as_float(raw[j]), __uint_as_float(raw_u[j]), 0.0f);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __uint_as_float(raw[j]);
+                    for (int j = 0; j < 32; ++j) r[j] = gated_value<0>(__uint_as_float(raw[j]), __uint_as_float(raw_u[j]), 0.0f);
                 }
                 const int here = f < p.N ? p.M - tok0 - c : 0;             // tokens of these 32 that exist
                 const size_t at = (size_t)(tok0 + c) * p.ldo + f;
