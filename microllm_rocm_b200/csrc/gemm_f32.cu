@@ -20,8 +20,10 @@
 //
 // Products of a step of 28 layers (1,536 wide, 8,960 inside, 151,936-row head) on a B200: two rows 1.31 ms, 4.7 TB/s of weights (51 ms with one 64 x
 // 64 tile kernel for every M, whose sixteen column threads held idle rows and whose grid left most SMs empty); 333 rows
-// 29 ms, 30 TFLOP/s (77 ms).  STREAM_MAX_M: 32 rows are two passes over W from the tile of 16, still less than a tile half
-// full.
+// 29 ms, 30 TFLOP/s (77 ms).  STREAM_MAX_M, measured (us, streamed / tiled): 17 .. 32 rows (two passes over W) 1,536 -> 2,048 16 / 36,
+// 8,960 -> 1,536 78 / 160, 1,536 -> 17,920 124 / 109; 33 .. 48 rows (three) 23 / 34, 79 / 160, 183 / 108; 64 rows 31 / 34, 117 / 160, 240 / 107: the
+// narrow products gain with every pass less, the wide one loses from the second on, and the products of a layer together are
+// even at about 48 rows (16 rows: 8 / 37, 40 / 160, 64 / 111).
 #include <cooperative_groups.h>
 
 #include "common.cuh"

@@ -11,10 +11,10 @@
 // gated form a CTA's 128 weight rows are 64 gate rows above the 64 up rows of the same outputs, and two epilogue warps exchange
 // halves of what they read (128 gate and 128 up rows in two accumulators of 256 columns would leave tensor memory no second pair).
 // The epilogue has to keep up with a tile's products (10 us at 2,048 elements of K): with a branch per value in it, the full
-// quotient's among them, it took three times that, and gate/up 285 us in place of 161.
+// quotient's among them, it took three times that, and gate/up 285 us in place of 168.
 //
-// At 2,048 tokens, 64 experts of 1,408, six chosen (192 rows an expert, width 2,048): 161 us for gate/up (142 GFLOP, 880 TFLOP/s; tensor
-// pipe 61 % busy, DRAM 62 %), 20 for gathering its rows, 110 for down; the mma.sync kernel (grouped_mma.cu) takes 617 and 379.
+// At 2,048 tokens, 64 experts of 1,408, six chosen (192 rows an expert, width 2,048): 168 us for gate/up (142 GFLOP, 845 TFLOP/s; tensor
+// pipe 61 % busy, DRAM 62 %), 30 for gathering its rows, half of it beside other kernels, 108 for down; the mma.sync kernel (grouped_mma.cu) takes 617 and 379.
 // The weights alone are 1.1 GB, 170 us of memory time.  Which kernel takes a product: kernels/grouped.py, pair_pays.
 //
 // Every mbarrier wait is bounded (error flag, then everybody falls through to the common end); the two cluster barriers

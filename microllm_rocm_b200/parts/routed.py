@@ -33,8 +33,12 @@ from ..kernels.ops import CLAMPED_ACTIVATION
 from .base import FEED_FORWARDS, FeedForward, Runtime, StepContext, WeightSpec, make, register_feed_forward, scratch
 
 
-# Steps up to which the shared expert runs beside the router (a decode step of 8 requests, 64 experts of 1,408 and a shared one of
-# 2,816, eight layers: 1.71 ms a step one after the other, 1.58 side by side)
+# Steps up to which the shared expert runs beside the router.  Captured decode steps of eight layers, us, one after the other / side by
+# side: 64 experts of 1,408 with a shared one of 2,816 (width 2,048): 1 token 1,087 / 960, 8 1,562 / 1,429, 16 1,953 / 1,836, 32 2,241 / 2,129;
+# 16 of 512 with one of 1,024 (width 1,024): 1 576 / 460, 8 576 / 528, 16 687 / 577, 32 751 / 649.  Beyond 32 tokens products of less than
+# 8 MB are the library's and stay on one stream, so the smaller shared expert could not go; the larger one would still gain (64 tokens
+# 2,385 / 2,294).  Prompts issued from the host, whose calls the fork adds to: 2 tokens 2,078 / 2,032 and 1,570 / 1,633, 32 tokens
+# 2,921 / 2,898 and 1,712 / 1,685.
 SIDE_MAX_TOKENS = 32
 
 
