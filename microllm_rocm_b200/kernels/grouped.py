@@ -73,7 +73,7 @@ def pair_pays(rows: int, groups: int, weight_rows: int, weight_bytes: int, sms: 
         of 512 23 / 21, down 16 / 12; sums of 256 lose (64 groups of 48 rows 15.5 / 16.5).
       * From 96 rows on (128 a tile) few tiles are enough, but sums below 1,024 need work to amortize: gate/up from 0.8 GFLOP on, plain
         from 2.  600 rows, width 2,048: gate/up of 704 44 / 28, down 17.2 / 19.2; 8 groups of 192 rows, 512 x 1,024: 15.1 / 17.9;
-        64 groups of 192 of 1,408, width 2,048: 616 / 170 and 379 / 108; sums of 256 lose (16 x 600 rows 25.6 / 29.0).
+        64 groups of 192 of 1,408, width 2,048: 617 / 186 and 379 / 108; sums of 256 lose (16 x 600 rows 25.6 / 29.0).
       * Up to 16 rows both stream the weights, 16 rows a tile on mma.sync: pairs where the weights in use are large and fill their
         waves of tiles.  48 rows for 64 groups of 1,408, width 2,048: 69 + 43 / 65 + 39; 12 rows for 32 of 1,408, width 4,096: gate/up 49 / 54; 512 rows for 64 of 704: 71 / 79 (384 tiles
         in six waves of 74); 48 rows for 16 groups of 1,408, width 4,096: 73 / 78 (176 tiles in three waves); 512 for 32 of 704, width 2,048:
