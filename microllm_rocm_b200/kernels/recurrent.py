@@ -27,11 +27,11 @@ ops.register_signatures("delta_rule.cu", {
                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "mlb_take_columns": [c_void_p, c_longlong, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
     "mlb_linear_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
-                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "mlb_head_scan": [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "mlb_delta_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                       c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                       c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "mlb_delta_output": [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_longlong, c_int, c_void_p, c_void_p, c_longlong, c_int,
                          c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
 })
@@ -133,7 +133,7 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, g: torch.Tensor, beta: torch.
     L = ops.lib("delta_rule.cu")
     build.check(L, L.mlb_delta_scan(qn.data_ptr(), kn.data_ptr(), g.data_ptr(), beta.data_ptr(), v.data_ptr(), v.stride(0),
                                     o.data_ptr(), state.data_ptr(), slots.data_ptr(), state.shape[0], ctx.seq_starts.data_ptr(),
-                                    ctx.seq_pos0.data_ptr(), ctx.num_seqs, heads, kv_heads, dk, dv, ops._ptr(ctx.error_flag),
+                                    ctx.seq_pos0.data_ptr(), v.shape[0], ctx.num_seqs, heads, kv_heads, dk, dv, ops._ptr(ctx.error_flag),
                                     ops._stream()))
 
 
@@ -185,7 +185,7 @@ def linear_scan(rule: str, q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor
     L = ops.lib("delta_rule.cu")
     build.check(L, L.mlb_linear_scan(RULES[rule], q.data_ptr(), k.data_ptr(), decay.data_ptr(), ops._ptr(bonus), v.data_ptr(), v.stride(0),
                                      o.data_ptr(), state.data_ptr(), slots.data_ptr(), state.shape[0], ctx.seq_starts.data_ptr(),
-                                     ctx.seq_pos0.data_ptr(), ctx.num_seqs, heads, heads, dk, dv, ops._ptr(ctx.error_flag), ops._stream()))
+                                     ctx.seq_pos0.data_ptr(), T, ctx.num_seqs, heads, heads, dk, dv, ops._ptr(ctx.error_flag), ops._stream()))
 
 
 def head_scan(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.Tensor, o: torch.Tensor, state: torch.Tensor,
@@ -224,5 +224,5 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.Te
     L = ops.lib("delta_rule.cu")
     build.check(L, L.mlb_head_scan(q.data_ptr(), k.data_ptr(), q.stride(0), G, decay.data_ptr(), 1 if per_token else 0, ops._ptr(weight), v.data_ptr(), v.stride(0),
                                    o.data_ptr(), state.data_ptr(), ops._ptr(n_state), ops._ptr(den), slots.data_ptr(), state.shape[0],
-                                   ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), ctx.num_seqs, heads, dk, dv, ops._ptr(ctx.error_flag),
+                                   ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), T, ctx.num_seqs, heads, dk, dv, ops._ptr(ctx.error_flag),
                                    ops._stream()))

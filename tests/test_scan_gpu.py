@@ -1,0 +1,62 @@
+"""The recurrences' scan kernel with one and with two columns a lane (scan_per_lane in csrc/delta_rule.cu): a row's bits do not depend on it."""
+import pytest
+import torch
+
+DEV = "cuda"
+
+
+def step(counts, pos0):
+    from microllm_rocm_b200.parts.base import StepContext
+    starts = [0]
+    for n in counts:
+        starts.append(starts[-1] + n)
+    on = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    A, T = len(counts), starts[-1]
+    ctx = StepContext(num_tokens=T, num_seqs=A, token_ids=on([0] * T), positions=on([p + i for n, p in zip(counts, pos0) for i in range(n)]),
+                      token_seq=on([a for a, n in enumerate(counts) for _ in range(n)]), seq_starts=on(starts), seq_pos0=on(pos0),
+                      seq_lens=on([n + p for n, p in zip(counts, pos0)]), block_tables={}, state_slots=on(list(range(A))), logit_rows=None,
+                      error_flag=torch.zeros(1, dtype=torch.int32, device=DEV), seq_starts_host=starts, seq_pos0_host=list(pos0),
+                      max_new_tokens=max(counts), max_seq_len=max(n + p for n, p in zip(counts, pos0)))
+    return ctx, ctx.state_slots
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dk, dv, alike", [(128, 128, True), (96, 52, True), (64, 64, True), (30, 37, False), (200, 40, True)])
+@pytest.mark.parametrize("rule", ["delta", "decayed_sum", "bonus_read", "head", "head and vector"])
+def test_many_sequences_have_the_bits_of_each_alone(rule, dk, dv, alike):
+    """Sequences together fill the device and take two columns a lane, one alone takes one; portions of one token, of part of a staged chunk and
+    of several, some from a state and some from zero."""
+    from microllm_rocm_b200.kernels import recurrent
+    H, counts, pos0 = 16, [1, 3, 8, 37, 64, 5, 17, 2, 9, 33], [4, 0, 7, 0, 12, 1, 0, 3, 0, 2]
+    A, T = len(counts), sum(counts)
+    g = torch.Generator(DEV).manual_seed(dk)
+    f = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    q, k, v = f(T, H * dk) * dk ** -0.5, torch.nn.functional.normalize(f(T, H, dk), dim=-1).reshape(T, -1), f(T, H * dv)
+    decay, head_decay = torch.rand(T, H * dk, generator=g, device=DEV) * 0.3 + 0.7, torch.rand(T, H, generator=g, device=DEV) * 0.2 + 0.8
+    beta, bonus, start, vector = torch.rand(T, H, generator=g, device=DEV), f(H, dk), f(A + 1, H, dk, dv), f(A + 1, H, dk)
+
+    def run(which):
+        starts = torch.cumsum(torch.tensor([0] + counts), 0).tolist()
+        rows = torch.cat([torch.arange(starts[a], starts[a + 1]) for a in which]).to(DEV)
+        ctx, slots = step([counts[a] for a in which], [pos0[a] for a in which])
+        cut = lambda t: t[rows].contiguous()
+        keep = torch.tensor(which, device=DEV)
+        state, n_state = torch.cat([start[keep], start[-1:]]).contiguous(), torch.cat([vector[keep], vector[-1:]]).contiguous()
+        o, den = torch.empty(len(rows), H * dv, device=DEV), torch.zeros(len(rows), H, device=DEV)
+        if rule == "delta":
+            recurrent.delta_scan(cut(q), cut(k), cut(decay), cut(beta), cut(v), o, state, slots, ctx, H, H, dk, dv)
+        elif rule.startswith("head"):
+            beside = dict(n_state=n_state, den=den) if rule != "head" else {}
+            recurrent.head_scan(cut(q), cut(k), cut(head_decay), cut(v), o, state, slots, ctx, H, dk, dv, weight=cut(beta), **beside)
+        else:
+            recurrent.linear_scan(rule, cut(q), cut(k), cut(decay), cut(v), o, state, slots, ctx, H, dk, dv, bonus=bonus if rule == "bonus_read" else None)
+        assert int(ctx.error_flag.item()) == 0
+        return o, state[:len(which)], n_state[:len(which)], den
+
+    together = run(list(range(A)) * 1)
+    at = 0
+    for a in range(A):
+        o, state, n_state, den = run([a])
+        assert torch.equal(together[0][at:at + counts[a]], o) and torch.equal(together[1][a], state[0])
+        assert torch.equal(together[2][a], n_state[0]) and torch.equal(together[3][at:at + counts[a]], den)
+        at += counts[a]
