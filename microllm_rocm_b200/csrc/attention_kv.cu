@@ -42,6 +42,20 @@ struct Columns {               // a block of columns of fp32 rows, possibly K-sp
         for (int k = 1; k < n_partials; ++k) v += p[(size_t)k * partial_stride];
         return v;
     }
+    // columns col + lane, col + lane + 32, ... of a row (zero from the n-th on): the partial results of all of them are asked for a step of
+    // the sum at a time, four steps together, where at() would make a trip to memory of every few of them
+    template <int N> __device__ __forceinline__ void at_lanes(long long row, int col, int n, float (&v)[N]) const {
+        const int lane = threadIdx.x & 31;
+        const float* p = base + row * ld + col + lane;
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = lane + 32 * i < n ? p[32 * i] : 0.0f;
+#pragma unroll 4
+        for (int k = 1; k < n_partials; ++k) {
+            p += partial_stride;
+#pragma unroll
+            for (int i = 0; i < N; ++i) if (lane + 32 * i < n) v[i] += p[32 * i];
+        }
+    }
 };
 
 struct PrepareParams {
@@ -80,10 +94,13 @@ __global__ void __launch_bounds__(WARPS * 32) qk_prepare_kernel(PrepareParams p)
     const Columns& src = is_q ? p.q : (is_k ? p.k : p.v);
     const int col = (is_q ? p.q_col : (is_k ? p.k_col : p.v_col)) + head * D;
     float x[NL];
+    src.at_lanes(t, col, D, x);
+    if (p.bias) {
 #pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        const int c = lane + 32 * i;
-        x[i] = c < D ? src.at(t, col + c) + (p.bias ? p.bias[col + c] : 0.0f) : 0.0f;
+        for (int i = 0; i < NL; ++i) {
+            const int c = lane + 32 * i;
+            if (c < D) x[i] += p.bias[col + c];
+        }
     }
     // where the item goes
     KVT* page_row = nullptr;
@@ -318,15 +335,28 @@ __global__ void gate_heads_x8_kernel(GateParams p) {
     uint4 raw = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.o + (t * p.H + h) * p.PV + c);
     if (p.gate.base) {
         __nv_bfloat162* pair = reinterpret_cast<__nv_bfloat162*>(&raw);
-        const float head_gate = p.gate_per_head ? sigmoid_f32(p.gate.at(t, p.gate_col + h)) : 1.0f;
+        float g[8];
+        if (p.gate_per_head) {
+            g[0] = p.gate.at(t, p.gate_col + h);
+#pragma unroll
+            for (int k = 1; k < 8; ++k) g[k] = g[0];
+        } else {                                 // (16 bytes at a time; the partial results of all eight a step of the sum at a time)
+            const float* at = p.gate.base + t * p.gate.ld + p.gate_col + h * p.DV + c;
+            *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(at);
+            *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(at + 4);
+#pragma unroll 4
+            for (int k = 1; k < p.gate.n_partials; ++k) {
+                at += p.gate.partial_stride;
+                const float4 lo = *reinterpret_cast<const float4*>(at), hi = *reinterpret_cast<const float4*>(at + 4);
+                g[0] += lo.x; g[1] += lo.y; g[2] += lo.z; g[3] += lo.w;
+                g[4] += hi.x; g[5] += hi.y; g[6] += hi.z; g[7] += hi.w;
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             float2 v = __bfloat1622float2(pair[k]);
-            if (p.gate_per_head) { v.x *= head_gate; v.y *= head_gate; }
-            else {
-                v.x *= sigmoid_f32(p.gate.at(t, p.gate_col + h * p.DV + c + 2 * k));
-                v.y *= sigmoid_f32(p.gate.at(t, p.gate_col + h * p.DV + c + 2 * k + 1));
-            }
+            v.x *= sigmoid_f32(g[2 * k]);
+            v.y *= sigmoid_f32(g[2 * k + 1]);
             pair[k] = __floats2bfloat162_rn(v.x, v.y);
         }
     }
@@ -356,7 +386,8 @@ MLB_EXPORT int mlb_gate_heads(const void* o, void* out, int dtype, const float* 
                  gate_per_head ? 1 : 0};
     const long long n = (long long)T * H * DV;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (dtype == MLB_BF16 && DV % 8 == 0 && stored_v % 8 == 0 && ((uintptr_t)o | (uintptr_t)out) % 16 == 0)
+    const bool gates_aligned = !gate || gate_per_head || (gate_col % 4 == 0 && gate_ld % 4 == 0 && gate_partial_stride % 4 == 0 && (uintptr_t)gate % 16 == 0);
+    if (dtype == MLB_BF16 && DV % 8 == 0 && stored_v % 8 == 0 && ((uintptr_t)o | (uintptr_t)out) % 16 == 0 && gates_aligned)
         launch_kernel(gate_heads_x8_kernel, (unsigned)((n / 8 + 255) / 256), 256, 0, stream, p);
     else if (dtype == MLB_BF16) launch_kernel(gate_heads_kernel<__nv_bfloat16>, blocks, 256, 0, stream, p);
     else if (dtype == MLB_F32) launch_kernel(gate_heads_kernel<float>, blocks, 256, 0, stream, p);

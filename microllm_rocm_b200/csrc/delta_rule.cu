@@ -44,6 +44,20 @@ struct Columns {
         for (int k = 1; k < n_partials; ++k) v += p[(size_t)k * partial_stride];
         return v;
     }
+    // columns col + lane, col + lane + 32, ... of a row (zero from the n-th on): the partial results of all of them are asked for a step of
+    // the sum at a time, four steps together, where at() would make a trip to memory of every few of them
+    template <int N> __device__ __forceinline__ void at_lanes(long long row, int col, int n, float (&v)[N]) const {
+        const int lane = threadIdx.x & 31;
+        const float* p = base + row * ld + col + lane;
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = lane + 32 * i < n ? p[32 * i] : 0.0f;
+#pragma unroll 4
+        for (int k = 1; k < n_partials; ++k) {
+            p += partial_stride;
+#pragma unroll
+            for (int i = 0; i < N; ++i) if (lane + 32 * i < n) v[i] += p[32 * i];
+        }
+    }
 };
 
 __device__ __forceinline__ float sigmoid(float v) {
@@ -96,18 +110,32 @@ __global__ void __launch_bounds__(WARPS * 32) delta_prepare_kernel(PrepareParams
     }
     const int h = which - 2 * p.G;
     const float rate = expf(p.a_log[h]);
-    for (int c = lane; c < p.DK; c += 32) {
-        float pre = 0.0f;
-        if (p.pre.base) {
-            pre = p.pre.at(t, h * p.DK + c);
-        } else {
-            const float* w = p.w2 + ((size_t)h * p.DK + c) * p.a_rank;
-            for (int r = 0; r < p.a_rank; ++r) pre = fmaf(w[r], p.proj.at(t, p.a_col + r), pre);
+    // beta's partial results, one a lane, on their way beside the decay's
+    const float* const beta_at = p.proj.base + (size_t)t * p.proj.ld + p.beta_col + h;
+    const bool together = p.proj.n_partials <= 32;
+    float part = together && lane < p.proj.n_partials ? beta_at[(size_t)lane * p.proj.partial_stride] : 0.0f;
+    float pre[PER_LANE];
+    if (p.pre.base) {
+        p.pre.at_lanes(t, h * p.DK, p.DK, pre);
+    } else {
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) pre[i] = 0.0f;
+        for (int r = 0; r < p.a_rank; ++r) {
+            const float a = p.proj.at(t, p.a_col + r);
+#pragma unroll
+            for (int i = 0; i < PER_LANE; ++i)
+                if (lane + 32 * i < p.DK) pre[i] = fmaf(p.w2[((size_t)h * p.DK + lane + 32 * i) * p.a_rank + r], a, pre[i]);
         }
-        pre += p.dt_bias[h * p.DK + c];
-        p.g[((size_t)t * p.H + h) * p.DK + c] = expf(-rate * softplus(pre));
     }
-    if (lane == 0) p.beta[(size_t)t * p.H + h] = sigmoid(p.proj.at(t, p.beta_col + h));
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int c = lane + 32 * i;
+        if (c < p.DK) p.g[((size_t)t * p.H + h) * p.DK + c] = expf(-rate * softplus(pre[i] + p.dt_bias[h * p.DK + c]));
+    }
+    float beta = __shfl_sync(0xffffffffu, part, 0);
+    for (int k = 1; k < min(p.proj.n_partials, 32); ++k) beta += __shfl_sync(0xffffffffu, part, k);       // in split order
+    if (!together) beta = p.proj.at(t, p.beta_col + h);
+    if (lane == 0) p.beta[(size_t)t * p.H + h] = sigmoid(beta);
 }
 
 // ------------------------------------------------------------------------------ the recurrence
@@ -502,20 +530,25 @@ __global__ void __launch_bounds__(WARPS * 32) delta_output_kernel(OutputParams p
         x[i] = c < p.DV ? src[c] : 0.0f;
         ss = fmaf(x[i], x[i], ss);
     }
+    float pre[PER_LANE];
+    if (p.pre.base) {
+        p.pre.at_lanes(t, h * p.DV, p.DV, pre);
+    } else {
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) pre[i] = 0.0f;
+        for (int r = 0; r < p.g_rank; ++r) {
+            const float a = p.proj.at(t, p.g_col + r);
+#pragma unroll
+            for (int i = 0; i < PER_LANE; ++i)
+                if (lane + 32 * i < p.DV) pre[i] = fmaf(p.w2[((size_t)h * p.DV + lane + 32 * i) * p.g_rank + r], a, pre[i]);
+        }
+    }
     const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)p.DV + p.eps);
     OutT* dst = (OutT*)p.out + ((size_t)t * p.H + h) * p.DV;
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) {
         const int c = lane + 32 * i;
-        if (c >= p.DV) continue;
-        float pre = 0.0f;
-        if (p.pre.base) {
-            pre = p.pre.at(t, h * p.DV + c);
-        } else {
-            const float* w = p.w2 + ((size_t)h * p.DV + c) * p.g_rank;
-            for (int r = 0; r < p.g_rank; ++r) pre = fmaf(w[r], p.proj.at(t, p.g_col + r), pre);
-        }
-        dst[c] = from_f32<OutT>(x[i] * inv * p.weight[c] * sigmoid(pre));
+        if (c < p.DV) dst[c] = from_f32<OutT>(x[i] * inv * p.weight[c] * sigmoid(pre[i]));
     }
 }
 
