@@ -8,7 +8,8 @@
 // tokens before the step; inputs of positions before the step come from the state of the sequence's slot
 // ([slots, taps - 1, C] fp32, oldest first), inputs of positions before 0 are zero whatever the slot holds (a slot
 // is never cleared when a new request takes it).  `mlb_short_conv_state` then moves the state on; it runs after the
-// convolution has read the old one.
+// convolution has read the old one.  Where every sequence brings one token (decoding) the thread that reads a channel's old inputs
+// is the only one that does, and moves them on itself (`move`).
 #include "common.cuh"
 
 using namespace mlb;
@@ -32,6 +33,7 @@ struct ConvParams {
     int T, A, C, taps, act;
     int* error_flag;
     int run = 1;               // tokens a thread of the four-channel kernel walks
+    int move = 0;              // 1: every sequence brings one token, whose thread moves the state on
     const float* bias = nullptr;   // [C] or null
 };
 
@@ -59,7 +61,13 @@ __global__ void short_conv_kernel(ConvParams p) {
         const int src = local - hist + j;              // index among this step's tokens of the sequence
         float u = 0.0f;
         if (src >= 0) u = input_at(p, (long long)start + src, c);
-        else if (pos0 + src >= 0 && slot_ok) u = p.state[((size_t)slot * hist + (hist + src)) * p.C + c];
+        else if (slot_ok) {
+            float* const st = p.state + ((size_t)slot * hist + (hist + src)) * p.C + c;
+            const float was = *st;
+            if (pos0 + src >= 0) u = was;
+            if (p.move && j > 0) st[-(ptrdiff_t)p.C] = was;           // (local is 0: j is the place in the state)
+        }
+        if (p.move && j == hist && slot_ok) p.state[((size_t)slot * hist + hist - 1) * p.C + c] = u;
         acc = fmaf(p.w[(size_t)c * p.taps + j], u, acc);
     }
     if (p.bias) acc += p.bias[c];
@@ -76,6 +84,7 @@ constexpr int CONV_RUN = 8;            // for steps of many tokens; a thread of 
 __device__ __forceinline__ float4 conv_row(const ConvParams& p, long long row, int c) {
     const float* at = p.u + row * p.ld + p.col0 + c;
     float4 u = *reinterpret_cast<const float4*>(at);
+#pragma unroll 4
     for (int k = 1; k < p.n_partials; ++k) {
         const float4 more = *reinterpret_cast<const float4*>(at + (size_t)k * p.partial_stride);
         u.x += more.x; u.y += more.y; u.z += more.z; u.w += more.w;
@@ -83,7 +92,8 @@ __device__ __forceinline__ float4 conv_row(const ConvParams& p, long long row, i
     return u;
 }
 
-template <int TAPS>
+// ONE: the thread's only token is its sequence's only one (p.move): its earlier inputs all come from the state, none from the rows above.
+template <int TAPS, bool ONE>
 __global__ void short_conv_x4_kernel(ConvParams p) {
     pdl_launch_dependents();
     constexpr int HIST = TAPS - 1;
@@ -94,12 +104,46 @@ __global__ void short_conv_x4_kernel(ConvParams p) {
     const int c = active ? (int)(i % C4) * 4 : 0;
     float wreg[4 * TAPS];               // the weights are never written by a kernel: fetched before the wait for the predecessor
 #pragma unroll
-    for (int k = 0; k < 4 * TAPS; ++k) wreg[k] = p.w[(size_t)c * TAPS + k];
+    for (int k = 0; k < TAPS; ++k) {    // (four channels' taps are 4 * TAPS neighbours)
+        const float4 w = *reinterpret_cast<const float4*>(p.w + (size_t)c * TAPS + 4 * k);
+        wreg[4 * k] = w.x; wreg[4 * k + 1] = w.y; wreg[4 * k + 2] = w.z; wreg[4 * k + 3] = w.w;
+    }
     const float4 shift = p.bias ? *reinterpret_cast<const float4*>(p.bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int t0 = active ? (int)(i / C4) * p.run : 0;
+    float4 win[HIST > 0 ? HIST : 1];    // rows t - HIST .. t - 1 of the flat batch, as they are
+    if (ONE) {
+        // the lists are older than the step's kernels; the state was written a step ago, by this kernel
+        const int a = p.token_seq[t0], pos0 = p.seq_pos0[a], slot = p.slots[a];
+        const bool slot_ok = slot >= 0 && slot < p.num_slots;
+        pdl_wait();
+        if (!active) return;
+        if (!slot_ok && p.error_flag) atomicExch(p.error_flag, 3);
+        float* const st = p.state + (size_t)(slot_ok ? slot : 0) * HIST * p.C + c;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < HIST; ++j) win[j] = slot_ok ? *reinterpret_cast<const float4*>(st + (size_t)j * p.C) : zero;
+        const float4 now = conv_row(p, t0, c);
+        float4 acc = make_float4(wreg[HIST] * now.x, wreg[TAPS + HIST] * now.y, wreg[2 * TAPS + HIST] * now.z, wreg[3 * TAPS + HIST] * now.w);
+#pragma unroll
+        for (int j = 0; j < HIST; ++j) {
+            const float4 u = pos0 - HIST + j >= 0 ? win[j] : zero;
+            acc.x = fmaf(wreg[j], u.x, acc.x); acc.y = fmaf(wreg[TAPS + j], u.y, acc.y);
+            acc.z = fmaf(wreg[2 * TAPS + j], u.z, acc.z); acc.w = fmaf(wreg[3 * TAPS + j], u.w, acc.w);
+        }
+        acc.x += shift.x; acc.y += shift.y; acc.z += shift.z; acc.w += shift.w;
+        if (p.act == 1) {
+            acc.x = acc.x / (1.0f + expf(-acc.x)); acc.y = acc.y / (1.0f + expf(-acc.y));
+            acc.z = acc.z / (1.0f + expf(-acc.z)); acc.w = acc.w / (1.0f + expf(-acc.w));
+        }
+        *reinterpret_cast<float4*>(p.y + (size_t)t0 * p.ldy + c) = acc;
+        if (slot_ok) {
+#pragma unroll
+            for (int j = 0; j < HIST; ++j) *reinterpret_cast<float4*>(st + (size_t)j * p.C) = j + 1 < HIST ? win[j + 1 < HIST ? j + 1 : 0] : now;
+        }
+        return;
+    }
     pdl_wait();
     if (!active) return;
-    const int t0 = (int)(i / C4) * p.run;
-    float4 win[HIST > 0 ? HIST : 1];    // rows t - HIST .. t - 1 of the flat batch, as they are
 #pragma unroll
     for (int m = 0; m < HIST; ++m) win[m] = t0 - HIST + m >= 0 ? conv_row(p, t0 - HIST + m, c) : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int t = t0; t < min(t0 + p.run, p.T); ++t) {
@@ -177,7 +221,7 @@ int check(const ConvParams& p, const char* what) {
 
 MLB_EXPORT int mlb_short_conv(const float* u, long long ld, int n_partials, long long partial_stride, int col0, const float* w,
                               const float* bias, float* state, const int* slots, int num_slots, const int* seq_starts, const int* seq_pos0,
-                              const int* token_seq, float* y, long long ldy, int T, int A, int C, int taps, int act,
+                              const int* token_seq, float* y, long long ldy, int T, int A, int C, int taps, int act, int move,
                               int* error_flag, cudaStream_t stream) {
     ConvParams p{u, ld, n_partials, partial_stride, col0, w, state, slots, num_slots, seq_starts, seq_pos0, token_seq, y, ldy,
                  T, A, C, taps, act, error_flag};
@@ -185,17 +229,26 @@ MLB_EXPORT int mlb_short_conv(const float* u, long long ld, int n_partials, long
     p.bias = bias;
     if (!y) return fail(MLB_INVALID_ARGUMENT, "short_conv: null output");
     if (T == 0) return MLB_OK;
+    if (move && (T != A || taps == 1)) return fail(MLB_INVALID_ARGUMENT, "short_conv: only steps of one token a sequence move the state themselves");
     const long long n = (long long)T * C;
     const bool x4 = C % 4 == 0 && ld % 4 == 0 && ldy % 4 == 0 && col0 % 4 == 0 && partial_stride % 4 == 0 &&
-                    ((uintptr_t)u | (uintptr_t)y | (uintptr_t)state | (uintptr_t)bias) % 16 == 0;
-    p.run = T >= 64 * CONV_RUN ? CONV_RUN : 1;
+                    ((uintptr_t)u | (uintptr_t)y | (uintptr_t)state | (uintptr_t)bias | (uintptr_t)w) % 16 == 0;
+    p.move = move;
+    p.run = !move && T >= 64 * CONV_RUN ? CONV_RUN : 1;
     const long long x4_threads = ((long long)T + p.run - 1) / p.run * (C / 4);
     const unsigned x4_blocks = (unsigned)((x4_threads + 127) / 128);
-    if (x4 && taps == 2) launch_kernel(short_conv_x4_kernel<2>, x4_blocks, 128, 0, stream, p);
-    else if (x4 && taps == 3) launch_kernel(short_conv_x4_kernel<3>, x4_blocks, 128, 0, stream, p);
-    else if (x4 && taps == 4) launch_kernel(short_conv_x4_kernel<4>, x4_blocks, 128, 0, stream, p);
-    else if (x4 && taps == 5) launch_kernel(short_conv_x4_kernel<5>, x4_blocks, 128, 0, stream, p);
-    else launch_kernel(short_conv_kernel, (unsigned)((n + 255) / 256), 256, 0, stream, p);
+    auto go = [&](auto several, auto one) {
+        if (move) launch_kernel(one, x4_blocks, 128, 0, stream, p);
+        else launch_kernel(several, x4_blocks, 128, 0, stream, p);
+    };
+    if (x4 && taps >= 2 && taps <= 5) {
+        if (taps == 2) go(short_conv_x4_kernel<2, false>, short_conv_x4_kernel<2, true>);
+        else if (taps == 3) go(short_conv_x4_kernel<3, false>, short_conv_x4_kernel<3, true>);
+        else if (taps == 4) go(short_conv_x4_kernel<4, false>, short_conv_x4_kernel<4, true>);
+        else go(short_conv_x4_kernel<5, false>, short_conv_x4_kernel<5, true>);
+    } else {
+        launch_kernel(short_conv_kernel, (unsigned)((n + 255) / 256), 256, 0, stream, p);
+    }
     return check_launch("short_conv");
 }
 

@@ -17,7 +17,7 @@ MAX_WIDTH = 256
 
 ops.register_signatures("short_conv.cu", {
     "mlb_short_conv": [c_void_p, c_longlong, c_int, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "mlb_short_conv_state": [c_void_p, c_longlong, c_int, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
                              c_int, c_void_p],
 })
@@ -67,10 +67,11 @@ def short_conv(u: torch.Tensor, col0: int, weight: torch.Tensor, state: Optional
             raise KernelError(f"short_conv: the state must be [slots, {taps - 1}, {C}], got {tuple(state.shape)}")
         num_slots = state.shape[0]
     L = ops.lib("short_conv.cu")
+    move = taps > 1 and update_state and T == ctx.num_seqs          # one token a sequence: the same launch moves the state on
     build.check(L, L.mlb_short_conv(u.data_ptr(), ld, n, stride, col0, weight.data_ptr(), ops._ptr(bias), ops._ptr(state), slots.data_ptr(), num_slots,
                                     ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), ctx.token_seq.data_ptr(), out.data_ptr(),
-                                    out.shape[1], T, ctx.num_seqs, C, taps, 1 if silu else 0, ops._ptr(ctx.error_flag), ops._stream()))
-    if taps > 1 and update_state:
+                                    out.shape[1], T, ctx.num_seqs, C, taps, 1 if silu else 0, 1 if move else 0, ops._ptr(ctx.error_flag), ops._stream()))
+    if taps > 1 and update_state and not move:
         build.check(L, L.mlb_short_conv_state(u.data_ptr(), ld, n, stride, col0, state.data_ptr(), slots.data_ptr(), num_slots,
                                               ctx.seq_starts.data_ptr(), ctx.num_seqs, C, taps, ops._stream()))
 

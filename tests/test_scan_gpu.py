@@ -1,4 +1,5 @@
-"""The recurrences' scan kernel with one and with two columns a lane (scan_per_lane in csrc/delta_rule.cu): a row's bits do not depend on it."""
+"""The recurrences' scan kernel with one and with two columns a lane (scan_per_lane in csrc/delta_rule.cu), and the convolution whose one token a
+sequence moves the state on itself: what a row's bits are depends on neither."""
 import pytest
 import torch
 
@@ -60,3 +61,27 @@ def test_many_sequences_have_the_bits_of_each_alone(rule, dk, dv, alike):
         assert torch.equal(together[0][at:at + counts[a]], o) and torch.equal(together[1][a], state[0])
         assert torch.equal(together[2][a], n_state[0]) and torch.equal(together[3][at:at + counts[a]], den)
         at += counts[a]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("taps, C", [(2, 12), (3, 260), (4, 1024), (5, 8), (4, 37), (7, 20)])
+@pytest.mark.parametrize("partials", [1, 6])
+def test_one_token_a_sequence_moves_the_state_on(taps, C, partials):
+    """Steps of one token a sequence, and the same tokens in one portion: the same bits and the same state behind them."""
+    from microllm_rocm_b200.kernels import recurrent
+    A, n = 5, 9
+    g = torch.Generator(DEV).manual_seed(C)
+    u = torch.randn(partials, A, n, C + 8, generator=g, device=DEV)
+    w, bias = torch.randn(C, taps, generator=g, device=DEV), torch.randn(C, generator=g, device=DEV)
+    held = torch.randn(A + 1, taps - 1, C, generator=g, device=DEV)
+    pos0 = [0, 1, 2, 5, 40]
+    one, whole = held.clone(), held.clone()
+    ctx, slots = step([n] * A, pos0)
+    want = torch.empty(A * n, C, device=DEV)
+    recurrent.short_conv(u.reshape(partials, A * n, C + 8), 4, w, whole, slots, ctx, want, silu=True, bias=bias)
+    for t in range(n):
+        ctx, slots = step([1] * A, [p + t for p in pos0])
+        got = torch.empty(A, C, device=DEV)
+        recurrent.short_conv(u[:, :, t].contiguous(), 4, w, one, slots, ctx, got, silu=True, bias=bias)
+        assert torch.equal(got, want.view(A, n, C)[:, t]) and int(ctx.error_flag.item()) == 0, t
+    assert torch.equal(one, whole)
