@@ -359,7 +359,7 @@ def library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
         N = weight.shape[0]
         if out is None:
             out = alloc((M, N), out_dtype) if alloc is not None else torch.empty((M, N), dtype=out_dtype, device=x.device)
-        key = str(x.device)
+        key = (str(x.device), ops.on_second_stream())          # products of the two streams may run at once
         work = _workspaces.get(key)
         if work is None:
             work = _workspaces[key] = torch.empty(LIBRARY_WORKSPACE_BYTES, dtype=torch.uint8, device=x.device)

@@ -699,6 +699,11 @@ def on_side_stream():
         _launch_on.side = outer
 
 
+def on_second_stream() -> bool:
+    """Whether this thread's launches go to the second stream just now."""
+    return getattr(_launch_on, "side", None) is not None
+
+
 def stream_synchronize() -> None:
     L = lib("basic.cu")
     status = L.mlb_stream_synchronize(_stream())

@@ -268,6 +268,12 @@ class Mixer(Part):
         """PagedKVNeed, FixedStateNeed or None."""
         return None
 
+    def beside_others(self) -> bool:
+        """Whether forward() may run on the device's second stream while another mixer runs on the first (ops.on_side_stream): it
+        launches this library's kernels and direct library products only, plans nothing that has to be uploaded, and uses the second
+        stream for nothing itself."""
+        return False
+
     def forward(self, x: torch.Tensor, ctx: StepContext, cache) -> torch.Tensor:
         raise NotImplementedError
 

@@ -121,6 +121,9 @@ class GatedDeltaRule(Mixer):
     def own_tensors(self):
         return [self.w_in, self.w_o, self.w_conv, self.w_a2, self.w_g2, self.a_log, self.dt_bias, self.norm_w]
 
+    def beside_others(self) -> bool:
+        return self.rt.is_fp32 or gemm_bf16._direct_library(self.rt.device)
+
     # --- compute ------------------------------------------------------------------------
     def forward(self, x: torch.Tensor, ctx: StepContext, cache) -> torch.Tensor:
         T, flag, f32 = x.shape[0], ctx.error_flag, torch.float32

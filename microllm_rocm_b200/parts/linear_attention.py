@@ -99,6 +99,9 @@ class GatedLinearAttention(Mixer):
         self.w_in = tensors["in_proj.weight"] if "in_proj.weight" in tensors else torch.cat([tensors[name] for name, _ in self._pieces()], 0).contiguous()
         self.w_a2, self.a_bias, self.norm_w, self.w_o = tensors[n["a2"]], tensors[n["a_bias"]], tensors[n["norm"]], tensors[n["o"]]
 
+    def beside_others(self) -> bool:
+        return self.rt.is_fp32 or gemm_bf16._direct_library(self.rt.device)
+
     def replay_key(self):
         if not self.rt.is_fp32 and not gemm_bf16._direct_library(self.rt.device):
             return None
@@ -179,6 +182,9 @@ class LightningAttention(Mixer):
         n = self.names
         self.w_in = tensors["in_proj.weight"] if "in_proj.weight" in tensors else torch.cat([tensors[name] for name, _ in self._pieces()], 0).contiguous()
         self.norm_w, self.w_o = tensors[n["norm"]], tensors[n["o"]]
+
+    def beside_others(self) -> bool:
+        return self.rt.is_fp32 or gemm_bf16._direct_library(self.rt.device)
 
     def replay_key(self):
         if not self.rt.is_fp32 and not gemm_bf16._direct_library(self.rt.device):

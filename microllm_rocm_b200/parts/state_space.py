@@ -96,6 +96,9 @@ class SelectiveStateSpace(Mixer):
     def own_tensors(self):
         return [self.w_in, self.w_o, self.w_conv, self.b_conv, self.dt_bias, self.a_log, self.d, self.norm_w]
 
+    def beside_others(self) -> bool:
+        return self.rt.is_fp32 or gemm_bf16._direct_library(self.rt.device)
+
     # --- compute ------------------------------------------------------------------------
     def forward(self, x: torch.Tensor, ctx: StepContext, cache) -> torch.Tensor:
         T, flag, f32 = x.shape[0], ctx.error_flag, torch.float32

@@ -85,3 +85,41 @@ def test_one_token_a_sequence_moves_the_state_on(taps, C, partials):
         recurrent.short_conv(u[:, :, t].contiguous(), 4, w, one, slots, ctx, got, silu=True, bias=bias)
         assert torch.equal(got, want.view(A, n, C)[:, t]) and int(ctx.error_flag.item()) == 0, t
     assert torch.equal(one, whole)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("family, dtype", [("matidra", "float32"), ("matidra", "bfloat16"), ("naburax", "float32"), ("lozepel", "bfloat16"), ("fonuvik", "bfloat16")])
+def test_branches_side_by_side_have_the_bits_of_one_after_another(tmp_path, family, dtype):
+    """A prompt, a step that decodes beside a prompt portion, and decoded tokens."""
+    from microllm_rocm_b200.config import find_preset
+    from microllm_rocm_b200.engine.loading import make_engine, prepare_kernels, require_gpu, resolve_dtype
+    from microllm_rocm_b200.engine.step import StepEntry
+    from microllm_rocm_b200.parts import parallel
+    from microllm_rocm_b200.parts.base import Runtime
+    from microllm_rocm_b200.parts.build import build_model
+    arch, cfg = find_preset(family + "-tiny")
+    results = []
+    for side in (False, True):
+        parallel.SIDE_BY_SIDE = side
+        try:
+            model = build_model(arch.build_spec(cfg), Runtime(require_gpu(), resolve_dtype(dtype)))
+            prepare_kernels(model)
+            g = torch.Generator(DEV).manual_seed(1)
+            made = {}
+            for name, spec in model.expected_tensors().items():
+                t = torch.randn(tuple(spec.shape), generator=g, device=DEV) * 0.1 + (1.0 if "norm" in name else 0.0)
+                made[name] = t if spec.role == "vector" else t.to(resolve_dtype(dtype))
+            model.bind(made)
+            engine = make_engine(model, 16, 32, 4)
+            out = []
+            for rid in "ab":
+                engine.cache.add(rid)
+            out.append(engine.step([StepEntry("a", list(range(5, 50)), [44])]).clone())
+            out.append(engine.step([StepEntry("a", [9], [0]), StepEntry("b", list(range(40, 60)), [19])]).clone())
+            for t in range(3):
+                out.append(engine.step([StepEntry("a", [t], [0]), StepEntry("b", [t + 7], [0])]).clone())
+            engine.check_device_errors()
+            results.append(torch.cat(out))
+        finally:
+            parallel.SIDE_BY_SIDE = True
+    assert torch.equal(results[0], results[1]) and bool(torch.isfinite(results[0]).all())
