@@ -184,15 +184,16 @@ gemm_f32_stream_kernel(const float* __restrict__ A, const float* __restrict__ W,
 // ------------------------------------------------------------------------------------------------------- many rows of A
 // Rows of a stage lie 36 floats apart: eight neighbouring rows' same piece fall into eight different groups of banks.  Per four
 // elements of K a thread reads 8 + 4 pieces and issues 64 packed FMAs, so the FMA pipe and not shared memory is the limit.
-constexpr int BM = 64, BN = 64, TILE_STAGES = 3, PITCH = STEP + 4;
-constexpr int STAGE_FLOATS = (BM + BN) * PITCH;
-constexpr int TILE_SMEM = TILE_STAGES * STAGE_FLOATS * 4;
+constexpr int BN = 64, TILE_STAGES = 3, PITCH = STEP + 4;
+constexpr int stage_floats(int ri) { return (8 * ri + BN) * PITCH; }
+constexpr int tile_smem(int ri) { return TILE_STAGES * stage_floats(ri) * 4; }
 
-template <bool VEC, bool ACCUMULATE>
+template <int RI, bool VEC, bool ACCUMULATE>
 __global__ void __launch_bounds__(128)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ C, int M, int N, int K, long long lda, long long ldw, long long ldc, int w_constant) {
     extern __shared__ __align__(128) float tiles[];
+    constexpr int BM = 8 * RI, STAGE_FLOATS = stage_floats(RI);
     pdl_prologue();
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -210,7 +211,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         const int k = k_base + step * STEP + piece * 4;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            copy_piece<VEC>(base + (row + 16 * i) * (PITCH * 4), A + (size_t)min(m0 + row + 16 * i, M - 1) * lda, k, K);
+            if (row + 16 * i < BM) copy_piece<VEC>(base + (row + 16 * i) * (PITCH * 4), A + (size_t)min(m0 + row + 16 * i, M - 1) * lda, k, K);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             copy_piece<VEC>(base + (BM + row + 16 * i) * (PITCH * 4), W + (size_t)min(n0 + row + 16 * i, N - 1) * ldw, k, K);
@@ -219,12 +220,12 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         if (s < steps) load(s);
         commit();
     }
-    const int ty = lane >> 3, tx = lane & 7;                              // rows ty + 4 i, columns tx + 8 j of the warp's 32 x 32
-    const int a_row = (warp >> 1) * 32 + ty, w_row = (warp & 1) * 32 + tx;
-    unsigned long long acc[8][4];
-    float sum[8][4];
+    const int ty = lane >> 3, tx = lane & 7;                              // rows ty + 4 i, columns tx + 8 j of the warp's 4 RI x 32
+    const int a_row = (warp >> 1) * (4 * RI) + ty, w_row = (warp & 1) * 32 + tx;
+    unsigned long long acc[RI][4];
+    float sum[RI][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) { acc[i][j] = 0ull; sum[i][j] = 0.0f; }
     int in_range = 0;
@@ -241,7 +242,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 #pragma unroll
             for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_base + 8 * j * PITCH + 4 * p);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < RI; ++i) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_base + 4 * i * PITCH + 4 * p);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { fma2(acc[i][j], a.x, w[j].x); fma2(acc[i][j], a.y, w[j].y); }
@@ -250,7 +251,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         if (++in_range == per_range || step + 1 == steps) {
             in_range = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { sum[i][j] += chains(acc[i][j]); acc[i][j] = 0ull; }
         }
@@ -260,7 +261,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     constexpr int OUT_PITCH = BN + 4;
     float* mine = tiles;                                                  // the quarter's 64 x 64 sums, over the ring
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) mine[(a_row + 4 * i) * OUT_PITCH + w_row + 8 * j] = sum[i][j];
     cluster.sync();
@@ -311,15 +312,24 @@ int launch_stream(const Call& c) {
     return check_launch("gemm_f32_stream");
 }
 
-template <bool VEC, bool ACCUMULATE>
+// Eighths of a tile's rows: equal tiles of at most 64 rows, five to eight for more than STREAM_MAX_M.  A last tile of 64 rows that holds 13
+// (333 rows) takes as long as a full one: six of 56 take 945 us where six of 64 take 1,061 (the four products of a layer of the 1.5B
+// shape; 33 rows 195 / 264, 65 305 / 432, 200 625 / 704, 500 and 1,000 the same).
+int tile_rows(int M) {
+    const int count = (M + 63) / 64;
+    return ((M + count - 1) / count + 7) / 8;
+}
+
+template <int RI, bool VEC, bool ACCUMULATE>
 int launch_tile(const Call& c) {
     static bool done[MAX_DEVICES] = {};
-    auto kernel = gemm_f32_tile_kernel<VEC, ACCUMULATE>;
-    if (int status = set_smem(kernel, TILE_SMEM, done)) return status;
+    auto kernel = gemm_f32_tile_kernel<RI, VEC, ACCUMULATE>;
+    constexpr int smem = tile_smem(RI);
+    if (int status = set_smem(kernel, smem, done)) return status;
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((c.N + BN - 1) / BN * QUARTERS, (c.M + BM - 1) / BM);
+    config.gridDim = dim3((c.N + BN - 1) / BN * QUARTERS, (c.M + 8 * RI - 1) / (8 * RI));
     config.blockDim = 128;
-    config.dynamicSmemBytes = TILE_SMEM;
+    config.dynamicSmemBytes = smem;
     config.stream = c.stream;
     cudaLaunchAttribute attributes[2];
     attributes[0].id = cudaLaunchAttributeClusterDimension;
@@ -340,7 +350,12 @@ int launch(const Call& c) {
     if (c.M <= 4) return launch_stream<4, 1, VEC, ACCUMULATE>(c);
     if (c.M <= 8) return launch_stream<8, 2, VEC, ACCUMULATE>(c);
     if (c.M <= STREAM_MAX_M) return launch_stream<16, 2, VEC, ACCUMULATE>(c);
-    return launch_tile<VEC, ACCUMULATE>(c);
+    switch (tile_rows(c.M)) {
+        case 5: return launch_tile<5, VEC, ACCUMULATE>(c);
+        case 6: return launch_tile<6, VEC, ACCUMULATE>(c);
+        case 7: return launch_tile<7, VEC, ACCUMULATE>(c);
+        default: return launch_tile<8, VEC, ACCUMULATE>(c);
+    }
 }
 
 }  // namespace
@@ -353,7 +368,7 @@ MLB_EXPORT int mlb_gemm_f32(const float* A, const float* W, const float* bias, f
     if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N)
         return fail(MLB_INVALID_ARGUMENT, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return MLB_OK;
-    if ((M + BM - 1) / BM > 65535) return fail(MLB_UNSUPPORTED_SIZE, "gemm_f32: M=%d exceeds %d rows per call", M, 65535 * BM);
+    if ((M + 63) / 64 > 65535) return fail(MLB_UNSUPPORTED_SIZE, "gemm_f32: M=%d exceeds %d rows per call", M, 65535 * 64);
     const Call c{A, W, bias, C, M, N, K, lda, ldw, ldc, w_constant, stream};
     const bool vec = lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
     if (vec) return accumulate ? launch<true, true>(c) : launch<true, false>(c);
