@@ -138,19 +138,95 @@ __device__ __forceinline__ void store_cache_row(const PrepareParams& p, int t, s
     normed_row(p, row, p.kv_col, p.rank, p.norm_weight, w, v, scratch, cache_row);
 }
 
-template <typename QT, typename KVT>
+// four neighbouring columns of the projection (partial results added up in split order), and four values on their way out
+__device__ __forceinline__ float4 proj4_at(const PrepareParams& p, size_t row_base, long long col) {
+    const float* at = p.proj + row_base + col;
+    float4 v = *reinterpret_cast<const float4*>(at);
+#pragma unroll 4
+    for (int k = 1; k < p.n_partials; ++k) {
+        at += p.partial_stride;
+        const float4 u = *reinterpret_cast<const float4*>(at);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    return v;
+}
+__device__ __forceinline__ void store4(float* to, float4 v) { *reinterpret_cast<float4*>(to) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* to, float4 v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+}
+
+// VEC: four columns a thread, two such pieces asked for together, where every piece of a row starts on four elements and is a multiple of
+// four long (pairs that are half a rotated part apart then lie in two pieces).  The token's cosines and sines, the same for
+// every head, are made once a block, while the kernel in front ends.  16 heads of 128 + 64 with a latent of 512, us, a column
+// a thread / so: 2,048 tokens 31 / 20, with a gate 43 / 29, two partial sums 40 / 26; 8 tokens of four partial sums 4.6 / 3.5.
+constexpr int SLICE_VEC = 2048, MAX_PAIRS = 320;
+template <typename QT, typename KVT, bool VEC>
 __global__ void __launch_bounds__(256)
 latent_prepare_kernel(PrepareParams p) {
     pdl_launch_dependents();
     float w[ROW_PER];
     fetch_weight(p.pages && blockIdx.y == 0 ? p.norm_weight : nullptr, p.rank, w);
-    pdl_wait();
     __shared__ float scratch[32];
+    __shared__ float2 turn_s[VEC ? MAX_PAIRS : 1];
     const int t = blockIdx.x;
     const size_t row = (size_t)t * p.ld;
-    const int pos = p.positions[t];
+    const int pos = p.positions[t];                  // (older than the step's kernels)
     const int half = p.rot_dims / 2;
     const int Dk = p.rank + p.rot_dim;
+    if (VEC && blockIdx.y > 0) {
+        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            const float angle = (float)pos * p.inv_freq[i];
+            turn_s[i] = make_float2(cosf(angle) * p.magnitude, sinf(angle) * p.magnitude);
+        }
+        __syncthreads();
+        pdl_wait();
+        const int per_head = p.dim + p.rot_dim, q_cols = p.heads * per_head;
+        const int lo = (blockIdx.y - 1) * SLICE_VEC, hi = min(lo + SLICE_VEC, q_cols + (p.gate_out ? p.gate_width : 0));
+        float4 v[2], o[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int e = lo + 4 * (threadIdx.x + k * blockDim.x);
+            if (e >= hi) continue;
+            v[k] = proj4_at(p, row, e >= q_cols ? p.gate_col + e - q_cols : p.q_col + e);
+            const int r = e % per_head - p.dim;
+            if (e < q_cols && r >= 0 && r < p.rot_dims && !p.interleaved) o[k] = proj4_at(p, row, p.q_col + e - r + pair_of(r, half, 0).other);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int e = lo + 4 * (threadIdx.x + k * blockDim.x);
+            if (e >= hi) continue;
+            if (e >= q_cols) {                                   // the gate's sigmoid
+                const float4 z = v[k];
+                store4(p.gate_out + (size_t)t * p.gate_width + e - q_cols,
+                       make_float4(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)), 1.0f / (1.0f + expf(-z.z)), 1.0f / (1.0f + expf(-z.w))));
+                continue;
+            }
+            // queries: plain parts to q_plain, rotated parts into the tail of each head's row of q_full
+            const int h = e / per_head, i = e % per_head, r = i - p.dim;
+            if (r < 0) {
+                store4((QT*)p.q_plain + ((size_t)t * p.heads + h) * p.dim + i, v[k]);
+                continue;
+            }
+            float4 out = v[k];
+            if (r < p.rot_dims) {
+                // (as turned() is contracted)
+                auto turn = [](float x, float other, bool first, float2 cs) { return fmaf(x, cs.x, __fmul_rn(first ? -other : other, cs.y)); };
+                if (p.interleaved) {                             // two pairs in this piece
+                    const float2 a = turn_s[r >> 1], c = turn_s[(r >> 1) + 1];
+                    out = make_float4(turn(v[k].x, v[k].y, true, a), turn(v[k].y, v[k].x, false, a), turn(v[k].z, v[k].w, true, c), turn(v[k].w, v[k].z, false, c));
+                } else {                                         // four pairs, their other elements in the piece half a rotated part away
+                    const Pair pr = pair_of(r, half, 0);
+                    const float2* cs = turn_s + pr.index;
+                    out = make_float4(turn(v[k].x, o[k].x, pr.first, cs[0]), turn(v[k].y, o[k].y, pr.first, cs[1]), turn(v[k].z, o[k].z, pr.first, cs[2]),
+                                      turn(v[k].w, o[k].w, pr.first, cs[3]));
+                }
+            }
+            store4((QT*)p.q_full + ((size_t)t * p.heads + h) * Dk + p.rank + r, out);
+        }
+        return;
+    }
+    pdl_wait();
 
     // blockIdx.y == 0: the token's cache row; blockIdx.y >= 1: a slice of SLICE query and gate columns
     if (blockIdx.y > 0) {
@@ -315,12 +391,18 @@ MLB_EXPORT int mlb_latent_prepare(const float* proj, long long ld, int n_partial
                     block_table, max_blocks, inv_freq, rot_dims, interleaved, magnitude, q_plain, q_full, pages, gate_out, num_pages, page_size,
                     tokens, heads, dim, rot_dim, rank, gate_width, error_flag, 0, 0, nullptr, nullptr};
     const int columns = heads * (dim + rot_dim) + (gate_out ? gate_width : 0);
-    const dim3 grid(tokens, 1 + (columns + SLICE - 1) / SLICE);
-    if (q_dtype == MLB_F32 && (kv_dtype == MLB_F32 || !pages))
-        launch_kernel(latent_prepare_kernel<float, float>, grid, 256, 0, stream, p);
-    else if (q_dtype == MLB_BF16 && (kv_dtype == MLB_BF16 || !pages))
-        launch_kernel(latent_prepare_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream, p);
-    else
+    const bool vec = rot_dims <= 2 * MAX_PAIRS && dim % 4 == 0 && rot_dim % 4 == 0 && rot_dims % (interleaved ? 4 : 8) == 0 && rank % 4 == 0 && ld % 4 == 0 && partial_stride % 4 == 0 &&
+                     q_col % 4 == 0 && gate_col % 4 == 0 && gate_width % 4 == 0 &&
+                     (((uintptr_t)proj | (uintptr_t)q_plain | (uintptr_t)q_full | (uintptr_t)gate_out) & 15) == 0;
+    const int slice = vec ? SLICE_VEC : SLICE;
+    const dim3 grid(tokens, 1 + (columns + slice - 1) / slice);
+    if (q_dtype == MLB_F32 && (kv_dtype == MLB_F32 || !pages)) {
+        if (vec) launch_kernel(latent_prepare_kernel<float, float, true>, grid, 256, 0, stream, p);
+        else launch_kernel(latent_prepare_kernel<float, float, false>, grid, 256, 0, stream, p);
+    } else if (q_dtype == MLB_BF16 && (kv_dtype == MLB_BF16 || !pages)) {
+        if (vec) launch_kernel(latent_prepare_kernel<__nv_bfloat16, __nv_bfloat16, true>, grid, 256, 0, stream, p);
+        else launch_kernel(latent_prepare_kernel<__nv_bfloat16, __nv_bfloat16, false>, grid, 256, 0, stream, p);
+    } else
         return fail(MLB_INVALID_ARGUMENT, "latent_prepare: unsupported dtypes %d / %d", q_dtype, kv_dtype);
     return check_launch("latent_prepare");
 }

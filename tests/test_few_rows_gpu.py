@@ -1,4 +1,5 @@
-"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, the split of latent attention's projection."""
+"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, per-head products of few rows, the split of
+latent attention's projection."""
 import pytest
 import torch
 
@@ -20,3 +21,54 @@ def test_fp32_rows_have_the_bits_of_a_row_alone(M, N, K):
         ops.gemm_f32(x[m:m + 1].contiguous(), w, row, bias=bias)
         assert torch.equal(out[m:m + 1], row), m
     assert bool(torch.isfinite(out).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("groups, N, K, factor", [(16, 512, 128, False), (16, 128, 512, True), (3, 40, 96, True), (5, 17, 32, False), (2, 64, 1056, True)])
+def test_per_head_products_of_few_rows(rows, groups, N, K, factor):
+    from microllm_rocm_b200.kernels import grouped
+    g = torch.Generator(DEV).manual_seed(N + K)
+    a = torch.randn(rows, groups * K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(groups, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    by = torch.rand(rows, groups * (N + 8), generator=g, device=DEV) if factor else None
+    out = torch.full((rows, groups * (N + 8)), 7.0, dtype=torch.bfloat16, device=DEV)          # (eight columns a group that nobody writes)
+    assert grouped.few_rows(a, w, out, rows, K) and not grouped.few_rows(a, w, out, 17, K)
+    grouped.grouped_linear(a, w, out, rows=rows, a_group_cols=K, c_group_cols=N + 8, factor=by, row_tile=16)
+    want = torch.einsum("mgk,gnk->mgn", a.double().view(rows, groups, K), w.double())
+    if factor:
+        want = want * by.double().view(rows, groups, N + 8)[..., :N]
+    got = out.view(rows, groups, N + 8)
+    assert bool((got[..., N:] == 7.0).all())
+    # the result's rounding, half a unit of eight bits, and fp32 sums of K products
+    assert bool(((got[..., :N].double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, dim, rot, rot_dims, interleaved, partials", [(3, 128, 64, 64, False, 1), (16, 128, 64, 32, False, 5), (5, 32, 16, 8, True, 3), (2, 64, 64, 64, True, 1)])
+def test_the_split_of_a_projection_four_columns_at_a_time(dtype, heads, dim, rot, rot_dims, interleaved, partials):
+    """Rows that start on 16 bytes go four columns a thread, the same rows one column further on do not: the same bits."""
+    from microllm_rocm_b200.kernels import latent
+    rank, T, page = 64, 9, 4
+    width = heads * (dim + rot) + rank + rot + heads * 32
+    g = torch.Generator(DEV).manual_seed(dim + rot_dims)
+    proj = torch.randn(partials, T, width, generator=g, device=DEV)
+    norm, freq = torch.rand(rank, generator=g, device=DEV), torch.rand(rot_dims // 2, generator=g, device=DEV)
+    on = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    positions, seq, table = on([0, 1, 2, 900, 901, 902, 5, 6, 7]), on([0] * 3 + [1] * 3 + [2] * 3), torch.full((3, 226), -1, dtype=torch.int32, device=DEV)
+    table[0, 0], table[1, 225], table[2, 1] = 3, 1, 0
+    results = []
+    for shift in (0, 1):
+        src = torch.zeros(partials, T, width + 4, device=DEV)
+        src[..., shift:shift + width] = proj
+        q_plain, q_full = torch.zeros(T, heads * dim, dtype=dtype, device=DEV), torch.zeros(T, heads * (rank + rot), dtype=dtype, device=DEV)
+        gate, pages = torch.zeros(T, heads * 32, device=DEV), torch.zeros(4, page, rank + rot, dtype=dtype, device=DEV)
+        flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+        latent.prepare(src, q_col=shift, kv_col=shift + heads * (dim + rot), gate_col=shift + heads * (dim + rot) + rank + rot, norm_weight=norm, eps=1e-5,
+                       positions=positions, token_seq=seq, block_table=table, inv_freq=freq, rot_dims=rot_dims, q_plain=q_plain, q_full=q_full, pages=pages,
+                       gate_out=gate, heads=heads, dim=dim, rot_dim=rot, rank=rank, error_flag=flag, interleaved=interleaved, magnitude=1.25)
+        results.append((q_plain, q_full, gate, pages))
+        assert int(flag.item()) == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b) and bool((a != 0).any())
