@@ -83,7 +83,9 @@ grouped_mma_kernel(MmaParams p) {
     constexpr int WN = BN / WARPS_N;                 // columns per warp: 32, 64 or 16
     constexpr int NT = WN / 8;                       // n-tiles per warp: 4, 8 or 2
     constexpr int NB = DUAL ? 2 : 1;
-    pdl_prologue();
+    pdl_launch_dependents();
+    const bool listed = p.group_offsets || p.a_rows || p.c_rows || p.row_scale;      // lists come from kernels of the same step, without them only
+    if (listed) pdl_wait();                          // A (and the factor) does, and the weights travel while its kernel ends
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typedef __nv_bfloat16 (*ATile)[BM][PITCH];
     typedef __nv_bfloat16 (*WTile)[NB][BN][PITCH];
@@ -163,7 +165,7 @@ grouped_mma_kernel(MmaParams p) {
         w_dst[i] = e < BN * PIECES ? row * PITCH + piece * 8 : -1;
         w_k[i] = piece * 8;
     }
-    auto load_stage = [&](int stage, int kt) {
+    auto load_a = [&](int stage, int kt) {
         const int k0 = kt * BK;
         __nv_bfloat16* a_stage = &As[stage][0][0];
 #pragma unroll
@@ -172,6 +174,9 @@ grouped_mma_kernel(MmaParams p) {
             const bool ok = a_src[i] != nullptr && k0 + a_k[i] < p.K;
             cp_async16(a_stage + a_dst[i], ok ? (const void*)(a_src[i] + k0) : (const void*)p.A, ok);
         }
+    };
+    auto load_w = [&](int stage, int kt) {
+        const int k0 = kt * BK;
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             __nv_bfloat16* w_stage = &Ws[stage][b][0][0];
@@ -195,9 +200,13 @@ grouped_mma_kernel(MmaParams p) {
                 for (int i = 0; i < 4; ++i) acc[m][b][j][i] = 0.0f;
 
 #pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < k_tiles) load_w(s, s);
+    if (!listed) pdl_wait();
+#pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < k_tiles) load_stage(s, s);
-        cp_async_commit();
+        if (s < k_tiles) load_a(s, s);
+        cp_async_commit();                            // (the first group holds W of every stage in front of it)
     }
     const int warp_m = warp % WARPS_M, warp_n = warp / WARPS_M;
     const int a_row = warp_m * 16 * MT + (lane & 7) + 8 * ((lane >> 3) & 1), a_col = 8 * (lane >> 4);
@@ -205,7 +214,7 @@ grouped_mma_kernel(MmaParams p) {
     for (int kt = 0; kt < k_tiles; ++kt) {
         cp_async_wait<STAGES - 2>();
         __syncthreads();                              // stage kt has landed for everyone; stage kt-1 is free to refill
-        if (kt + STAGES - 1 < k_tiles) load_stage((kt + STAGES - 1) % STAGES, kt + STAGES - 1);
+        if (kt + STAGES - 1 < k_tiles) { load_a((kt + STAGES - 1) % STAGES, kt + STAGES - 1); load_w((kt + STAGES - 1) % STAGES, kt + STAGES - 1); }
         cp_async_commit();
         const int stage = kt % STAGES;
 #pragma unroll
