@@ -1,5 +1,4 @@
-"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, per-head products of few rows, the split of
-latent attention's projection."""
+"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, the split of latent attention's projection."""
 import pytest
 import torch
 
@@ -21,27 +20,6 @@ def test_fp32_rows_have_the_bits_of_a_row_alone(M, N, K):
         ops.gemm_f32(x[m:m + 1].contiguous(), w, row, bias=bias)
         assert torch.equal(out[m:m + 1], row), m
     assert bool(torch.isfinite(out).all())
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16])
-@pytest.mark.parametrize("groups, N, K, factor", [(16, 512, 128, False), (16, 128, 512, True), (3, 40, 96, True), (5, 17, 32, False), (2, 64, 1056, True)])
-def test_per_head_products_of_few_rows(rows, groups, N, K, factor):
-    from microllm_rocm_b200.kernels import grouped
-    g = torch.Generator(DEV).manual_seed(N + K)
-    a = torch.randn(rows, groups * K, generator=g, device=DEV).bfloat16()
-    w = (torch.randn(groups, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
-    by = torch.rand(rows, groups * (N + 8), generator=g, device=DEV) if factor else None
-    out = torch.full((rows, groups * (N + 8)), 7.0, dtype=torch.bfloat16, device=DEV)          # (eight columns a group that nobody writes)
-    assert grouped.few_rows(a, w, out, rows, K) and not grouped.few_rows(a, w, out, 17, K)
-    grouped.grouped_linear(a, w, out, rows=rows, a_group_cols=K, c_group_cols=N + 8, factor=by, row_tile=16)
-    want = torch.einsum("mgk,gnk->mgn", a.double().view(rows, groups, K), w.double())
-    if factor:
-        want = want * by.double().view(rows, groups, N + 8)[..., :N]
-    got = out.view(rows, groups, N + 8)
-    assert bool((got[..., N:] == 7.0).all())
-    # the result's rounding, half a unit of eight bits, and fp32 sums of K products
-    assert bool(((got[..., :N].double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
 
 
 @pytest.mark.gpu
