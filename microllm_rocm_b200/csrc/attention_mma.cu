@@ -1050,12 +1050,63 @@ __device__ __forceinline__ void merge_and_store_t(const FaParams& p, const TileG
 
 // shared memory (dynamic): queries | per-warp fragments [DW][FRAGS_T][32] | warp max/sum per head |
 // this CTA's merged heads [8][D] with their max and sum | block table
-constexpr size_t decode_t_smem(int dw) {
-    return 16 * Q_STRIDE * sizeof(__nv_bfloat16) + (size_t)dw * FRAGS_T * 32 * sizeof(float) + 2 * dw * 8 * sizeof(float) +
+
+// A thread's own pieces of a key tile (what load_keys leaves in its registers) on their way to its own places in shared memory, [piece][lane]:
+// nobody else reads them, so waiting for its own copies is all that a thread needs.  False where the page is not there.
+constexpr int TILE_PIECES = 2 * KCHUNKS + 4 * VBLOCKS;
+__device__ __forceinline__ bool copy_keys(const FaParams& p, const TileGeometry& geo, const PageTable& pt, int kt, int hi_tile, uint4* slot) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int base = kt * 16;
+    const int block = p.page_shift >= 0 ? base >> p.page_shift : base / p.page_size;
+    const int in_page = p.page_shift >= 0 ? base & (p.page_size - 1) : base % p.page_size;
+    const int page = pt.page_of(block);
+    if (page < 0 || page >= p.num_pages) {
+        if (lane == 0 && p.error_flag) atomicExch(p.error_flag, 3);
+        return false;
+    }
+    const __nv_bfloat16* kbase = p.pages + (size_t)page * 2 * p.num_kv_heads * p.page_size * D + ((size_t)geo.kvh * p.page_size + in_page) * D;
+    const __nv_bfloat16* vbase = kbase + (size_t)p.num_kv_heads * p.page_size * D;
+    const unsigned to = (unsigned)__cvta_generic_to_shared(slot + lane);
+    auto copy = [&](int piece, const __nv_bfloat16* src, bool valid) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + piece * 512), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    };
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int c = 0; c < KCHUNKS; ++c) copy(nb * KCHUNKS + c, kbase + (size_t)(nb * 8 + g) * D + c * 32 + t * 8, true);
+#pragma unroll
+    for (int vb = 0; vb < VBLOCKS; ++vb)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int key = 2 * t + (r & 1) + 8 * (r >> 1), col = vb * 64 + g * 8;
+            copy(2 * KCHUNKS + vb * 4 + r, vbase + (size_t)key * D + (col < D ? col : 0), col < D && base + key <= hi_tile);
+        }
+    return true;
+}
+__device__ __forceinline__ void take_keys(const uint4* slot, int base, KeyTile& kv) {
+    const uint4* at = slot + (threadIdx.x & 31);
+    kv.base = base;
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int c = 0; c < KCHUNKS; ++c) kv.k[nb][c] = at[(nb * KCHUNKS + c) * 32];
+#pragma unroll
+    for (int vb = 0; vb < VBLOCKS; ++vb)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) kv.v[vb][r] = at[(2 * KCHUNKS + vb * 4 + r) * 32];
+}
+
+constexpr size_t decode_t_smem(int dw, int depth = 0) {
+    return 16 * Q_STRIDE * sizeof(__nv_bfloat16) + (size_t)dw * 128 * (depth > 0 ? depth * TILE_PIECES * 4 : FRAGS_T) + 2 * dw * 8 * sizeof(float) +
            (size_t)8 * D * sizeof(float) + 16 * sizeof(float) + TABLE_SPAN * sizeof(int);
 }
 
-template <int DW>
+// DEPTH 0: a warp's next key tile is on its way to registers while it multiplies one; else DEPTH tiles are, to shared memory, beside the one in
+// registers.  The tiles of a warp, their order and what the products see are the same, and so are the bits.  Two tiles a ring (74 KB a CTA of four
+// warps) leave two CTAs a multiprocessor; three, four and six gave less (decode of 4 x 6,144 tokens on the 7B shapes, four steps: 14,990 us in
+// registers, 14,490 with two, 14,270 with three, but 41 requests of 64 to 2,048 on the 1.5B 8,830 / 8,350 / 8,370, and one CTA a multiprocessor 15,900).
+[[maybe_unused]] constexpr int RING_DEPTH = 2;
+template <int DW, int DEPTH>
 __global__ void __launch_bounds__(DW * 32, DW == 4 ? 2 : 1) fa_decode_t_kernel(FaParams p) {
     pdl_launch_dependents();       // the wait comes after the sequence's length, block table and first keys are on their way
     namespace cg = cooperative_groups;
@@ -1063,7 +1114,7 @@ __global__ void __launch_bounds__(DW * 32, DW == 4 ? 2 : 1) fa_decode_t_kernel(F
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);                             // [8 heads used of 16][Q_STRIDE]
     float* frag = reinterpret_cast<float*>(smem_raw + 16 * Q_STRIDE * sizeof(__nv_bfloat16));   // [DW][FRAGS_T][32]
-    float* warp_m = frag + DW * FRAGS_T * 32;      // [DW][8]
+    float* warp_m = frag + (DEPTH > 0 ? DW * DEPTH * TILE_PIECES * 128 : DW * FRAGS_T * 32);      // [DW][8]  (fragments come when the tiles are gone)
     float* warp_l = warp_m + DW * 8;               // [DW][8]
     float* cta_o = warp_l + DW * 8;                // [8][D]  this CTA's heads, scaled to cta_m
     float* cta_m = cta_o + 8 * D;                  // [8]
@@ -1099,7 +1150,21 @@ __global__ void __launch_bounds__(DW * 32, DW == 4 ? 2 : 1) fa_decode_t_kernel(F
     KeyTile tile_a, tile_b;
     int kt = tile_begin + warp;
     int in_flight = 0;
-    if (kt < tile_end && tiles.at(kt) < last_pos / 16) {
+    uint4* const ring = reinterpret_cast<uint4*>(frag) + warp * DEPTH * TILE_PIECES * 32;
+    unsigned here = 0;                       // ring slots whose page is there
+    auto ask = [&](int slot, int tile) {
+        if (tile < tile_end) {
+            const bool there = copy_keys(p, geo, pt, tiles.at(tile), last_pos, ring + slot * TILE_PIECES * 32);
+            here = there ? here | (1u << slot) : here & ~(1u << slot);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if constexpr (DEPTH > 0) {
+        while (in_flight < DEPTH && kt + in_flight * DW < tile_end && tiles.at(kt + in_flight * DW) < last_pos / 16) {
+            ask(in_flight, kt + in_flight * DW);
+            ++in_flight;
+        }
+    } else if (kt < tile_end && tiles.at(kt) < last_pos / 16) {
         load_keys(p, geo, pt, tiles.at(kt), last_pos, tile_a);
         in_flight = 1;
         if (USE_PREFETCH && kt + DW < tile_end && tiles.at(kt + DW) < last_pos / 16) {
@@ -1127,7 +1192,19 @@ __global__ void __launch_bounds__(DW * 32, DW == 4 ? 2 : 1) fa_decode_t_kernel(F
         for (int e = 0; e < 4; ++e) st.o[k][e] = 0.0f;
     const float* bias_row[2];
     bias_rows_t(p, geo.kvh, bias_row);
-    if (kt < tile_end) {
+    if constexpr (DEPTH > 0) {
+        for (; in_flight < DEPTH; ++in_flight) ask(in_flight, kt + in_flight * DW);
+        for (int slot = 0; kt < tile_end; kt += DW, slot = slot + 1 < DEPTH ? slot + 1 : 0) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH > 0 ? DEPTH - 1 : 0) : "memory");
+            const bool there = (here >> slot) & 1u;
+            if (there) take_keys(ring + slot * TILE_PIECES * 32, tiles.at(kt) * 16, tile_a);
+            __syncwarp();                    // (taken before its place is given to the next)
+            ask(slot, kt + DEPTH * DW);
+            if (there) consume_keys_t(p, q_s, tile_a, last_pos, lo, bias_row, st);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                     // the rings become the warps' fragments
+    } else if (kt < tile_end) {
         if (USE_PREFETCH) {
             if (in_flight < 1) load_keys(p, geo, pt, tiles.at(kt), last_pos, tile_a);
             while (true) {
@@ -1445,6 +1522,7 @@ MLB_EXPORT int mlb_paged_attention_mma(const void* q, const void* pages, void* o
     if (num_pages <= 0 || max_blocks <= 0 || window < 0 || keep < 0 || chunk < 0 || num_work < 0)
         return fail(MLB_INVALID_ARGUMENT, "paged_attention_mma: bad cache geometry");
     const bool force_ring = (mode & 4) != 0, forbid_ring = (mode & 8) != 0;
+    [[maybe_unused]] const bool own_rings = (mode & 16) != 0;
     mode &= 3;
     if (mode < 0 || mode > 2) return fail(MLB_INVALID_ARGUMENT, "paged_attention_mma: unknown mode %d", mode);
     if (mode == 2 && !work) return fail(MLB_INVALID_ARGUMENT, "paged_attention_mma: mode 2 needs the list of sequences");
@@ -1483,10 +1561,10 @@ MLB_EXPORT int mlb_paged_attention_mma(const void* q, const void* pages, void* o
             e = cudaFuncSetAttribute(fa_decode_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem(8));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_kernel<8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_t_smem(4));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_t_smem(8));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_t_smem(4));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<8, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_t_smem(8));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<4, 0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_decode_t_kernel<8, 0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return fail(MLB_CUDA_ERROR, "fa_decode: cannot reserve %d bytes of shared memory: %s",
                                           (int)decode_smem(8), cudaGetErrorString(e));
         configured = true;
@@ -1544,9 +1622,28 @@ MLB_EXPORT int mlb_paged_attention_mma(const void* q, const void* pages, void* o
         cudaLaunchKernelEx(&config, fa_decode_ring_kernel, map_kv, p);
         return check_launch("fa_decode_ring");
     }
+#if HEAD_DIM == 128          // (the width whose rings were measured: 8 KB a tile)
+    if (keys_on_m && own_rings && splits <= 8) {
+        static bool rings_configured_on[MAX_DEVICES] = {false};
+        bool& rings_configured = rings_configured_on[device_index()];
+        if (!rings_configured) {
+            auto allow = [](auto kernel, int dw) {
+                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_t_smem(dw, RING_DEPTH));
+                return e == cudaSuccess ? cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : e;
+            };
+            cudaError_t e = allow(fa_decode_t_kernel<4, RING_DEPTH>, 4);
+            if (e == cudaSuccess) e = allow(fa_decode_t_kernel<8, RING_DEPTH>, 8);
+            if (e != cudaSuccess) return fail(MLB_CUDA_ERROR, "fa_decode_t: cannot reserve shared memory for the rings: %s", cudaGetErrorString(e));
+            rings_configured = true;
+        }
+        config.dynamicSmemBytes = decode_t_smem(wide ? 8 : 4, RING_DEPTH);
+        cudaLaunchKernelEx(&config, wide ? fa_decode_t_kernel<8, RING_DEPTH> : fa_decode_t_kernel<4, RING_DEPTH>, p);
+        return check_launch("fa_decode_t (rings)");
+    }
+#endif
     if (keys_on_m) {
-        if (wide) cudaLaunchKernelEx(&config, fa_decode_t_kernel<8>, p);
-        else cudaLaunchKernelEx(&config, fa_decode_t_kernel<4>, p);
+        if (wide) cudaLaunchKernelEx(&config, fa_decode_t_kernel<8, 0>, p);
+        else cudaLaunchKernelEx(&config, fa_decode_t_kernel<4, 0>, p);
         return check_launch("fa_decode_t");
     }
     if (wide) cudaLaunchKernelEx(&config, fa_decode_kernel<8>, p);

@@ -30,6 +30,8 @@ WIDE_CLUSTER_CTAS = 48              # measured: one sequence of two kv heads gai
 # Which decode kernel takes heads of 128: None = by the step's shape (`decode_ring_pays`); True / False = always /
 # never.  Tests set it to run both kernels on the same inputs.
 DECODE_RING = None
+OWN_RINGS = None                    # the same for the kernel that brings them into registers: by way of shared memory where `own_rings_pay`
+RINGS_MIN_KEYS_PER_CTA = 400
 RING_MIN_KEYS_PER_CTA = 1024        # measured: 16 stages of 64 keys per CTA and the ring wins by 7-8 %, 8 stages and it loses 12 %
 # Measured in whole decode steps at context 8,192 (8 layers of the 14B / 7B shapes), when the products around the
 # attention were still the few-token mma.sync kernels: with 8 tokens the ring cost 2.64 against 2.01 ms / 2.08
@@ -113,11 +115,23 @@ def decode_ring_pays(items: int, splits: int, max_seq_len: int, sms: int = DEFAU
             and not beside_mma_products)
 
 
+def own_rings_pay(splits: int, max_seq_len: int, beside_mma_products: bool, visible: int = 1 << 30) -> bool:
+    """Whether the decode kernel that has its keys in registers gets them by way of its warps' own rings in shared memory: from 400 keys a CTA
+    on (of the `visible` last ones, where a window ends them), away from the few-token mma.sync products (whose shared memory then finds no room early: 8 requests of 2,048 on the 1.5B shapes
+    5,230 -> 7,800 us).  Measured in whole decode steps, heads of 128 (us for four steps, registers / rings): 7B 4 x 6,144 (768 keys a CTA)
+    14,990 / 14,490, 1 x 6,144 13,950 / 13,470, 5 x 4,000 13,760 / 13,430, 7 of 300 to 3,400 12,930 / 12,810; 1.5B 41 of 64 to 2,048
+    (1,024) 8,800 / 8,340; 30 of 80 to 800 13,430 / 13,420.  Below: 7B 8 x 2,048 (256) 13,340 / 13,640, 8 of 1,000 to 3,000 13,320 / 13,450;
+    1.5B 32 of 300 to 700 (175) 5,990 / 6,060; but 16 x 2,048 6,400 / 6,150."""
+    return min(max_seq_len, visible) // max(1, splits) >= RINGS_MIN_KEYS_PER_CTA and not beside_mma_products
+
+
 def decode_plan_stale(ctx, max_seq_len: int, sms: int = DEFAULT_SM_COUNT) -> bool:
     """Whether a decode step planned for `ctx` (its plans are kept in ctx.extras, and frozen into a captured
     graph) would be cut differently at this context length: a step captured at a short context has one CTA
     per (sequence, kv head) and must not serve a context of thousands that way."""
     for key, plan in ctx.extras.items():
+        if isinstance(key, tuple) and key and key[0] == "attention_rings" and not plan and own_rings_pay(key[1], max_seq_len, *key[2:]):
+            return True                # (not the other way: rings cost a short context a percent, and a step is not captured back and forth)
         if isinstance(key, tuple) and key and key[0] == "attention_mma" and plan[2] == 1:
             splits = decode_splits(plan[1] * key[2], max_seq_len, sms)
             beside = bool(key[4]) if len(key) > 4 else False
@@ -127,7 +141,7 @@ def decode_plan_stale(ctx, max_seq_len: int, sms: int = DEFAULT_SM_COUNT) -> boo
 
 
 def forget_plans(ctx) -> None:
-    for key in [k for k in ctx.extras if isinstance(k, tuple) and k and k[0] == "attention_mma"]:
+    for key in [k for k in ctx.extras if isinstance(k, tuple) and k and k[0] in ("attention_mma", "attention_rings")]:
         del ctx.extras[key]
 
 
@@ -212,6 +226,12 @@ def paged_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, ctx
     work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring = _plan(
         ctx, num_heads // num_kv_heads, num_kv_heads, use_tc, beside_mma_products)
     ring_bits = 4 if (ring if DECODE_RING is None else DECODE_RING) else 8
+    visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
+    own = own_rings_pay(splits if mode else listed_splits, ctx.max_seq_len, beside_mma_products, visible)
+    if mode:
+        ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own
+    if own if OWN_RINGS is None else OWN_RINGS:
+        ring_bits |= 16
     side = None
     if num_tc:
         # Prompt portions and the decoded tokens beside them are different sequences: their two launches write
