@@ -31,11 +31,19 @@ ops.register_signatures(MMA_SOURCE, {
     "mlb_latent_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
 })
+TC_SOURCE = "latent_tc.cu"
+ops.register_signatures(TC_SOURCE, {
+    "mlb_latent_tc_rows_per_tile": [],
+    "mlb_latent_attention_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                c_int, c_int, c_float, c_void_p, c_void_p],
+})
+TC_ROWS_PER_TILE = 128              # of which a CTA of the tcgen05 kernel owns half the output columns
 ROWS_PER_TILE = 16                  # (token, head) rows of one sequence that a group of warps of the tensor-core kernel owns
 KEYS_PER_TILE = 32
 MIN_KEY_TILES_PER_SPLIT = 4         # a CTA that shares a work item's keys streams 128 of them at least
 MAX_SPLITS = 64
 GROUPS = None                       # 1 or 2: tests set the groups of rows a CTA holds (where the keys are not split); None: _plan decides
+TCGEN05 = None                      # tests set which sequences go to the tcgen05 kernel: True all (where the keys are not split), False none; None: the rule
 USE_TENSOR_CORES = True             # tests set it to False to run the plain kernel on the same inputs
 
 
@@ -45,6 +53,14 @@ def mma_supported(rank: int, rot_dim: int) -> bool:
 
 def mma_sources(rank: int, rot_dim: int):
     return [(MMA_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})] if mma_supported(rank, rot_dim) else []
+
+
+def tc_supported(rank: int, rot_dim: int, page_size: int = KEYS_PER_TILE) -> bool:
+    return rank % 128 == 0 and 0 < rank <= MAX_RANK and rot_dim == 64 and page_size % 8 == 0 and (KEYS_PER_TILE % page_size == 0 or page_size % KEYS_PER_TILE == 0)
+
+
+def tc_sources(rank: int, rot_dim: int):
+    return [(TC_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})] if tc_supported(rank, rot_dim) else []
 
 
 def key_splits(num_work: int, max_seq_len: int, sms: int) -> int:
@@ -94,6 +110,44 @@ def _plan(ctx, heads: int):
     return plan
 
 
+def tc_pays(tiles: int, mean_keys: float) -> bool:
+    """Whether a step's sequences of 128 (token, head) rows and more, `tiles` tiles of 128 rows whose tokens see `mean_keys` keys, go to the tcgen05
+    kernel: a CTA takes 9 us before its first tile of keys and 1.8 for each, so many tiles want 64 keys and few tiles thousands.
+    Measured (512 + 64 wide, 148 SMs, us, mma.sync / tcgen05): 16 heads, a prompt of 2,048 tokens 427 / 249, 1,024 118 / 78, 512 47 / 41, 256 26 / 25,
+    128 13 / 18; 512 behind 2,000 356 / 158, 64 behind 2,000 130 / 120; 8 times 128 tokens 32.6 / 30.4, 45 13 / 15, 16 behind 1,000 80 / 66,
+    8 behind 1,000 62 / 66; 40 times 40 35.0 / 36.3; 4 heads, 2,048 tokens 163 / 126, 512 36.8 / 38.3; 64 heads, 128 tokens 22 / 19."""
+    return (tiles >= 32 and mean_keys >= 64) or tiles * mean_keys >= 12000
+
+
+def _tc_plan(ctx, heads: int):
+    """(work of the tcgen05 kernel, its length, work of the mma.sync kernel, its length, its groups) of a step whose keys are not split: items
+    as in _plan, of 128 rows and of 16 or 32; None where the first would be empty."""
+    from .device import sm_count
+    key = ("latent_tc", heads)
+    if key in ctx.extras:
+        return ctx.extras[key]
+    device = ctx.positions.device
+    sms = sm_count(device)
+    starts, front = ctx.seq_starts_host, ctx.seq_pos0_host or [0] * ctx.num_seqs
+    new = [starts[a + 1] - starts[a] for a in range(ctx.num_seqs)]
+    rows = [n * heads for n in new]
+    takes = [n > 0 and (n >= TC_ROWS_PER_TILE if TCGEN05 is None else TCGEN05) for n in rows]
+    tiles = sum(-(-n // TC_ROWS_PER_TILE) for n, t in zip(rows, takes) if t)
+    mean = sum(n * (p + 0.5 * (n + 1)) for n, p, t in zip(new, front, takes) if t) / max(1, sum(n for n, t in zip(new, takes) if t))
+    rest = [a for a in range(ctx.num_seqs) if not takes[a]]
+
+    def upload(step, which):
+        work = [(front[a] + min(rows[a], first + step) // heads, a, first) for a in which for first in range(0, rows[a], step)]
+        work.sort(key=lambda item: -item[0])
+        return ops.upload([x for _, a, first in work for x in (a, first)], "int32", device) if work else None, len(work)
+    plan = None
+    if 0 < tiles < 65536 and (TCGEN05 or tc_pays(tiles, mean)):
+        groups = 2 if sum(-(-rows[a] // ROWS_PER_TILE) for a in rest) >= 5 * sms else 1
+        plan = (*upload(TC_ROWS_PER_TILE, [a for a in range(ctx.num_seqs) if takes[a]]), *upload(groups * ROWS_PER_TILE, rest), groups)
+    ctx.extras[key] = plan
+    return plan
+
+
 def plan_stale(ctx, max_seq_len: int) -> bool:
     from .device import sm_count
     for key, plan in ctx.extras.items():
@@ -110,8 +164,9 @@ def forget_plans(ctx) -> None:
 
 def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Optional[torch.Tensor], ctx,
               block_table: torch.Tensor, heads: int, rank: int, rot_dim: int, scale: float, window: Optional[int]) -> None:
-    """The step's attention over the compressed cache: bf16 on the tensor cores when the widths suit them, else (and
-    always in fp32) the plain kernel."""
+    """The step's attention over the compressed cache: bf16 on the tensor cores when the widths suit them (sequences of many new rows on
+    the tcgen05 kernel, which gives the same bits as the mma.sync one; the two write disjoint rows), else (and always in fp32) the plain
+    kernel."""
     if not (USE_TENSOR_CORES and q.dtype == torch.bfloat16 and pages.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
             and mma_supported(rank, rot_dim)):
         attention_plain(q, pages, out, sink, ctx.positions, ctx.token_seq, block_table, heads, rank, rot_dim, scale, window,
@@ -123,6 +178,22 @@ def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Opt
     if width != rank + rot_dim or q.shape[1] != heads * width or tuple(out.shape) != (T, heads * rank):
         raise KernelError("latent.attention: shapes do not agree")
     work, num_work, splits, groups = _plan(ctx, heads)
+    side = None
+    if splits == 1 and not ctx.decode_only and GROUPS is None and TCGEN05 is not False and tc_supported(rank, rot_dim, page_size):
+        plan = _tc_plan(ctx, heads)
+        if plan is not None:
+            tc_work, num_tc, work, num_work, groups = plan
+            stream = ops._stream()
+            if num_work:                     # other sequences, other rows: the two launches run side by side
+                side = stream = ops.side_stream()
+                ops.fork(side)
+            L = ops.lib(TC_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})
+            build.check(L, L.mlb_latent_attention_tc(
+                q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), block_table.data_ptr(),
+                tc_work.data_ptr(), num_tc, block_table.shape[1], num_pages, page_size, heads, int(window or 0), T * heads, float(scale),
+                ops._ptr(ctx.error_flag), stream))
+            if num_work == 0:
+                return
     part_o = part_ml = None
     if splits > 1:
         part_o = ctx.buffer("latent.part_o", (splits, T * heads, rank), torch.float32)
@@ -132,6 +203,8 @@ def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Opt
         q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(),
         block_table.data_ptr(), work.data_ptr(), num_work, ops._ptr(part_o), ops._ptr(part_ml), block_table.shape[1], num_pages,
         page_size, heads, int(window or 0), splits, groups, T * heads, float(scale), ops._ptr(ctx.error_flag), ops._stream()))
+    if side is not None:
+        ops.join(side)
 
 
 def sources():

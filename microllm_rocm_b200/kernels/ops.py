@@ -149,6 +149,11 @@ def lagged_group_sources():
     return [("grouped_tc2.cu", {"MLB_LAG_WARP": w, "MLB_LAG_RANK": r}) for w, r in ((0, 1), (1, 0), (3, 0), (4, 1))]
 
 
+def lagged_latent_sources():
+    """And of latent attention's prompts."""
+    return [("latent_tc.cu", {"LAT_R": 512, "LAT_DR": 64, "MLB_LAG_WARP": w}) for w in (0, 1, 2, 5, 7)]
+
+
 def lib(source: str, defines=None) -> ctypes.CDLL:
     if TEST_DEFINES.get(source):
         defines = {**(defines or {}), **TEST_DEFINES[source]}
@@ -198,7 +203,7 @@ def all_sources():
         out += attention.mma_sources(d) + attention.tc_sources(d)
     from . import gemm_bf16, latent
     return (out + gemm_bf16.sources() + [("gemv_noalloc.cu", {})] + part_sources()
-            + latent.mma_sources(32, 8) + latent.mma_sources(256, 32) + latent.mma_sources(512, 64))      # the widths of the presets
+            + latent.mma_sources(32, 8) + latent.mma_sources(256, 32) + latent.mma_sources(512, 64) + latent.tc_sources(512, 64))      # the widths of the presets
 
 
 # ------------------------------------------------------------------------------ basic

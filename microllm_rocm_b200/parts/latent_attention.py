@@ -102,7 +102,7 @@ class LatentAttention(Mixer):
 
     def kernel_sources(self):
         own = latent.sources() + grouped.sources()
-        return own if self.rt.is_fp32 else own + latent.mma_sources(self.rank, self.rot_dim) + gemm_bf16.sources(engine_only=True)
+        return own if self.rt.is_fp32 else own + latent.mma_sources(self.rank, self.rot_dim) + latent.tc_sources(self.rank, self.rot_dim) + gemm_bf16.sources(engine_only=True)
 
     def bind(self, tensors):
         n = self.names
