@@ -1,4 +1,5 @@
-"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, the split of latent attention's projection."""
+"""Kernels whose tiles or pieces follow the sizes: fp32 products of more rows than the streaming kernel's, the split of latent attention's projection, the
+stores of the grouped product."""
 import pytest
 import torch
 
@@ -50,3 +51,30 @@ def test_the_split_of_a_projection_four_columns_at_a_time(dtype, heads, dim, rot
         assert int(flag.item()) == 0
     for a, b in zip(*results):
         assert torch.equal(a, b) and bool((a != 0).any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("row_tile", [16, 64, 128])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N, K, factor, listed", [(512, 128, False, False), (128, 512, True, False), (72, 64, True, False), (96, 40, False, True)])
+def test_outputs_stored_together_have_the_bits_of_each_alone(row_tile, out_dtype, N, K, factor, listed):
+    """Rows that start on 16 bytes take several columns to a store, rows of an odd pitch one: whole tiles and parts, rows that nobody wants."""
+    from microllm_rocm_b200.kernels import grouped
+    G, rows = 3, 131
+    g = torch.Generator(DEV).manual_seed(N)
+    w = (torch.randn(G, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    on = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    kw, width = (dict(a_group_cols=K, c_group_cols=N), G * N) if not listed else \
+        (dict(group_offsets=on([0, 70, 70, rows]), a_rows=on([(7 * i) % rows for i in range(rows)]), c_rows=on([-1 if i % 5 == 0 else i for i in range(rows)])), N)
+    a = torch.randn(rows, K if listed else G * K, generator=g, device=DEV).bfloat16()
+    by = torch.rand(rows, width + 1, generator=g, device=DEV)
+    results = []
+    for extra in (0, 1):
+        out = torch.full((rows, width + extra), 7.0, dtype=out_dtype, device=DEV)
+        grouped.USE_PAIRS = False
+        try:
+            grouped.grouped_linear(a, w, out, rows=rows, factor=by[:, :width + extra].contiguous() if factor else None, row_tile=row_tile, **kw)
+        finally:
+            grouped.USE_PAIRS = None
+        results.append(out[:, :width])
+    assert torch.equal(*results) and int((results[0] == 7.0).sum()) == (len(range(0, rows, 5)) * N if listed else 0)
