@@ -33,7 +33,7 @@ struct ConvParams {
     int T, A, C, taps, act;
     int* error_flag;
     int run = 1;               // tokens a thread of the four-channel kernel walks
-    int move = 0;              // 1: every sequence brings one token, whose thread moves the state on
+    int move = 0;              // 1: every sequence brings one token (the caller's word: the counts lie on the device), whose thread moves the state on
     const float* bias = nullptr;   // [C] or null
 };
 

@@ -67,7 +67,8 @@ def short_conv(u: torch.Tensor, col0: int, weight: torch.Tensor, state: Optional
             raise KernelError(f"short_conv: the state must be [slots, {taps - 1}, {C}], got {tuple(state.shape)}")
         num_slots = state.shape[0]
     L = ops.lib("short_conv.cu")
-    move = taps > 1 and update_state and T == ctx.num_seqs          # one token a sequence: the same launch moves the state on
+    # one token a sequence: the same launch moves the state on (as many tokens as sequences may also be two of one and none of another)
+    move = taps > 1 and update_state and getattr(ctx, "max_new_tokens", 0) == 1 and T == ctx.num_seqs
     build.check(L, L.mlb_short_conv(u.data_ptr(), ld, n, stride, col0, weight.data_ptr(), ops._ptr(bias), ops._ptr(state), slots.data_ptr(), num_slots,
                                     ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), ctx.token_seq.data_ptr(), out.data_ptr(),
                                     out.shape[1], T, ctx.num_seqs, C, taps, 1 if silu else 0, 1 if move else 0, ops._ptr(ctx.error_flag), ops._stream()))

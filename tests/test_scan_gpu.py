@@ -88,6 +88,27 @@ def test_one_token_a_sequence_moves_the_state_on(taps, C, partials):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("counts", [[2, 0], [0, 2], [3, 0, 0], [0, 1, 2], [1, 0, 1]])
+@pytest.mark.parametrize("C", [12, 37])
+def test_sequences_without_tokens_beside_others(counts, C):
+    """As many tokens as sequences, but not one each: outputs and states of a step that does not name the empty ones, whose states stay."""
+    from microllm_rocm_b200.kernels import recurrent
+    taps, pos0 = 4, [5, 1, 40][:len(counts)]
+    g = torch.Generator(DEV).manual_seed(C)
+    u, w = torch.randn(sum(counts), C + 8, generator=g, device=DEV), torch.randn(C, taps, generator=g, device=DEV)
+    held = torch.randn(len(counts) + 1, taps - 1, C, generator=g, device=DEV)
+
+    def run(which):
+        state, out = held.clone(), torch.empty(sum(counts), C, device=DEV)
+        ctx, _ = step([counts[a] for a in which], [pos0[a] for a in which])
+        recurrent.short_conv(u, 4, w, state, torch.tensor(which, dtype=torch.int32, device=DEV), ctx, out, silu=True)
+        assert int(ctx.error_flag.item()) == 0
+        return out, state
+    got, want = run(list(range(len(counts)))), run([a for a, n in enumerate(counts) if n])
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("family, dtype", [("matidra", "float32"), ("matidra", "bfloat16"), ("naburax", "float32"), ("lozepel", "bfloat16"), ("fonuvik", "bfloat16")])
 def test_branches_side_by_side_have_the_bits_of_one_after_another(tmp_path, family, dtype):
     """A prompt, a step that decodes beside a prompt portion, and decoded tokens."""
