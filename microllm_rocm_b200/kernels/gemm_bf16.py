@@ -348,6 +348,19 @@ def _direct_library(device) -> bool:
     return _direct_ok
 
 
+def _library_workspace(device) -> torch.Tensor:
+    """Products of two streams may run at once and then need two workspaces.  Every host thread has a second stream of its own, so
+    the one for products there belongs to the step that asked for that stream, and goes with it; without a step to a stream's handle."""
+    side, scratch = ops.second_stream()
+    if scratch is not None:
+        return scratch(LIBRARY_WORKSPACE_BYTES)
+    key = (str(device), side)
+    work = _workspaces.get(key)
+    if work is None:
+        work = _workspaces[key] = torch.empty(LIBRARY_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
+    return work
+
+
 def library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype,
                    out: Optional[torch.Tensor], alloc=None) -> torch.Tensor:
     """cuBLASLt: bf16 operands, fp32 accumulate, output written in out_dtype.  `alloc(shape, dtype)` supplies
@@ -359,10 +372,7 @@ def library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
         N = weight.shape[0]
         if out is None:
             out = alloc((M, N), out_dtype) if alloc is not None else torch.empty((M, N), dtype=out_dtype, device=x.device)
-        key = (str(x.device), ops.on_second_stream())          # products of the two streams may run at once
-        work = _workspaces.get(key)
-        if work is None:
-            work = _workspaces[key] = torch.empty(LIBRARY_WORKSPACE_BYTES, dtype=torch.uint8, device=x.device)
+        work = _library_workspace(x.device)
         L = ops.lib("gemm_lib.cu")
         build.check(L, L.mlb_lt_matmul(x.data_ptr(), x.stride(0), weight.data_ptr(), weight.stride(0), out.data_ptr(),
                                        out.stride(0), 1 if out_dtype == torch.bfloat16 else 0, 0, M, N, K,

@@ -687,26 +687,27 @@ def join(side: int) -> None:
 
 
 @contextlib.contextmanager
-def on_side_stream():
+def on_side_stream(scratch=None):
     """This library's launches inside go to the device's second stream, which continues from where the current one stands; the
     caller joins (`join(side)`, side being what this yields) before anything reads what they write, and lets go of none of their
-    tensors before that.  Only for work that launches kernels of this library and nothing through the tensor framework."""
-    side, outer = side_stream(), getattr(_launch_on, "side", None)
+    tensors before that.  Only for work that launches kernels of this library and nothing through the tensor framework.
+    `scratch(bytes)` -> uint8 tensor: memory of the step for what a launch inside needs beside its operands (a library product's workspace)."""
+    side, outer, outer_scratch = side_stream(), getattr(_launch_on, "side", None), getattr(_launch_on, "scratch", None)
     fork(side)
-    _launch_on.side = side
+    _launch_on.side, _launch_on.scratch = side, scratch or outer_scratch
     try:
         yield side
     except BaseException:
-        _launch_on.side = outer
+        _launch_on.side, _launch_on.scratch = outer, outer_scratch
         join(side)                                   # whoever catches this lets go of the tensors, and may be capturing
         raise
     finally:
-        _launch_on.side = outer
+        _launch_on.side, _launch_on.scratch = outer, outer_scratch
 
 
-def on_second_stream() -> bool:
-    """Whether this thread's launches go to the second stream just now."""
-    return getattr(_launch_on, "side", None) is not None
+def second_stream():
+    """(the second stream's handle while this thread's launches go there, else None; its `scratch`, or None)."""
+    return getattr(_launch_on, "side", None), getattr(_launch_on, "scratch", None)
 
 
 def stream_synchronize() -> None:

@@ -17,7 +17,7 @@ def calls(monkeypatch):
     class Library:
         def __init__(self, source):
             text = open(f"{build.CSRC}/{source}").read()
-            self.names = {fn: [p.strip().split()[-1].lstrip("*") for p in params.split(",")]
+            self.names = {fn: [p.strip().split()[-1].lstrip("*") for p in params.split(",") if p.strip()]
                           for fn, params in re.findall(r"MLB_EXPORT\s+int\s+(\w+)\s*\(([^)]*)\)", text, re.S)}
 
         def __getattr__(self, fn):
@@ -53,3 +53,58 @@ def test_only_steps_of_one_token_a_sequence_move_the_convolutions_state_in_its_l
     recurrent.short_conv(f(T, C), 0, f(C, taps), f(len(counts), taps - 1, C), ctx.token_seq, ctx, f(T, C), silu=False)
     assert [fn for fn, _ in calls] == ["mlb_short_conv"] + ([] if alone else ["mlb_short_conv_state"])
     assert calls[0][1]["move"] == (1 if alone else 0)
+
+
+def test_library_products_on_second_streams_have_a_workspace_of_their_step(calls, monkeypatch):
+    """Every host thread has a second stream of its own, and nothing orders two of them: their products may not share a workspace, with each other or
+    with the first stream's.  Those of one step may, and theirs goes when the step does."""
+    import gc
+    import threading
+    import weakref
+
+    from microllm_rocm_b200.kernels import gemm_bf16
+    from microllm_rocm_b200.parts.base import Mixer, StepContext
+    from microllm_rocm_b200.parts.parallel import ParallelMixers
+    monkeypatch.setattr(ops, "_stream", lambda: ops._launch_on.__dict__.get("side") or 1)
+    monkeypatch.setattr(ops, "side_stream", lambda: 100 + threading.get_ident())
+    monkeypatch.setattr(gemm_bf16, "_direct_library", lambda device: True)
+    monkeypatch.setattr(gemm_bf16, "_workspaces", {})
+    monkeypatch.setattr(gemm_bf16, "LIBRARY_WORKSPACE_BYTES", 64)
+
+    class Main(Mixer):
+        def forward(self, x, ctx, cache):
+            on_device = SimpleNamespace(is_cuda=True, shape=x.shape, device=x.device, stride=x.stride, data_ptr=x.data_ptr)
+            for role in ("in", "out"):
+                y = gemm_bf16.library_linear(on_device, x, None, torch.float32, None, alloc=lambda shape, dtype: ctx.buffer(role, shape, dtype))
+            return y
+
+    class Aside(Main):
+        beside_others = lambda self: True
+
+    def context():
+        ids = torch.zeros(8, dtype=torch.int32)
+        return StepContext(num_tokens=8, num_seqs=1, token_ids=ids, positions=ids, token_seq=ids, seq_starts=ids, seq_pos0=ids, seq_lens=ids, block_tables={},
+                           state_slots=ids, logit_rows=ids, error_flag=ids)
+    mixer = ParallelMixers.__new__(ParallelMixers)
+    mixer.branches = [("left", 1.0, "", Main()), ("right", 1.0, "", Aside())]
+    contexts, used = [context(), context()], [None, None]
+    lock = threading.Lock()
+
+    def work(i):
+        with lock:
+            calls.clear()
+            for _ in range(2):                                # two layers of one step
+                mixer.forward_terms(torch.zeros(8, 8), contexts[i], {})
+            used[i] = [(a["stream"], a["workspace"]) for fn, a in calls if fn == "mlb_lt_matmul"]
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    aside, first = [{w for s, w in u if s != 1} for u in used], [{w for s, w in u if s == 1} for u in used]
+    assert [len(u) for u in used] == [8, 8] and all(len(s) == 1 for s in aside + first)
+    assert aside[0] != aside[1] and first[0] == first[1] and not (aside[0] | aside[1]) & first[0]
+    gone = [weakref.ref(t) for ctx in contexts for t in ctx.extras.values()]
+    contexts.clear()
+    gc.collect()
+    assert gone and not any(r() is not None for r in gone)

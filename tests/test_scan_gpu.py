@@ -144,3 +144,42 @@ def test_branches_side_by_side_have_the_bits_of_one_after_another(tmp_path, fami
         finally:
             parallel.SIDE_BY_SIDE = True
     assert torch.equal(results[0], results[1]) and bool(torch.isfinite(results[0]).all())
+
+
+@pytest.mark.gpu
+def test_library_products_on_the_second_streams_of_two_threads():
+    """Long sums into few columns, which the library splits and meets in its workspace: two threads at once get the bits of one after another."""
+    import threading
+
+    from microllm_rocm_b200.kernels import gemm_bf16, ops
+    g = torch.Generator(DEV).manual_seed(3)
+    shapes = [(300, 256, 8192), (300, 384, 6144), (520, 128, 8192)]
+    pairs = [[(torch.randn(M, K, generator=g, device=DEV).bfloat16(), torch.randn(N, K, generator=g, device=DEV).bfloat16()) for M, N, K in shapes] for _ in range(2)]
+    want = [[gemm_bf16.library_linear(x, w, None, torch.float32, None) for x, w in own] for own in pairs]
+    torch.cuda.synchronize()
+    got, failures, barrier = [[], []], [], threading.Barrier(2)
+
+    def work(i):
+        try:
+            kept = {}
+            outs = [[torch.empty(x.shape[0], w.shape[0], device=DEV) for x, w in pairs[i]] for _ in range(20)]
+            barrier.wait(timeout=60)
+            with ops.on_side_stream(lambda size: kept.setdefault(size, torch.empty(size, dtype=torch.uint8, device=DEV))) as side:
+                for row in outs:
+                    for (x, w), out in zip(pairs[i], row):
+                        gemm_bf16.library_linear(x, w, None, torch.float32, out)
+            ops.join(side)
+            torch.cuda.synchronize()
+            got[i] = outs
+            assert len(kept) == 1
+        except BaseException as e:                        # noqa: BLE001  (reported by the test's thread)
+            failures.append(repr(e))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+    for i in range(2):
+        for row in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(row, want[i]))
