@@ -37,6 +37,7 @@ struct MmaParams {
     int M, N, K, G;
     int act;                                   // DUAL: the activation (gated_value)
     const float* row_scale;                    // DUAL: both products times row_scale[a_rows[place]] (null: 1)
+    int w_constant;              // nothing in front of this on the stream writes W (which is read before the wait then)
     int vector_out;              // rows of C start on 16 bytes (fp32: 8), a group's columns too, and the factor's pairs on 8
 };
 
@@ -104,8 +105,9 @@ grouped_mma_kernel(MmaParams p) {
     constexpr int NT = WN / 8;                       // n-tiles per warp: 4, 8 or 2
     constexpr int NB = DUAL ? 2 : 1;
     pdl_launch_dependents();
-    const bool listed = p.group_offsets || p.a_rows || p.c_rows || p.row_scale;      // lists come from kernels of the same step, without them only
-    if (listed) pdl_wait();                          // A (and the factor) does, and the weights travel while its kernel ends
+    // lists come from kernels of the same step, without them only A (and the factor) does, and constant weights travel while its kernel ends
+    const bool ahead = p.w_constant && !(p.group_offsets || p.a_rows || p.c_rows || p.row_scale);
+    if (!ahead) pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typedef __nv_bfloat16 (*ATile)[BM][PITCH];
     typedef __nv_bfloat16 (*WTile)[NB][BN][PITCH];
@@ -222,7 +224,7 @@ grouped_mma_kernel(MmaParams p) {
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s)
         if (s < k_tiles) load_w(s, s);
-    if (!listed) pdl_wait();
+    if (ahead) pdl_wait();
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
         if (s < k_tiles) load_a(s, s);
@@ -344,12 +346,12 @@ void launch(const MmaParams& p, int row_tile, unsigned tiles_y, cudaStream_t str
 }  // namespace
 
 // dual_rows > 0: W holds gate rows [0, N) and up rows [dual_rows, dual_rows + N) per group; C = silu(A gate^T) * (A up^T), or the
-// clamped form when `act` holds the bits of its limit.
+// clamped form when `act` holds the bits of its limit.  w_constant != 0: no kernel that may still run in front of this one on the stream writes W.
 MLB_EXPORT int mlb_grouped_mma(const void* A, long long lda, long long a_group_cols, const void* W, long long ldw,
                                long long w_group_stride, void* C, long long ldc, long long c_group_cols,
                                const int* group_offsets, const int* a_rows, const int* c_rows, int a_row_div,
                                const float* factor, long long ldf, long long dual_rows, int M, int N, int K, int G,
-                               int out_dtype, int row_tile, int act, const float* row_scale, cudaStream_t stream) {
+                               int out_dtype, int row_tile, int act, const float* row_scale, int w_constant, cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0 || G <= 0 || a_row_div <= 0 || dual_rows < 0 || (row_tile != 16 && row_tile != 64 && row_tile != 128))
         return fail(MLB_INVALID_ARGUMENT, "grouped_mma: bad sizes M=%d N=%d K=%d G=%d", M, N, K, G);
     if (K % 8 || lda % 8 || ldw % 8 || a_group_cols % 8 || w_group_stride % 8 || (uintptr_t)A % 16 || (uintptr_t)W % 16)
@@ -359,7 +361,7 @@ MLB_EXPORT int mlb_grouped_mma(const void* A, long long lda, long long a_group_c
     if (group_offsets && G > MAX_GROUPS) return fail(MLB_UNSUPPORTED_SIZE, "grouped_mma: more than %d groups", MAX_GROUPS);
     if (M == 0) return MLB_OK;
     MmaParams p{(const __nv_bfloat16*)A, lda, a_group_cols, (const __nv_bfloat16*)W, ldw, w_group_stride, C, ldc, c_group_cols,
-                group_offsets, a_rows, c_rows, a_row_div, factor, ldf, dual_rows, M, N, K, G, act, row_scale, 0};
+                group_offsets, a_rows, c_rows, a_row_div, factor, ldf, dual_rows, M, N, K, G, act, row_scale, w_constant, 0};
     const int unit = out_dtype == MLB_BF16 ? 8 : 2;
     p.vector_out = ldc % unit == 0 && c_group_cols % unit == 0 && (uintptr_t)C % (out_dtype == MLB_BF16 ? 16 : 8) == 0 &&
                    (!factor || (ldf % 2 == 0 && (uintptr_t)factor % 8 == 0));

@@ -28,7 +28,7 @@ MMA_SOURCE = "grouped_mma.cu"
 ops.register_signatures(MMA_SOURCE, {
     "mlb_grouped_mma": [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong,
                         c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_int,
-                        c_int, c_int, c_void_p, c_void_p],
+                        c_int, c_int, c_void_p, c_int, c_void_p],
 })
 
 # CTA pairs on the fifth-generation tensor cores: groups of many rows (csrc/grouped_tc2.cu)
@@ -129,7 +129,8 @@ def row_tile_for(rows: int, groups: int, listed: bool, tensor_cores: bool) -> in
 def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, rows: int, a_group_cols: int = 0,
                    c_group_cols: int = 0, group_offsets: Optional[torch.Tensor] = None, a_rows: Optional[torch.Tensor] = None,
                    c_rows: Optional[torch.Tensor] = None, a_row_div: int = 1, factor: Optional[torch.Tensor] = None,
-                   row_scale: Optional[torch.Tensor] = None, row_tile: int = 64, error_flag: Optional[torch.Tensor] = None) -> None:
+                   row_scale: Optional[torch.Tensor] = None, row_tile: int = 64, error_flag: Optional[torch.Tensor] = None,
+                   w_constant: bool = False) -> None:
     """weight [G, N, K]; a [*, lda] and out [*, ldc] are 2-D and row-major.
 
     group g multiplies the K columns of `a` that start at g * a_group_cols with weight[g] and writes N columns of
@@ -137,7 +138,8 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
     offsets[g]..offsets[g+1]-1 of a sorted list of `rows` places; `a_rows[place] // a_row_div` is the row read and
     `c_rows[place]` the row written (None: the place itself).  Without it every group takes rows 0..rows-1.
     `factor` (fp32, the shape of `out`): the result is multiplied by it element by element.  `row_scale` (fp32, one number per
-    entry that a_rows may name): a row's result is multiplied by row_scale[a_rows[place]] (not on the tensor cores)."""
+    entry that a_rows may name): a row's result is multiplied by row_scale[a_rows[place]] (not on the tensor cores).  `w_constant`: no kernel of the same step
+    writes `weight`, which may then be read while the kernel in front still runs (without lists)."""
     ops._need(a, "a", dims=2); ops._need(weight, "weight", dims=3); ops._need(out, "out", dims=2)
     if a.dtype != weight.dtype:
         raise KernelError(f"grouped_linear: operands are {a.dtype} and {weight.dtype}")
@@ -169,7 +171,7 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, 
             a.data_ptr(), a.stride(0), a_group_cols, weight.data_ptr(), weight.stride(1), weight.stride(0), out.data_ptr(),
             out.stride(0), c_group_cols, ops._ptr(group_offsets), ops._ptr(a_rows), ops._ptr(c_rows), int(a_row_div),
             ops._ptr(factor), factor.stride(0) if factor is not None else 0, 0, int(rows), N, K, G, ops.dtype_tag(out),
-            int(row_tile), 0, None, ops._stream()))
+            int(row_tile), 0, None, 1 if w_constant else 0, ops._stream()))
         return
     L = ops.lib(SOURCE)
     build.check(L, L.mlb_grouped_gemm(
@@ -210,7 +212,7 @@ def grouped_silu_mul(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *
         build.check(L, L.mlb_grouped_mma(
             a.data_ptr(), a.stride(0), 0, weight.data_ptr(), weight.stride(1), weight.stride(0), out.data_ptr(), out.stride(0), 0,
             group_offsets.data_ptr(), ops._ptr(a_rows), None, int(a_row_div), None, 0, F, int(rows), F, K, G,
-            ops.dtype_tag(out), int(row_tile), ops.activation_code(activation, limit), ops._ptr(row_scale), ops._stream()))
+            ops.dtype_tag(out), int(row_tile), ops.activation_code(activation, limit), ops._ptr(row_scale), 0, ops._stream()))
         return
     row_tile = min(row_tile, 64)
     gate_up = alloc((rows, two_f), a.dtype) if alloc is not None else torch.empty((rows, two_f), dtype=a.dtype, device=a.device)

@@ -170,13 +170,13 @@ class LatentAttention(Mixer):
         row_tile = grouped.row_tile_for(T, H, False, grouped.mma_supported(q_plain, self.w_uk_t, self.dim))
         # a_h = Wuk_h^T q_h,plain into the first `rank` columns of each head's query row
         grouped.grouped_linear(q_plain, self.w_uk_t, q_full, rows=T, a_group_cols=self.dim, c_group_cols=self.kv_width,
-                               row_tile=row_tile)
+                               row_tile=row_tile, w_constant=True)
         o_latent = ctx.buffer("latent.o_latent", (T, H * self.rank), dt)
         latent.attention(q_full, cache.pages, o_latent, self.sink, ctx, cache.block_table, H, self.rank, self.rot_dim,
                          self.scale, self.window)
         # o_h = Wuv_h (sum_j p_j c_j), times the gate
         o = ctx.buffer("latent.o", (T, H * self.vdim), dt)
         grouped.grouped_linear(o_latent, self.w_uv, o, rows=T, a_group_cols=self.rank, c_group_cols=self.vdim, factor=gate,
-                               row_tile=row_tile)
+                               row_tile=row_tile, w_constant=True)
         return linear(o, self.w_o, None, torch.float32, partials_ok=True, error_flag=flag,
                       alloc=lambda shape, dtype: ctx.buffer("latent.out", shape, dtype))

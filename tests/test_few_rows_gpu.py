@@ -78,3 +78,23 @@ def test_outputs_stored_together_have_the_bits_of_each_alone(row_tile, out_dtype
             grouped.USE_PAIRS = None
         results.append(out[:, :width])
     assert torch.equal(*results) and int((results[0] == 7.0).sum()) == (len(range(0, rows, 5)) * N if listed else 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w_constant", [False, True])
+def test_products_of_weights_that_the_kernel_in_front_writes(w_constant):
+    """Without the caller's word nothing is read before that kernel has ended; with it the weights are as they were all along."""
+    from microllm_rocm_b200.kernels import grouped, ops
+    G, N, K, rows = 16, 512, 512, 8
+    g = torch.Generator(DEV).manual_seed(1)
+    a = torch.randn(rows, G * K, generator=g, device=DEV).bfloat16()
+    source = torch.randn(8, G, N, K, generator=g, device=DEV)
+    for i in range(8):
+        w, out, want = torch.zeros(G, N, K, dtype=torch.bfloat16, device=DEV), torch.empty(rows, G * N, device=DEV), torch.empty(rows, G * N, device=DEV)
+        ops.cast_f32_bf16(source[i], w)
+        if w_constant:
+            torch.cuda.synchronize()
+        grouped.grouped_linear(a, w, out, rows=rows, a_group_cols=K, c_group_cols=N, row_tile=16, w_constant=w_constant)
+        torch.cuda.synchronize()
+        grouped.grouped_linear(a, w, want, rows=rows, a_group_cols=K, c_group_cols=N, row_tile=16)
+        assert torch.equal(out, want) and bool((want != 0).any())

@@ -108,3 +108,12 @@ def test_library_products_on_second_streams_have_a_workspace_of_their_step(calls
     contexts.clear()
     gc.collect()
     assert gone and not any(r() is not None for r in gone)
+
+
+@pytest.mark.parametrize("w_constant", [False, True])
+def test_a_grouped_products_weights_are_read_ahead_only_on_the_callers_word(calls, monkeypatch, w_constant):
+    """The kernel in front may be the one that writes them."""
+    from microllm_rocm_b200.kernels import grouped
+    a, w = torch.zeros(9, 3 * 64, dtype=torch.bfloat16), torch.zeros(3, 32, 64, dtype=torch.bfloat16)
+    grouped.grouped_linear(a, w, torch.zeros(9, 96), rows=9, a_group_cols=64, c_group_cols=32, **({"w_constant": True} if w_constant else {}))
+    assert calls[0][0] == "mlb_grouped_mma" and calls[0][1].get("w_constant", 1) == int(w_constant)
