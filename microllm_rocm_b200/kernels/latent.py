@@ -178,33 +178,35 @@ def attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, sink: Opt
     if width != rank + rot_dim or q.shape[1] != heads * width or tuple(out.shape) != (T, heads * rank):
         raise KernelError("latent.attention: shapes do not agree")
     work, num_work, splits, groups = _plan(ctx, heads)
-    side = None
+    tc_work = side = None
     if splits == 1 and not ctx.decode_only and GROUPS is None and TCGEN05 is not False and tc_supported(rank, rot_dim, page_size):
         plan = _tc_plan(ctx, heads)
         if plan is not None:
             tc_work, num_tc, work, num_work, groups = plan
-            stream = ops._stream()
-            if num_work:                     # other sequences, other rows: the two launches run side by side
-                side = stream = ops.side_stream()
-                ops.fork(side)
+    if tc_work is not None and num_work:     # other sequences, other rows: the two launches run side by side
+        side = ops.side_stream()
+        ops.fork(side)
+    try:
+        if tc_work is not None:
             L = ops.lib(TC_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})
             build.check(L, L.mlb_latent_attention_tc(
                 q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(), block_table.data_ptr(),
                 tc_work.data_ptr(), num_tc, block_table.shape[1], num_pages, page_size, heads, int(window or 0), T * heads, float(scale),
-                ops._ptr(ctx.error_flag), stream))
+                ops._ptr(ctx.error_flag), ops._stream() if side is None else side))
             if num_work == 0:
                 return
-    part_o = part_ml = None
-    if splits > 1:
-        part_o = ctx.buffer("latent.part_o", (splits, T * heads, rank), torch.float32)
-        part_ml = ctx.buffer("latent.part_ml", (splits, T * heads, 2), torch.float32)
-    L = ops.lib(MMA_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})
-    build.check(L, L.mlb_latent_attention_mma(
-        q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(),
-        block_table.data_ptr(), work.data_ptr(), num_work, ops._ptr(part_o), ops._ptr(part_ml), block_table.shape[1], num_pages,
-        page_size, heads, int(window or 0), splits, groups, T * heads, float(scale), ops._ptr(ctx.error_flag), ops._stream()))
-    if side is not None:
-        ops.join(side)
+        part_o = part_ml = None
+        if splits > 1:
+            part_o = ctx.buffer("latent.part_o", (splits, T * heads, rank), torch.float32)
+            part_ml = ctx.buffer("latent.part_ml", (splits, T * heads, 2), torch.float32)
+        L = ops.lib(MMA_SOURCE, {"LAT_R": rank, "LAT_DR": rot_dim})
+        build.check(L, L.mlb_latent_attention_mma(
+            q.data_ptr(), pages.data_ptr(), out.data_ptr(), ops._ptr(sink), ctx.seq_starts.data_ptr(), ctx.seq_pos0.data_ptr(),
+            block_table.data_ptr(), work.data_ptr(), num_work, ops._ptr(part_o), ops._ptr(part_ml), block_table.shape[1], num_pages,
+            page_size, heads, int(window or 0), splits, groups, T * heads, float(scale), ops._ptr(ctx.error_flag), ops._stream()))
+    finally:
+        if side is not None:                 # (also where a launch is refused: whoever catches that lets go of the tensors, and may be capturing)
+            ops.join(side)
 
 
 def sources():

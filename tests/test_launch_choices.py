@@ -117,3 +117,33 @@ def test_a_grouped_products_weights_are_read_ahead_only_on_the_callers_word(call
     a, w = torch.zeros(9, 3 * 64, dtype=torch.bfloat16), torch.zeros(3, 32, 64, dtype=torch.bfloat16)
     grouped.grouped_linear(a, w, torch.zeros(9, 96), rows=9, a_group_cols=64, c_group_cols=32, **({"w_constant": True} if w_constant else {}))
     assert calls[0][0] == "mlb_grouped_mma" and calls[0][1].get("w_constant", 1) == int(w_constant)
+
+
+@pytest.mark.parametrize("refuses", ["mlb_latent_attention_tc", "mlb_latent_attention_mma", None])
+def test_latent_attention_joins_the_second_stream_whichever_launch_refuses(calls, monkeypatch, refuses):
+    """Whoever catches the error lets go of tensors that the other launch may still use, and may be capturing."""
+    from microllm_rocm_b200.kernels import latent
+    heads, seqs = 16, [(700, 0), (1, 900), (700, 0)]
+    ctx = lists([n for n, _ in seqs])
+    ctx.extras, ctx.seq_pos0_host, ctx.max_seq_len, ctx.positions, ctx.decode_only = {}, [p for _, p in seqs], 901, ctx.token_seq, False
+    monkeypatch.setattr("microllm_rocm_b200.kernels.device.sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "upload", lambda values, dtype, device: torch.tensor(values, dtype=torch.int32))
+    monkeypatch.setattr(ops, "side_stream", lambda: 200)
+    monkeypatch.setattr(ops, "fork", lambda side: calls.append(("fork", side)))
+    monkeypatch.setattr(ops, "join", lambda side: calls.append(("join", side)))
+
+    def check(lib, status):
+        if calls[-1][0] == refuses:
+            raise build.KernelError("refused")
+    monkeypatch.setattr(build, "check", check)
+    T, bf16 = ctx.num_tokens, torch.bfloat16
+    run = lambda: latent.attention(torch.zeros(T, heads * 576, dtype=bf16), torch.zeros(4, 16, 576, dtype=bf16), torch.zeros(T, heads * 512, dtype=bf16), None, ctx,
+                                   torch.zeros(3, 64, dtype=torch.int32), heads, 512, 64, 0.1, None)
+    if refuses is None:
+        run()
+    else:
+        with pytest.raises(build.KernelError, match="refused"):
+            run()
+    names = [name for name, _ in calls]
+    assert names[0] == "fork" and names[-1] == "join" and names.count("join") == 1
+    assert [a["stream"] for name, a in calls if name == "mlb_latent_attention_tc"] == [200]
