@@ -125,6 +125,11 @@ def own_rings_pay(splits: int, max_seq_len: int, beside_mma_products: bool, visi
     return min(max_seq_len, visible) // max(1, splits) >= RINGS_MIN_KEYS_PER_CTA and not beside_mma_products
 
 
+def own_rings_possible(head_dim: int, group: int, splits: int, ring: bool) -> bool:
+    """Whether the launcher has that choice at all (csrc/attention_mma.cu): heads of 128 in groups of up to 8, clusters of up to 8, no TMA ring."""
+    return head_dim == 128 and group <= 8 and splits <= 8 and not ring
+
+
 def decode_plan_stale(ctx, max_seq_len: int, sms: int = DEFAULT_SM_COUNT) -> bool:
     """Whether a decode step planned for `ctx` (its plans are kept in ctx.extras, and frozen into a captured
     graph) would be cut differently at this context length: a step captured at a short context has one CTA
@@ -227,8 +232,10 @@ def paged_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, ctx
         ctx, num_heads // num_kv_heads, num_kv_heads, use_tc, beside_mma_products)
     ring_bits = 4 if (ring if DECODE_RING is None else DECODE_RING) else 8
     visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
-    own = own_rings_pay(splits if mode else listed_splits, ctx.max_seq_len, beside_mma_products, visible)
-    if mode:
+    cut = splits if mode else listed_splits
+    possible = own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring)
+    own = possible and own_rings_pay(cut, ctx.max_seq_len, beside_mma_products, visible)
+    if mode and possible:                # (where there is no choice, a captured step has nothing to be planned again for)
         ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own
     if own if OWN_RINGS is None else OWN_RINGS:
         ring_bits |= 16

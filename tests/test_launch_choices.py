@@ -147,3 +147,34 @@ def test_latent_attention_joins_the_second_stream_whichever_launch_refuses(calls
     names = [name for name, _ in calls]
     assert names[0] == "fork" and names[-1] == "join" and names.count("join") == 1
     assert [a["stream"] for name, a in calls if name == "mlb_latent_attention_tc"] == [200]
+
+
+def paged_step(calls, monkeypatch, head_dim, nkv, group, lens, news=None):
+    """The context behind one call of paged_attention over sequences of `lens` tokens, `news` of them new (one each)."""
+    from microllm_rocm_b200.kernels import attention
+    monkeypatch.setattr(attention, "sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "upload", lambda values, dtype, device: torch.tensor(values, dtype=torch.int32))
+    monkeypatch.setattr(ops, "side_stream", lambda: 200)
+    monkeypatch.setattr(ops, "fork", lambda side: None)
+    monkeypatch.setattr(ops, "join", lambda side: None)
+    news = news or [1] * len(lens)
+    ctx = lists(news)
+    ctx.extras, ctx.seq_pos0_host, ctx.max_seq_len, ctx.positions = {}, [n - k for n, k in zip(lens, news)], max(lens), ctx.token_seq
+    q = torch.zeros(ctx.num_tokens, nkv * group * head_dim, dtype=torch.bfloat16)
+    attention.paged_attention(q, torch.zeros(4, 2, nkv, 16, head_dim, dtype=torch.bfloat16), torch.zeros_like(q), ctx, torch.zeros(len(lens), 8, dtype=torch.int32),
+                              nkv * group, nkv, head_dim, 0.1, None)
+    return ctx
+
+
+@pytest.mark.parametrize("head_dim, nkv, group, lens, later", [
+    (128, 2, 6, [1000] * 4, 3200),                           # 8 CTAs share the keys: the rings take over at 400 keys each
+    (64, 2, 6, [1000] * 4, None), (128, 2, 16, [1000] * 4, None),          # widths and groups that have no rings
+    (128, 2, 6, [1100], None),                               # clusters of 16: none either
+    (128, 4, 7, [9000] * 10, None)])                         # the TMA ring took the step
+def test_a_captured_step_is_planned_again_only_where_another_kernel_would_run(calls, monkeypatch, head_dim, nkv, group, lens, later):
+    from microllm_rocm_b200.kernels import attention
+    ctx = paged_step(calls, monkeypatch, head_dim, nkv, group, lens)
+    plan = next(v for k, v in ctx.extras.items() if k[0] == "attention_mma")
+    assert plan[3] == (16 if len(lens) == 1 else plan[3]) and plan[9] == (len(lens) == 10)
+    at = [n for n in range(max(lens), 20000, 100) if attention.decode_plan_stale(ctx, n, 148)]
+    assert (at[0] if at else None) == later
