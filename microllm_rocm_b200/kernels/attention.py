@@ -189,14 +189,14 @@ def _plan(ctx, group: int, num_kv_heads: int, use_tc: bool, beside_mma_products:
     tc_dev = lists[len(flat_work):len(flat_work) + len(flat_tc)]
     splits = decode_splits(len(work) * num_kv_heads, ctx.max_seq_len, sms) if decode else 1
     ring = decode and decode_ring_pays(len(work) * num_kv_heads, splits, ctx.max_seq_len, sms, beside_mma_products)
-    listed_dev, listed_splits = None, 1
+    listed_dev, listed_splits, longest = None, 1, ctx.max_seq_len if decode else 0         # longest: of the sequences that take the decode shape
     if listed:
         listed_dev = lists[len(flat_work) + len(flat_tc):]
         longest = max(ctx.seq_pos0_host[a] for a in listed) + 1
         listed_splits = decode_splits(len(listed) * tiles_per_token * num_kv_heads, longest, sms)
         ring = decode_ring_pays(len(listed) * tiles_per_token * num_kv_heads, listed_splits, longest, sms, beside_mma_products)
     plan = (work_dev, len(work), 1 if decode else 0, splits, tc_dev, len(tc_work), listed_dev, len(listed) * tiles_per_token,
-            listed_splits, ring)
+            listed_splits, ring, longest)
     ctx.extras[key] = plan
     return plan
 
@@ -228,13 +228,13 @@ def paged_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, ctx
         raise KernelError("paged_attention: the tensor-core kernel wants bf16 queries, pages and output")
     bias_args = ops.distance_bias_args(bias, num_heads)
     use_tc = tc_supported(head_dim, page_size, scale) and q.is_contiguous() and out.is_contiguous()
-    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring = _plan(
+    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring, longest = _plan(
         ctx, num_heads // num_kv_heads, num_kv_heads, use_tc, beside_mma_products)
     ring_bits = 4 if (ring if DECODE_RING is None else DECODE_RING) else 8
     visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
     cut = splits if mode else listed_splits
     possible = own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring)
-    own = possible and own_rings_pay(cut, ctx.max_seq_len, beside_mma_products, visible)
+    own = possible and own_rings_pay(cut, longest, beside_mma_products, visible)
     if mode and possible:                # (where there is no choice, a captured step has nothing to be planned again for)
         ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own
     if own if OWN_RINGS is None else OWN_RINGS:

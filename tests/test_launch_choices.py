@@ -178,3 +178,16 @@ def test_a_captured_step_is_planned_again_only_where_another_kernel_would_run(ca
     assert plan[3] == (16 if len(lens) == 1 else plan[3]) and plan[9] == (len(lens) == 10)
     at = [n for n in range(max(lens), 20000, 100) if attention.decode_plan_stale(ctx, n, 148)]
     assert (at[0] if at else None) == later
+
+
+@pytest.mark.parametrize("lens, news, rings", [
+    ([3000, 200, 300, 250], [512, 1, 1, 1], False),          # a long prompt portion beside short decoded tokens
+    ([3000, 2000, 3900, 200], [512, 1, 1, 1], True), ([3000, 700], [2, 300], False)])
+def test_own_rings_go_by_the_tokens_that_take_them(calls, monkeypatch, lens, news, rings):
+    """Keys a CTA of the listed sequences, not of the prompt portions beside them (which another kernel takes); none where nothing is listed."""
+    from microllm_rocm_b200.kernels import attention
+    ctx = paged_step(calls, monkeypatch, 128, 4, 7, lens, news)
+    plan = next(v for k, v in ctx.extras.items() if k[0] == "attention_mma")
+    decoded = [a for fn, a in calls if fn == "mlb_paged_attention_mma"]
+    assert len(decoded) == (1 if 1 in news else 0) and all(bool(a["mode"] & 16) == rings for a in decoded)
+    assert not decoded or attention.own_rings_pay(plan[8], max(n for n, k in zip(lens, news) if k == 1), False) == rings
