@@ -15,12 +15,12 @@
 //                    accumulator in tensor memory rescaled where any row of the warp has a new maximum
 // The last three spans of the queries lie in tensor memory (an A operand may), which leaves shared memory for a ring of four tiles.
 //
-// 2,048 tokens of 16 heads, 512 + 64 wide: 249 us, latent_mma.cu 427; 512 tokens behind 2,000 158 and 356.  What bounds it is a tile's chain:
+// 2,048 tokens of 16 heads, 512 + 64 wide: 242 us, latent_mma.cu 427; 512 tokens behind 2,000 152 and 356.  What bounds it is a tile's chain:
 // nine dependent steps of four MMAs of 32 columns (the order of the sums asks for them; each takes its 4 KB of queries from shared
 // memory), the scores' way through the softmax, and the accumulator's through registers where a maximum grew.  Measured and no faster:
 // two tiles' scores in tensor memory with weights in their place (251 us: the ring was two tiles short), two threads a row (264).
 //
-// Every wait on an mbarrier is bounded; when a bound is hit the error flag is raised, the CTA waits (bounded) for the copies it
+// Every wait on an mbarrier is bounded; when a bound is hit the error flag is raised, the CTA waits (bounded) for the copies and products it
 // still has in flight, frees its tensor memory and returns.
 #include "common.cuh"
 
@@ -49,7 +49,7 @@ constexpr int Q_TMEM = SPANS > 3 ? 3 : 1, Q_SMEM = SPANS - Q_TMEM;      // spans
 constexpr int Q_BYTES = Q_SMEM * Q_SPAN_BYTES, V_BYTES = OWN * K_SPAN_BYTES, V_BUFS = 3;
 constexpr int SLOTS_FIT = (226 * 1024 - 1024 - Q_BYTES - V_BUFS * V_BYTES) / K_SPAN_BYTES;
 constexpr int SLOTS = SLOTS_FIT > 4 * OTHERS ? 4 * OTHERS : SLOTS_FIT;
-static_assert(SLOTS >= OTHERS, "the ring holds a tile's other spans");
+static_assert(SLOTS >= OTHERS && SLOTS % OTHERS == 0, "the ring holds whole tiles' other spans");
 constexpr int SMEM_BYTES = Q_BYTES + V_BUFS * V_BYTES + SLOTS * K_SPAN_BYTES + 1024;
 constexpr int THREADS = 256;
 constexpr int PRODUCERS = 3, EACH = (SPANS + PRODUCERS - 1) / PRODUCERS;      // warps that copy, spans of each
@@ -58,7 +58,11 @@ constexpr int TMEM_COLS = 512, S_COL = 256, P_COL = S_COL + PARTS * KEYS, Q_COL 
 static_assert(HALF <= S_COL && Q_COL + 32 * Q_TMEM <= TMEM_COLS, "room in tensor memory");
 constexpr int MAX_PAGES_PER_TILE = 4;
 constexpr int PARTLY = BM;                   // keys that only some of 128 rows see: fewer than 128 at either end of a window
-constexpr int SPIN_LIMIT = 1 << 21;          // polls of up to 2 us each
+#ifndef MLB_SPIN_LIMIT                       // (the tests build objects whose waits run out at once)
+#define MLB_SPIN_LIMIT (1 << 21)
+#endif
+constexpr int SPIN_LIMIT = MLB_SPIN_LIMIT;   // polls of up to 2 us each
+constexpr int DRAIN_LIMIT = 1 << 14;         // the same for what is in flight when a wait has run out: microseconds, or never
 
 struct LatentTcParams {
     const __nv_bfloat16* q;         // [rows, DK]
@@ -96,6 +100,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
         if (mbar_try_wait(bar, parity)) return true;
     if (error_flag) atomicCAS(error_flag, 0, code);          // the first failure is the one worth reporting
     return false;
+}
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < DRAIN_LIMIT; ++i)
+        if (mbar_try_wait(bar, parity)) return;
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
@@ -187,9 +195,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     pdl_launch_dependents();
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) unsigned long long q_full, v_full[V_BUFS], v_empty[V_BUFS], slot_full[SLOTS], slot_empty[SLOTS], q_there, s_full, s_empty, p_full[2], pv_done[2],
-        looked;
+        looked, finished, stopped;
     __shared__ uint32_t tmem_base_s;
-    __shared__ int failed_s;
     __shared__ unsigned bad_s[2 * PARTLY / 32];            // keys that some rows see and others do not, whose values are not finite
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -214,7 +221,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             mbar_init(smem_u32(&pv_done[s]), 1);          // P V of the even tiles, and of the odd ones
         }
         mbar_init(smem_u32(&looked), 4);                  // the softmax warps, about values that are not finite
-        failed_s = 0;
+        mbar_init(smem_u32(&finished), 1);                // every product is done,
+        mbar_init(smem_u32(&stopped), 1);                 // or those issued before a wait ran out are
         for (int i = 0; i < 2 * PARTLY / 32; ++i) bad_s[i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -280,13 +288,14 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             if (works) tma_load_2d(dst + box * p.box_rows * ROW_BYTES, &map_kv, span * 64, page * p.page_size + first_key % p.page_size, full);
             loaded = j + 1;
         }
-        __syncwarp();
-        if (works && (loaded < n_tiles || failed_s)) {
-            // give the copies in flight a bounded chance to land before the CTA's memory goes away
-            if (warp == 0 && lane == 0) mbar_wait(smem_u32(&q_full), 0, nullptr, 0);
-            for (int j = max(0, loaded - max(V_BUFS, SLOTS / OTHERS + 1)); j < loaded; ++j)
-                mbar_wait(full_of(j, item0 + j * OTHERS), (own ? j / V_BUFS : (item0 + j * OTHERS) / SLOTS) & 1, nullptr, 0);
+        // Products that are done have had their copies.  Where they never are, or a wait above ran out, the copies in flight get a bounded chance to
+        // land before the CTA's memory goes away: of each buffer the last one (behind it the parity of an earlier one would say the opposite).
+        if (works && !(loaded == n_tiles && mbar_wait(smem_u32(&finished), 0, nullptr, 0))) {
+            if (warp == 0 && lane == 0) mbar_drain(smem_u32(&q_full), 0);
+            for (int j = max(0, loaded - (own ? V_BUFS : SLOTS / OTHERS)); j < loaded; ++j)
+                mbar_drain(full_of(j, item0 + j * OTHERS), (own ? j / V_BUFS : (item0 + j * OTHERS) / SLOTS) & 1);
         }
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issue: one lane, the descriptors made once (a step of 16 bytes
         // is one of their units; put together for each of a tile's 38 instructions they were what bounded it)
@@ -341,7 +350,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 umma_commit(smem_u32(&pv_done[j & 1]));
                 if (++buf_pv == V_BUFS) buf_pv = 0;
             }
-            if (!ok) failed_s = 1;
+            umma_commit(smem_u32(ok ? &finished : &stopped));
+            if (!ok) mbar_drain(smem_u32(&stopped), 0);      // products in flight read shared and write tensor memory
         }
         __syncwarp();
     } else {
@@ -545,7 +555,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 }
             }
         }
-        if (!ok) failed_s = 1;
+        if (!ok) tmem_wait_st();
     }
 
     tc_fence_before();

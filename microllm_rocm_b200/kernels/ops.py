@@ -150,8 +150,9 @@ def lagged_group_sources():
 
 
 def lagged_latent_sources():
-    """And of latent attention's prompts."""
-    return [("latent_tc.cu", {"LAT_R": 512, "LAT_DR": 64, "MLB_LAG_WARP": w}) for w in (0, 1, 2, 5, 7)]
+    """And of latent attention's prompts, with those whose waits run out after so many polls."""
+    return [("latent_tc.cu", {"LAT_R": 512, "LAT_DR": 64, **how}) for how in
+            [{"MLB_LAG_WARP": w} for w in (0, 1, 2, 5, 7)] + [{"MLB_SPIN_LIMIT": n} for n in (0, 1, 4)]]
 
 
 def lib(source: str, defines=None) -> ctypes.CDLL:

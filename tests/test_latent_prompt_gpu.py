@@ -108,3 +108,27 @@ def test_a_held_back_warp_changes_nothing(warp):
         assert torch.equal(run(ctx, q, pages, table, None, heads, None), clean)
     finally:
         ops.TEST_DEFINES.pop("latent_tc.cu")
+
+
+@pytest.mark.parametrize("polls", [0, 1, 4])
+def test_a_wait_that_runs_out_is_reported_and_leaves_nothing_behind(polls):
+    """Every wait gives up after a few polls: the error flag says so (or, where none ran out, the rows are right), the kernel ends, and the next launch is as ever."""
+    from microllm_rocm_b200.kernels import ops
+    heads, seqs = 16, [(150, 200), (64, 0), (40, 700)]
+    ctx, q, pages, table, _ = step(seqs, heads, 16, 9)
+    clean = run(ctx, q, pages, table, None, heads, None)
+    ops.TEST_DEFINES["latent_tc.cu"] = {"MLB_SPIN_LIMIT": polls}
+    latent.TCGEN05 = True
+    try:
+        for _ in range(3):
+            ctx.error_flag.zero_()
+            out = torch.empty_like(clean)
+            latent.attention(q, pages, out, None, ctx, table, heads, RANK, ROT, (RANK + ROT) ** -0.5, None)
+            code = int(ctx.error_flag.item())
+            assert 61 <= code <= 73 if polls == 0 else code == 0 or 61 <= code <= 73
+            assert code != 0 or torch.equal(out, clean)
+    finally:
+        latent.TCGEN05 = None
+        ops.TEST_DEFINES.pop("latent_tc.cu")
+    ctx.error_flag.zero_()
+    assert torch.equal(run(ctx, q, pages, table, None, heads, None), clean)
