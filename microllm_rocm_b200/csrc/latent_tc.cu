@@ -45,12 +45,15 @@ constexpr int PARTS = 4;                                     // partial scores: 
 constexpr int HALF = R / 2;                                  // output columns of a CTA
 constexpr int SPANS = DK / 64, OWN = HALF / 64, OTHERS = SPANS - OWN;
 constexpr int Q_SPAN_BYTES = BM * ROW_BYTES, K_SPAN_BYTES = KEYS * ROW_BYTES;
-constexpr int Q_TMEM = SPANS > 3 ? 3 : 1, Q_SMEM = SPANS - Q_TMEM;      // spans of the queries in tensor memory (an A operand may lie there) and in shared memory
+constexpr int Q_TMEM = 3, Q_SMEM = SPANS - Q_TMEM;      // spans of the queries in tensor memory (an A operand may lie there) and in shared memory
 constexpr int Q_BYTES = Q_SMEM * Q_SPAN_BYTES, V_BYTES = OWN * K_SPAN_BYTES, V_BUFS = 3;
 constexpr int SLOTS_FIT = (226 * 1024 - 1024 - Q_BYTES - V_BUFS * V_BYTES) / K_SPAN_BYTES;
 constexpr int SLOTS = SLOTS_FIT > 4 * OTHERS ? 4 * OTHERS : SLOTS_FIT;
 static_assert(SLOTS >= OTHERS && SLOTS % OTHERS == 0, "the ring holds whole tiles' other spans");
 constexpr int SMEM_BYTES = Q_BYTES + V_BUFS * V_BYTES + SLOTS * K_SPAN_BYTES + 1024;
+// A CTA takes all of its multiprocessor's tensor memory ahead of its wait for the kernel in front.  Were there room for another CTA, one of the launch
+// behind could get the memory that one of this launch is still to get, and wait for this launch: neither would end.
+static_assert(Q_SMEM > 0 && SMEM_BYTES > 200 * 1024, "a CTA has its multiprocessor to itself");
 constexpr int THREADS = 256;
 constexpr int PRODUCERS = 3, EACH = (SPANS + PRODUCERS - 1) / PRODUCERS;      // warps that copy, spans of each
 // Tensor memory: O [0, HALF), a tile's partial scores, two tiles' weights, the last spans of the queries

@@ -56,7 +56,8 @@ def mma_sources(rank: int, rot_dim: int):
 
 
 def tc_supported(rank: int, rot_dim: int, page_size: int = KEYS_PER_TILE) -> bool:
-    return rank % 128 == 0 and 0 < rank <= MAX_RANK and rot_dim == 64 and page_size % 8 == 0 and (KEYS_PER_TILE % page_size == 0 or page_size % KEYS_PER_TILE == 0)
+    """The width that was measured and whose CTA has a multiprocessor to itself (csrc/latent_tc.cu says why it must)."""
+    return rank == 512 and rot_dim == 64 and page_size % 8 == 0 and (KEYS_PER_TILE % page_size == 0 or page_size % KEYS_PER_TILE == 0)
 
 
 def tc_sources(rank: int, rot_dim: int):

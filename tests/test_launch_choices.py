@@ -191,3 +191,12 @@ def test_own_rings_go_by_the_tokens_that_take_them(calls, monkeypatch, lens, new
     decoded = [a for fn, a in calls if fn == "mlb_paged_attention_mma"]
     assert len(decoded) == (1 if 1 in news else 0) and all(bool(a["mode"] & 16) == rings for a in decoded)
     assert not decoded or attention.own_rings_pay(plan[8], max(n for n, k in zip(lens, news) if k == 1), False) == rings
+
+
+def test_the_tcgen05_kernel_of_latent_prompts_takes_only_widths_that_fill_a_multiprocessor():
+    """It asks for all of the tensor memory ahead of its wait for the kernel in front: where two CTAs fit one multiprocessor (128 and 256 wide), one of a launch
+    behind could hold the memory that one of the launch in front still waits for, and wait for that launch."""
+    from microllm_rocm_b200.kernels import latent
+    assert latent.tc_supported(512, 64, 16) and latent.tc_sources(512, 64) == [(latent.TC_SOURCE, {"LAT_R": 512, "LAT_DR": 64})]
+    for rank in (128, 256, 384):
+        assert latent.mma_supported(rank, 64) and not latent.tc_supported(rank, 64, 16) and not latent.tc_sources(rank, 64)
