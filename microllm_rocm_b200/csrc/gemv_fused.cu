@@ -349,16 +349,16 @@ MLB_EXPORT int mlb_gemv_fused_max_k() { return 6144; }
 
 // out[M, I] (bf16) = silu(x Wg^T) * (x Wu^T), Wg = W rows [0, I), Wu = W rows [up_offset, up_offset + I)
 MLB_EXPORT int mlb_gemv_gated(const void* x, long long ldx, const void* w, long long ldw, int w_rows, int up_offset, void* out,
-                              long long ldo, int M, int I, int K, int act, cudaStream_t stream);
+                              long long ldo, int M, int I, int K, int act, int beside, cudaStream_t stream);
 
 MLB_EXPORT int mlb_gemv_silu(const void* x, long long ldx, const void* w, long long ldw, int w_rows, int up_offset, void* out,
                              long long ldo, int M, int I, int K, cudaStream_t stream) {
-    return mlb_gemv_gated(x, ldx, w, ldw, w_rows, up_offset, out, ldo, M, I, K, 0, stream);
+    return mlb_gemv_gated(x, ldx, w, ldw, w_rows, up_offset, out, ldo, M, I, K, 0, 0, stream);
 }
 
-// the same with the gate's activation chosen: act = 0 silu, 1 the tanh form of gelu
+// the same with the gate's activation chosen: act = 0 silu, 1 the tanh form of gelu; beside != 0: another stream's kernels run at the same time
 MLB_EXPORT int mlb_gemv_gated(const void* x, long long ldx, const void* w, long long ldw, int w_rows, int up_offset, void* out,
-                              long long ldo, int M, int I, int K, int act, cudaStream_t stream) {
+                              long long ldo, int M, int I, int K, int act, int beside, cudaStream_t stream) {
     if (act < 0) return fail(MLB_INVALID_ARGUMENT, "gemv_gated: unknown activation %d", act);
     int status = check_operands("gemv_silu", x, ldx, w, ldw, M, K);
     if (status != MLB_OK) return status;
@@ -377,9 +377,13 @@ MLB_EXPORT int mlb_gemv_gated(const void* x, long long ldx, const void* w, long 
         if (status != MLB_OK) return status;
         // A grid that leaves multiprocessors room for more CTAs than their share waits for its predecessor the plain way: started early it
         // lands wherever that one leaves room, four CTAs on some SMs, one or none on others, and the fullest SM decides.  Width 2,048, 352 CTAs behind the
-        // 2,048-wide projection of two mixers: 27.7 us a layer started early, 13 so (a turn of 8 decode steps of 4 requests 7.28 -> 6.60 ms); 560 CTAs,
-        // four a multiprocessor, fill the device either way and gain their early weights (8 steps of one request 8.26 ms early, 8.32 not).
-        if (blocks <= 3u * (unsigned)sm_count()) gemv_silu_kernel<1><<<blocks, SILU_WARPS * 32, smem, stream>>>(p);
+        // 2,048-wide projection of two mixers: 27.7 us a layer started early, 13 so; 560 CTAs, four a multiprocessor, fill the device either way
+        // and gain their early weights.  Decode steps of 1, 4 and 8 requests, us, early / plain: 352 CTAs 418 / 375, 471 / 397, 463 / 436 (four
+        // layers of matidra-3b-layers), 417 / 413, 456 / 452, 440 / 439 (lozepel-3b-layers); 176 CTAs of width 1,024 180 / 171, 188 / 184, 217 / 211 (matidra-small);
+        // one of 1.5B's (560) 8,260 / 8,320 for 8 steps.  On a second stream, beside the router's kernels (a shared expert), the weights
+        // are worth more than the places: 64 CTAs 506 / 523, 533 / 562, 566 / 563, 88 CTAs 270 / 281, 317 / 328, 337 / 337, 176 CTAs 971 / 1,002,
+        // 1,358 / 1,420, 1,488 / 1,480 and 531 / 544, 611 / 635, 639 / 659 (gedalix-small, fonuvik-small, gedalix-16b-layers, fonuvik-3b-layers).
+        if (!beside && blocks <= 3u * (unsigned)sm_count()) gemv_silu_kernel<1><<<blocks, SILU_WARPS * 32, smem, stream>>>(p);
         else launch_kernel(gemv_silu_kernel<1>, blocks, SILU_WARPS * 32, smem, stream, p);
     } else {
         status = reserve(gemv_silu_kernel<2>, smem, configured2, "gemv_silu");

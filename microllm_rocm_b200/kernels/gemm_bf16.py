@@ -29,7 +29,7 @@ ops.register_signatures("gemv_fused.cu", {
                        c_int, c_void_p],
     "mlb_gemv_silu": [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_int, c_int, c_int,
                       c_void_p],
-    "mlb_gemv_gated": [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p],
+    "mlb_gemv_gated": [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "mlb_gemv_qkv_rope": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                           c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                           c_void_p],
@@ -188,7 +188,7 @@ def gemv_silu_mul(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, acti
         raise KernelError("gemv_silu_mul: the weight must hold gate rows then up rows, the output be bf16 [M, I]")
     L = ops.lib("gemv_fused.cu")
     build.check(L, L.mlb_gemv_gated(x.data_ptr(), x.stride(0), weight.data_ptr(), weight.stride(0), 2 * I, I, out.data_ptr(),
-                                    out.stride(0), M, I, K, ops.activation_code(activation, limit), ops._stream()))
+                                    out.stride(0), M, I, K, ops.activation_code(activation, limit), 0 if ops.second_stream()[0] is None else 1, ops._stream()))
 
 
 def gemv_qkv_rope(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], positions: torch.Tensor,

@@ -200,3 +200,15 @@ def test_the_tcgen05_kernel_of_latent_prompts_takes_only_widths_that_fill_a_mult
     assert latent.tc_supported(512, 64, 16) and latent.tc_sources(512, 64) == [(latent.TC_SOURCE, {"LAT_R": 512, "LAT_DR": 64})]
     for rank in (128, 256, 384):
         assert latent.mma_supported(rank, 64) and not latent.tc_supported(rank, 64, 16) and not latent.tc_sources(rank, 64)
+
+
+def test_a_gated_few_row_product_on_the_second_stream_says_so(calls, monkeypatch):
+    """There it starts early whatever its grid: its weights travel beside the first stream's kernels."""
+    from microllm_rocm_b200.kernels import gemm_bf16
+    monkeypatch.setattr(ops, "side_stream", lambda: 200)
+    x, w, out = (torch.zeros(*s, dtype=torch.bfloat16) for s in ((4, 64), (64, 64), (4, 32)))
+    gemm_bf16.gemv_silu_mul(x, w, out)
+    with ops.on_side_stream():
+        gemm_bf16.gemv_silu_mul(x, w, out)
+    gemm_bf16.gemv_silu_mul(x, w, out)
+    assert [a.get("beside") for fn, a in calls if fn == "mlb_gemv_gated"] == [0, 1, 0]
