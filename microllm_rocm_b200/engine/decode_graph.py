@@ -126,6 +126,7 @@ class DecodeGraph:
         self.dev.copy_(self.host, non_blocking=True)
         self._mark_upload()
         self.ctx.max_seq_len = max(lengths) + 1
+        self.ctx.mean_seq_len = (sum(lengths) + A) / A             # (the filling rows' sequences are one token long)
 
     def _mark_upload(self) -> None:
         self._upload_pending = True

@@ -186,7 +186,7 @@ class Engine:
             block_tables={g: d(s_tables[g]).view(A, widths[g]) for g in groups},
             state_slots=d(s_slots), logit_rows=d(s_rows), error_flag=self.error_flag,
             seq_starts_host=[int(x) for x in starts], seq_pos0_host=list(pos0), state_slots_host=slots_host,
-            max_new_tokens=max(counts), max_seq_len=max(p + n for p, n in zip(pos0, counts)))
+            max_new_tokens=max(counts), max_seq_len=max(p + n for p, n in zip(pos0, counts)), mean_seq_len=sum(p + n for p, n in zip(pos0, counts)) / A)
 
     # ------------------------------------------------------------------ the step
     def step(self, entries: Sequence[StepEntry], tensor_sink=None, patch=None) -> torch.Tensor:

@@ -116,13 +116,30 @@ def decode_ring_pays(items: int, splits: int, max_seq_len: int, sms: int = DEFAU
 
 
 def own_rings_pay(splits: int, max_seq_len: int, beside_mma_products: bool, visible: int = 1 << 30) -> bool:
-    """Whether the decode kernel that has its keys in registers gets them by way of its warps' own rings in shared memory: from 400 keys a CTA
-    on (of the `visible` last ones, where a window ends them), away from the few-token mma.sync products (whose shared memory then finds no room early: 8 requests of 2,048 on the 1.5B shapes
-    5,230 -> 7,800 us).  Measured in whole decode steps, heads of 128 (us for four steps, registers / rings): 7B 4 x 6,144 (768 keys a CTA)
-    14,990 / 14,490, 1 x 6,144 13,950 / 13,470, 5 x 4,000 13,760 / 13,430, 7 of 300 to 3,400 12,930 / 12,810; 1.5B 41 of 64 to 2,048
-    (1,024) 8,800 / 8,340; 30 of 80 to 800 13,430 / 13,420.  Below: 7B 8 x 2,048 (256) 13,340 / 13,640, 8 of 1,000 to 3,000 13,320 / 13,450;
-    1.5B 32 of 300 to 700 (175) 5,990 / 6,060; but 16 x 2,048 6,400 / 6,150."""
+    """Whether the keys of a decode step are enough for its kernel's warps to get them by way of rings of their own in shared memory, where
+    `own_rings_suit` says that the step's shape is one for it: from 400 keys a CTA on (of the `visible` last ones, where a window ends
+    them), away from the few-token mma.sync products (whose shared memory then finds no room early: 8 requests of 2,048 on the 1.5B shapes
+    5,230 -> 7,800 us).  Below, the gain gets small and then turns (four decode steps, us, registers / rings): 250 keys a CTA 7B 1 x 2,048
+    12,620 / 12,410, 1.5B 16 x 2,048 6,040 / 5,870, 20 x 1,024 5,920 / 5,910, 40 x 512 6,790 / 6,840."""
     return min(max_seq_len, visible) // max(1, splits) >= RINGS_MIN_KEYS_PER_CTA and not beside_mma_products
+
+
+def own_rings_suit(sequences: int, splits: int, ctas: int, even: float, sms: int = DEFAULT_SM_COUNT) -> bool:
+    """Whether a decode step of `sequences` sequences on `ctas` CTAs has the shape for the warps' own rings; `even`: the mean length of the sequences
+    over the longest.  The rings shorten the way of one CTA through its keys.  Up to 16 sequences that is what the step waits for; more of about
+    one length draw the device's bandwidth either way, and the rings' shared memory keeps the next product from starting early.
+    Four decode steps, heads of 128, us, registers / rings:
+      * up to 16: 7B 1 x 4,096 13,360 / 12,840, 4 x 4,096 13,990 / 13,620, 6 x 7,000 15,090 / 14,420, 10 x 2,400 14,180 / 13,780, 16 x 3,000 14,870 / 14,360;
+        14B 4 x 4,096 32,490 / 31,610, 8 x 3,600 32,310 / 30,950, 16 x 1,500 31,530 / 30,570; 1.5B 9 x 5,000 7,020 / 6,700, 16 x 3,300 6,650 / 6,390;
+      * but eight of one length on clusters of eight: 7B 8 x 3,300 13,610 / 13,920, 8 x 4,096 14,080 / 14,410, 8 x 6,144 15,090 / 15,150; of lengths whose mean is
+        0.9, 0.77 and 0.55 of 6,144: 14,890 / 14,900, 14,770 / 14,510, 14,620 / 14,060; seven of 4,096 13,880 / 13,520;
+      * more, of one length: 7B 20 x 1,000 13,620 / 13,820, 28 x 820 13,710 / 13,750, 28 x 1,950 15,330 / 15,260, 40 x 900 15,720 / 15,650; 14B 40 x 900 37,880 / 37,800;
+        1.5B 24 x 1,700 6,410 / 6,500, 34 x 1,700 8,390 / 8,570, 60 x 1,500 8,160 / 8,370, 80 x 900 9,170 / 9,280;
+      * more, the mean 0.5, 0.3 and 0.15 of the longest: 1.5B 24 x 2,000 6,350 / 6,360, 6,310 / 6,190, 6,240 / 6,030; 64 x 1,900 8,710 / 8,740, 8,560 / 8,330, 8,540 / 8,160;
+        72 x 900 8,710 / 8,920, 8,860 / 8,620, 8,830 / 8,460; 7B 20 x 1,900 14,590 / 14,690, 14,550 / 14,590, 14,430 / 14,020."""
+    if sequences > 16:
+        return even <= 0.35
+    return not (4 < sequences <= 8 and splits == 8 and ctas > 1.6 * sms and even > 0.88)
 
 
 def own_rings_possible(head_dim: int, group: int, splits: int, ring: bool) -> bool:
@@ -189,14 +206,17 @@ def _plan(ctx, group: int, num_kv_heads: int, use_tc: bool, beside_mma_products:
     tc_dev = lists[len(flat_work):len(flat_work) + len(flat_tc)]
     splits = decode_splits(len(work) * num_kv_heads, ctx.max_seq_len, sms) if decode else 1
     ring = decode and decode_ring_pays(len(work) * num_kv_heads, splits, ctx.max_seq_len, sms, beside_mma_products)
-    listed_dev, listed_splits, longest = None, 1, ctx.max_seq_len if decode else 0         # longest: of the sequences that take the decode shape
+    # longest and mean length of the sequences that take the decode shape
+    listed_dev, listed_splits, longest = None, 1, ctx.max_seq_len if decode else 0
+    mean = getattr(ctx, "mean_seq_len", 0) or longest
     if listed:
         listed_dev = lists[len(flat_work) + len(flat_tc):]
-        longest = max(ctx.seq_pos0_host[a] for a in listed) + 1
+        lengths = [ctx.seq_pos0_host[a] + 1 for a in listed]
+        longest, mean = max(lengths), sum(lengths) / len(lengths)
         listed_splits = decode_splits(len(listed) * tiles_per_token * num_kv_heads, longest, sms)
         ring = decode_ring_pays(len(listed) * tiles_per_token * num_kv_heads, listed_splits, longest, sms, beside_mma_products)
     plan = (work_dev, len(work), 1 if decode else 0, splits, tc_dev, len(tc_work), listed_dev, len(listed) * tiles_per_token,
-            listed_splits, ring, longest)
+            listed_splits, ring, longest, mean)
     ctx.extras[key] = plan
     return plan
 
@@ -228,12 +248,14 @@ def paged_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, ctx
         raise KernelError("paged_attention: the tensor-core kernel wants bf16 queries, pages and output")
     bias_args = ops.distance_bias_args(bias, num_heads)
     use_tc = tc_supported(head_dim, page_size, scale) and q.is_contiguous() and out.is_contiguous()
-    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring, longest = _plan(
+    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring, longest, mean = _plan(
         ctx, num_heads // num_kv_heads, num_kv_heads, use_tc, beside_mma_products)
     ring_bits = 4 if (ring if DECODE_RING is None else DECODE_RING) else 8
     visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
     cut = splits if mode else listed_splits
-    possible = own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring)
+    possible = own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring) and own_rings_suit(
+        num_work if mode else num_listed, cut, (num_work if mode else num_listed) * num_kv_heads * cut,
+        min(mean, visible) / max(1, min(longest, visible)), sm_count(q.device))
     own = possible and own_rings_pay(cut, longest, beside_mma_products, visible)
     if mode and possible:                # (where there is no choice, a captured step has nothing to be planned again for)
         ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own

@@ -161,6 +161,7 @@ class StepContext:
     # (residual stream and the delta not yet added to it), after the final norm and for the logits: a per-step
     # tensor trace.  Such a step runs every layer call by call.
     tensor_sink: Optional[Callable[[str, torch.Tensor], None]] = None
+    mean_seq_len: float = 0.0      # mean length of the sequences after the step (0: not known, taken for the longest)
 
     @property
     def decode_only(self) -> bool:

@@ -160,6 +160,7 @@ def paged_step(calls, monkeypatch, head_dim, nkv, group, lens, news=None):
     news = news or [1] * len(lens)
     ctx = lists(news)
     ctx.extras, ctx.seq_pos0_host, ctx.max_seq_len, ctx.positions = {}, [n - k for n, k in zip(lens, news)], max(lens), ctx.token_seq
+    ctx.mean_seq_len = sum(lens) / len(lens)
     q = torch.zeros(ctx.num_tokens, nkv * group * head_dim, dtype=torch.bfloat16)
     attention.paged_attention(q, torch.zeros(4, 2, nkv, 16, head_dim, dtype=torch.bfloat16), torch.zeros_like(q), ctx, torch.zeros(len(lens), 8, dtype=torch.int32),
                               nkv * group, nkv, head_dim, 0.1, None)
@@ -212,3 +213,17 @@ def test_a_gated_few_row_product_on_the_second_stream_says_so(calls, monkeypatch
         gemm_bf16.gemv_silu_mul(x, w, out)
     gemm_bf16.gemv_silu_mul(x, w, out)
     assert [a.get("beside") for fn, a in calls if fn == "mlb_gemv_gated"] == [0, 1, 0]
+
+
+@pytest.mark.parametrize("nkv, group, lens, rings", [
+    (4, 7, [4096], True), (4, 7, [4096] * 4, True), (8, 5, [4096] * 4, True), (4, 7, [4096] * 7, True), (4, 7, [3000] * 12, True), (2, 6, [4000] * 16, True),
+    (4, 7, [4096] * 8, False), (4, 7, [4096, 600, 2000, 900, 4000, 300, 1500, 3000], True), (8, 5, [2400] * 8, True),      # eight of one length on clusters of eight
+    (2, 6, [1700] * 24, False), (2, 6, [900] * 48, False), (2, 6, [900] * 72, False), (4, 7, [1000] * 20, False),             # many of one length
+    (2, 6, [100 + 40 * i for i in range(41)] + [300] * 7, False), (2, 6, [300] * 40 + [1900], True), (2, 6, [80] * 30, False)])   # many, one or a few much longer
+def test_own_rings_are_taken_where_they_were_the_faster_ones(calls, monkeypatch, nkv, group, lens, rings):
+    """The same bits either way: sequences of one length that fill the device by their number were 1 to 3 % slower with them."""
+    from microllm_rocm_b200.kernels import attention
+    ctx = paged_step(calls, monkeypatch, 128, nkv, group, lens)
+    plan = next(v for k, v in ctx.extras.items() if k[0] == "attention_mma")
+    decoded = [a for fn, a in calls if fn == "mlb_paged_attention_mma"]
+    assert not plan[9] and len(decoded) == 1 and bool(decoded[0]["mode"] & 16) == rings
