@@ -22,9 +22,9 @@ def step(counts, pos0):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dk, dv, alike", [(128, 128, True), (96, 52, True), (64, 64, True), (30, 37, False), (200, 40, True)])
+@pytest.mark.parametrize("dk, dv", [(128, 128), (96, 52), (64, 64), (30, 37), (200, 40)])
 @pytest.mark.parametrize("rule", ["delta", "decayed_sum", "bonus_read", "head", "head and vector"])
-def test_many_sequences_have_the_bits_of_each_alone(rule, dk, dv, alike):
+def test_many_sequences_have_the_bits_of_each_alone(rule, dk, dv):
     """Sequences together fill the device and take two columns a lane, one alone takes one; portions of one token, of part of a staged chunk and
     of several, some from a state and some from zero."""
     from microllm_rocm_b200.kernels import recurrent
@@ -54,7 +54,7 @@ def test_many_sequences_have_the_bits_of_each_alone(rule, dk, dv, alike):
         assert int(ctx.error_flag.item()) == 0
         return o, state[:len(which)], n_state[:len(which)], den
 
-    together = run(list(range(A)) * 1)
+    together = run(list(range(A)))
     at = 0
     for a in range(A):
         o, state, n_state, den = run([a])
@@ -110,7 +110,7 @@ def test_sequences_without_tokens_beside_others(counts, C):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("family, dtype", [("matidra", "float32"), ("matidra", "bfloat16"), ("naburax", "float32"), ("lozepel", "bfloat16"), ("fonuvik", "bfloat16")])
-def test_branches_side_by_side_have_the_bits_of_one_after_another(tmp_path, family, dtype):
+def test_branches_side_by_side_have_the_bits_of_one_after_another(family, dtype):
     """A prompt, a step that decodes beside a prompt portion, and decoded tokens."""
     from microllm_rocm_b200.config import find_preset
     from microllm_rocm_b200.engine.loading import make_engine, prepare_kernels, require_gpu, resolve_dtype
@@ -183,3 +183,46 @@ def test_library_products_on_the_second_streams_of_two_threads():
     for i in range(2):
         for row in got[i]:
             assert all(torch.equal(a, b) for a, b in zip(row, want[i]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("preset, prompt, requests", [("matidra-tiny", 40, 3), ("lozepel-tiny", 40, 2), ("matidra-3b-layers", 700, 2), ("lozepel-3b-layers", 300, 1)])
+def test_branches_side_by_side_in_prompts_of_library_products_and_in_captured_steps(preset, prompt, requests):
+    """Logits of a prompt (of hundreds of tokens: products of the library on both streams), then of captured steps, against one branch after the other."""
+    from microllm_rocm_b200.config import find_preset
+    from microllm_rocm_b200.engine.decode_graph import DecodeGraphPool
+    from microllm_rocm_b200.engine.loading import random_engine
+    from microllm_rocm_b200.engine.step import StepEntry
+    from microllm_rocm_b200.kernels.build import LaunchCounter
+    from microllm_rocm_b200.parts import parallel
+    from microllm_rocm_b200.sampling import GenerationConfig
+    results, products = [], 0
+    for side in (False, True):
+        parallel.SIDE_BY_SIDE = side
+        try:
+            engine = random_engine(find_preset(preset)[1], seed=5, dtype="bfloat16", max_tokens=2048, max_requests=requests, draw_on_device=True)
+            ids = [f"{i}" for i in range(requests)]
+            for rid in ids:
+                engine.cache.add(rid)
+            before = LaunchCounter.library
+            out = [engine.step([StepEntry(rid, [(7 * i + 3 * t) % 250 for t in range(prompt - i)], [prompt - i - 1]) for i, rid in enumerate(ids)]).clone()]
+            products = LaunchCounter.library - before
+            for rid in ids:
+                assert engine.cache.reserve(rid, prompt + 8)
+            graph, kept = DecodeGraphPool(engine).get(ids, headroom_tokens=8), {}
+            graph.ctx.tensor_sink = lambda name, t: kept.__setitem__(name, t) if name == "logits" else None
+            load = lambda: graph.load(ids, [3] * requests, [prompt - i for i in range(requests)], [GenerationConfig(max_new_tokens=8, temperature=0.0)] * requests, [0] * requests)
+            load()
+            graph.capture()
+            load()
+            for _ in range(4):
+                graph.replay()
+                out.append(kept["logits"][:requests].clone())
+                out.append(torch.tensor(graph.read_tokens(), device=DEV))
+            engine.check_device_errors()
+            results.append(out)
+        finally:
+            parallel.SIDE_BY_SIDE = True
+    assert products > 0 or prompt < 300
+    for a, b in zip(*results):
+        assert torch.equal(a, b) and bool(torch.isfinite(a.float()).all())
