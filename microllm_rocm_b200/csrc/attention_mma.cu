@@ -1048,9 +1048,6 @@ __device__ __forceinline__ void merge_and_store_t(const FaParams& p, const TileG
     cluster.sync();                          // nobody leaves while its shared memory may still be read
 }
 
-// shared memory (dynamic): queries | per-warp fragments [DW][FRAGS_T][32] | warp max/sum per head |
-// this CTA's merged heads [8][D] with their max and sum | block table
-
 // A thread's own pieces of a key tile (what load_keys leaves in its registers) on their way to its own places in shared memory, [piece][lane]:
 // nobody else reads them, so waiting for its own copies is all that a thread needs.  False where the page is not there.
 constexpr int TILE_PIECES = 2 * KCHUNKS + 4 * VBLOCKS;
@@ -1096,6 +1093,8 @@ __device__ __forceinline__ void take_keys(const uint4* slot, int base, KeyTile& 
         for (int r = 0; r < 4; ++r) kv.v[vb][r] = at[(2 * KCHUNKS + vb * 4 + r) * 32];
 }
 
+// shared memory (dynamic): queries | per-warp fragments [DW][FRAGS_T][32], or the warps' rings [DW][depth][TILE_PIECES][32] of 16 bytes, then
+// their fragments | warp max/sum per head | this CTA's merged heads [8][D] with their max and sum | block table
 constexpr size_t decode_t_smem(int dw, int depth = 0) {
     return 16 * Q_STRIDE * sizeof(__nv_bfloat16) + (size_t)dw * 128 * (depth > 0 ? depth * TILE_PIECES * 4 : FRAGS_T) + 2 * dw * 8 * sizeof(float) +
            (size_t)8 * D * sizeof(float) + 16 * sizeof(float) + TABLE_SPAN * sizeof(int);
@@ -1105,6 +1104,7 @@ constexpr size_t decode_t_smem(int dw, int depth = 0) {
 // registers.  The tiles of a warp, their order and what the products see are the same, and so are the bits.  Two tiles a ring (74 KB a CTA of four
 // warps) leave two CTAs a multiprocessor; three, four and six gave less (decode of 4 x 6,144 tokens on the 7B shapes, four steps: 14,990 us in
 // registers, 14,490 with two, 14,270 with three, but 41 requests of 64 to 2,048 on the 1.5B 8,830 / 8,350 / 8,370, and one CTA a multiprocessor 15,900).
+// Which steps take them: own_rings_suit and own_rings_pay in kernels/attention.py, with what both sides measured.
 [[maybe_unused]] constexpr int RING_DEPTH = 2;
 template <int DW, int DEPTH>
 __global__ void __launch_bounds__(DW * 32, DW == 4 ? 2 : 1) fa_decode_t_kernel(FaParams p) {

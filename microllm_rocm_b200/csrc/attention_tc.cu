@@ -195,8 +195,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // What bounds a tile is the softmax warps' serial path and, in short prompts, the trip of their instructions from memory: maxima of three
-// operands, pairs in one instruction, P where the scores were, and the rarely taken loops (rescaling, epilogue) rolled up.  12 query heads of
-// 128, 28 layers: 4.1 us a layer less in a prompt of 45 tokens (one tile; 1,894 -> 1,780 us) and 4.7 in one of 2,048 (7,220 -> 7,087), same bits.
+// operands, pairs in one instruction, P where the scores were, and the rarely taken loops (rescaling, epilogue) rolled up.  The kernel in a row of
+// its own, heads of 128, us, before / so: 12 heads, 45 tokens (one tile) 8.3 / 7.7, 512 14.3 / 13.4, 2,048 34.2 / 32.0; 28 heads, 2,048 68.7 / 63.9; same
+// bits.  Whole prompts move by 1 to 5 %, little more than two runs of one side differ.
 // The largest of a row's scores: eight chains of three operands a step.
 __device__ __forceinline__ float row_max(const uint32_t (&s)[BN]) {
     float m[8];

@@ -183,7 +183,8 @@ gemm_f32_stream_kernel(const float* __restrict__ A, const float* __restrict__ W,
 
 // ------------------------------------------------------------------------------------------------------- many rows of A
 // Rows of a stage lie 36 floats apart: eight neighbouring rows' same piece fall into eight different groups of banks.  Per four
-// elements of K a thread reads 8 + 4 pieces and issues 64 packed FMAs, so the FMA pipe and not shared memory is the limit.
+// elements of K a thread reads RI + 4 pieces of 16 bytes and issues 8 RI packed FMAs (RI = 5 to 8, an eighth of the tile's rows): full tiles reach 38
+// of the FMA pipe's 74 TFLOP/s, the reads of shared memory beside it.
 constexpr int BN = 64, TILE_STAGES = 3, PITCH = STEP + 4;
 constexpr int stage_floats(int ri) { return (8 * ri + BN) * PITCH; }
 constexpr int tile_smem(int ri) { return TILE_STAGES * stage_floats(ri) * 4; }
@@ -259,7 +260,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     wait_groups<0>();
     __syncthreads();
     constexpr int OUT_PITCH = BN + 4;
-    float* mine = tiles;                                                  // the quarter's 64 x 64 sums, over the ring
+    float* mine = tiles;                                                  // the quarter's 8 RI x 64 sums, over the ring
 #pragma unroll
     for (int i = 0; i < RI; ++i)
 #pragma unroll

@@ -106,6 +106,7 @@ grouped_mma_kernel(MmaParams p) {
     constexpr int NB = DUAL ? 2 : 1;
     pdl_launch_dependents();
     // lists come from kernels of the same step, without them only A (and the factor) does, and constant weights travel while its kernel ends
+    // (two products a layer, 8 requests, 8 layers, eight decode steps: 12,310 us with the weights behind the wait, 12,060 so)
     const bool ahead = p.w_constant && !(p.group_offsets || p.a_rows || p.c_rows || p.row_scale);
     if (!ahead) pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -114,9 +114,9 @@ def _plan(ctx, heads: int):
 def tc_pays(tiles: int, mean_keys: float) -> bool:
     """Whether a step's sequences of 128 (token, head) rows and more, `tiles` tiles of 128 rows whose tokens see `mean_keys` keys, go to the tcgen05
     kernel: a CTA takes 9 us before its first tile of keys and 1.8 for each, so many tiles want 64 keys and few tiles thousands.
-    Measured (512 + 64 wide, 148 SMs, us, mma.sync / tcgen05): 16 heads, a prompt of 2,048 tokens 427 / 249, 1,024 118 / 78, 512 47 / 41, 256 26 / 25,
-    128 13 / 18; 512 behind 2,000 356 / 158, 64 behind 2,000 130 / 120; 8 times 128 tokens 32.6 / 30.4, 45 13 / 15, 16 behind 1,000 80 / 66,
-    8 behind 1,000 62 / 66; 40 times 40 35.0 / 36.3; 4 heads, 2,048 tokens 163 / 126, 512 36.8 / 38.3; 64 heads, 128 tokens 22 / 19."""
+    Measured (512 + 64 wide, 148 SMs, us, mma.sync / tcgen05): 16 heads, a prompt of 2,048 tokens 427 / 242, 1,024 118 / 78, 512 47 / 41, 256 26 / 25,
+    128 13 / 18; 512 behind 2,000 356 / 152, 64 behind 2,000 130 / 120; 8 times 128 tokens 32.6 / 30.4, 45 13 / 15, 16 behind 1,000 80 / 66,
+    8 behind 1,000 62 / 66; 40 times 40 35.0 / 36.3; 4 heads, 2,048 tokens 163 / 122, 512 36.8 / 38.3; 64 heads, 128 tokens 22 / 19."""
     return (tiles >= 32 and mean_keys >= 64) or tiles * mean_keys >= 12000
 
 
@@ -143,6 +143,10 @@ def _tc_plan(ctx, heads: int):
         return ops.upload([x for _, a, first in work for x in (a, first)], "int32", device) if work else None, len(work)
     plan = None
     if 0 < tiles < 65536 and (TCGEN05 or tc_pays(tiles, mean)):
+        # Two groups a CTA from five tiles a multiprocessor on and not from four, as two_groups_pay has it for tiles that see as many keys: beside the other
+        # kernel the CTAs do not all run at once.  16 heads, beside a prompt of 700, us, one / two: 85 x 7 tokens behind 1,500 (595 tiles) 366 / 404, 90 x 7 behind
+        # 500 165 / 169, 100 x 7 behind 1,000 (700) 288 / 294, 600 x 1 behind 300 119 / 151, but 160 x 4 behind 1,000 (640) 284 / 254; 110 x 7 behind 200
+        # (770) 105 / 108, 130 x 7 behind 800 (910) 303 / 260, 400 x 2 behind 300 (800) 136 / 135.
         groups = 2 if sum(-(-rows[a] // ROWS_PER_TILE) for a in rest) >= 5 * sms else 1
         plan = (*upload(TC_ROWS_PER_TILE, [a for a in range(ctx.num_seqs) if takes[a]]), *upload(groups * ROWS_PER_TILE, rest), groups)
     ctx.extras[key] = plan
