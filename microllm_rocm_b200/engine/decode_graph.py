@@ -80,7 +80,8 @@ class DecodeGraph:
             seq_starts=d("seq_starts"), seq_pos0=d("seq_pos0"), seq_lens=d("seq_lens"),
             block_tables={g: self.dev[v[0]:v[1]].view(A, self.widths[g]) for g, v in self._tables.items()},
             state_slots=d("slots"), logit_rows=d("logit_rows"), error_flag=engine.error_flag,
-            seq_starts_host=list(range(A + 1)), seq_pos0_host=[], state_slots_host=[], max_new_tokens=1, max_seq_len=1)
+            seq_starts_host=list(range(A + 1)), seq_pos0_host=[], state_slots_host=[], max_new_tokens=1, max_seq_len=1,
+            captured=True)
         self.views = engine.cache_views(self.ctx)
         self._planners = list({b.mixer.plan_group(): b.mixer for b in engine.model.blocks}.values())    # one mixer per shared plan
         self.graph: Optional[torch.cuda.CUDAGraph] = None

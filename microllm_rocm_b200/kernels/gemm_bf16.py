@@ -11,6 +11,7 @@ Grid sizes and K splits follow the multiprocessor count of the device the operan
 """
 from __future__ import annotations
 
+import threading
 from ctypes import c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -57,6 +58,7 @@ _error_flags = {}
 
 LIBRARY_WORKSPACE_BYTES = 32 << 20
 _workspaces = {}
+_second_workspaces = threading.local()           # device -> tensor, of each thread
 _direct_ok = None
 
 
@@ -349,15 +351,16 @@ def _direct_library(device) -> bool:
 
 
 def _library_workspace(device) -> torch.Tensor:
-    """Products of two streams may run at once and then need two workspaces.  Every host thread has a second stream of its own, so
-    the one for products there belongs to the step that asked for that stream, and goes with it; without a step to a stream's handle."""
+    """Products of two streams may run at once and then need two workspaces.  Every host thread has a second stream of its own, so the one for
+    products there is the thread's too, and goes with it; a captured step, which any thread may run again, brings its own.  (One that every
+    step brings costs 10 to 30 us a prompt, and 0.4 ms to 10 in the first of an engine.)"""
     side, scratch = ops.second_stream()
     if scratch is not None:
         return scratch(LIBRARY_WORKSPACE_BYTES)
-    key = (str(device), side)
-    work = _workspaces.get(key)
+    kept, key = _workspaces if side is None else _second_workspaces.__dict__, str(device)
+    work = kept.get(key)
     if work is None:
-        work = _workspaces[key] = torch.empty(LIBRARY_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
+        work = kept[key] = torch.empty(LIBRARY_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
     return work
 
 

@@ -692,7 +692,8 @@ def on_side_stream(scratch=None):
     """This library's launches inside go to the device's second stream, which continues from where the current one stands; the
     caller joins (`join(side)`, side being what this yields) before anything reads what they write, and lets go of none of their
     tensors before that.  Only for work that launches kernels of this library and nothing through the tensor framework.
-    `scratch(bytes)` -> uint8 tensor: memory of the step for what a launch inside needs beside its operands (a library product's workspace)."""
+    `scratch(bytes)` -> uint8 tensor: memory of the step for what a launch inside needs beside its operands (a library product's workspace),
+    for a step that is captured; else that is the host thread's."""
     side, outer, outer_scratch = side_stream(), getattr(_launch_on, "side", None), getattr(_launch_on, "scratch", None)
     fork(side)
     _launch_on.side, _launch_on.scratch = side, scratch or outer_scratch

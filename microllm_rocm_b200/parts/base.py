@@ -162,6 +162,7 @@ class StepContext:
     # tensor trace.  Such a step runs every layer call by call.
     tensor_sink: Optional[Callable[[str, torch.Tensor], None]] = None
     mean_seq_len: float = 0.0      # mean length of the sequences after the step (0: not known, taken for the longest)
+    captured: bool = False         # its launches are recorded and run again, by whichever thread: nothing of theirs may be a thread's own
 
     @property
     def decode_only(self) -> bool:

@@ -105,7 +105,7 @@ class ParallelMixers(Mixer):
         run = lambda i: self.branches[i][3].forward(x, ctx, sub_views(views, self.branches[i][0]))
         aside, side = self._aside(), None
         if aside is not None:
-            with ops.on_side_stream(lambda size: ctx.buffer("parallel.second_stream", (size,), torch.uint8)) as side:
+            with ops.on_side_stream((lambda size: ctx.buffer("parallel.second_stream", (size,), torch.uint8)) if getattr(ctx, "captured", False) else None) as side:
                 terms[aside] = run(aside)
         try:
             for i in range(len(self.branches)):

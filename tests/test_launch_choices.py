@@ -55,9 +55,11 @@ def test_only_steps_of_one_token_a_sequence_move_the_convolutions_state_in_its_l
     assert calls[0][1]["move"] == (1 if alone else 0)
 
 
-def test_library_products_on_second_streams_have_a_workspace_of_their_step(calls, monkeypatch):
+@pytest.mark.parametrize("captured", [False, True])
+def test_library_products_on_second_streams_have_a_workspace_of_their_thread_or_captured_step(calls, monkeypatch, captured):
     """Every host thread has a second stream of its own, and nothing orders two of them: their products may not share a workspace, with each other or
-    with the first stream's.  Those of one step may, and theirs goes when the step does."""
+    with the first stream's.  Those of one thread may, and theirs goes when the thread does; a captured step, which another thread may run again
+    while the one that captured it goes on, has its own."""
     import gc
     import threading
     import weakref
@@ -84,11 +86,11 @@ def test_library_products_on_second_streams_have_a_workspace_of_their_step(calls
     def context():
         ids = torch.zeros(8, dtype=torch.int32)
         return StepContext(num_tokens=8, num_seqs=1, token_ids=ids, positions=ids, token_seq=ids, seq_starts=ids, seq_pos0=ids, seq_lens=ids, block_tables={},
-                           state_slots=ids, logit_rows=ids, error_flag=ids)
+                           state_slots=ids, logit_rows=ids, error_flag=ids, captured=captured)
     mixer = ParallelMixers.__new__(ParallelMixers)
     mixer.branches = [("left", 1.0, "", Main()), ("right", 1.0, "", Aside())]
     contexts, used = [context(), context()], [None, None]
-    lock = threading.Lock()
+    lock, both, gone = threading.Lock(), threading.Barrier(2), []
 
     def work(i):
         with lock:
@@ -96,15 +98,20 @@ def test_library_products_on_second_streams_have_a_workspace_of_their_step(calls
             for _ in range(2):                                # two layers of one step
                 mixer.forward_terms(torch.zeros(8, 8), contexts[i], {})
             used[i] = [(a["stream"], a["workspace"]) for fn, a in calls if fn == "mlb_lt_matmul"]
+            mixer.forward_terms(torch.zeros(8, 8), context(), {})          # another step of this thread
+            used[i].append(next((a["stream"], a["workspace"]) for fn, a in calls[-4:] if fn == "mlb_lt_matmul" and a["stream"] != 1))
+            gone.extend(weakref.ref(t) for t in list(contexts[i].extras.values()) + list(gemm_bf16._second_workspaces.__dict__.values()))
+        both.wait(timeout=30)                                 # (until both have theirs)
     threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
+    other = [u.pop()[1] for u in used]
     aside, first = [{w for s, w in u if s != 1} for u in used], [{w for s, w in u if s == 1} for u in used]
     assert [len(u) for u in used] == [8, 8] and all(len(s) == 1 for s in aside + first)
     assert aside[0] != aside[1] and first[0] == first[1] and not (aside[0] | aside[1]) & first[0]
-    gone = [weakref.ref(t) for ctx in contexts for t in ctx.extras.values()]
+    assert captured or other == [w for s in aside for w in s]             # (an eager step takes its thread's again)
     contexts.clear()
     gc.collect()
     assert gone and not any(r() is not None for r in gone)
