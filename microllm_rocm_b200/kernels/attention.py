@@ -216,7 +216,7 @@ def _plan(ctx, group: int, num_kv_heads: int, use_tc: bool, beside_mma_products:
         listed_splits = decode_splits(len(listed) * tiles_per_token * num_kv_heads, longest, sms)
         ring = decode_ring_pays(len(listed) * tiles_per_token * num_kv_heads, listed_splits, longest, sms, beside_mma_products)
     plan = (work_dev, len(work), 1 if decode else 0, splits, tc_dev, len(tc_work), listed_dev, len(listed) * tiles_per_token,
-            listed_splits, ring, longest, mean)
+            listed_splits, ring, longest, mean, sms)
     ctx.extras[key] = plan
     return plan
 
@@ -248,17 +248,17 @@ def paged_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, ctx
         raise KernelError("paged_attention: the tensor-core kernel wants bf16 queries, pages and output")
     bias_args = ops.distance_bias_args(bias, num_heads)
     use_tc = tc_supported(head_dim, page_size, scale) and q.is_contiguous() and out.is_contiguous()
-    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring, longest, mean = _plan(
+    work, num_work, mode, splits, tc_work, num_tc, listed, num_listed, listed_splits, ring, longest, mean, sms = _plan(
         ctx, num_heads // num_kv_heads, num_kv_heads, use_tc, beside_mma_products)
     ring_bits = 4 if (ring if DECODE_RING is None else DECODE_RING) else 8
-    visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
-    cut = splits if mode else listed_splits
-    possible = own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring) and own_rings_suit(
-        num_work if mode else num_listed, cut, (num_work if mode else num_listed) * num_kv_heads * cut,
-        min(mean, visible) / max(1, min(longest, visible)), sm_count(q.device))
-    own = possible and own_rings_pay(cut, longest, beside_mma_products, visible)
-    if mode and possible:                # (where there is no choice, a captured step has nothing to be planned again for)
-        ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own
+    decoding, cut = (num_work, splits) if mode else (num_listed, listed_splits)
+    own = False
+    if decoding and own_rings_possible(head_dim, num_heads // num_kv_heads, cut, ring):
+        visible = min(int(window) + int(keep_first) if window else 1 << 30, int(chunk) if chunk else 1 << 30)
+        if own_rings_suit(decoding, cut, decoding * num_kv_heads * cut, min(mean, visible) / max(1, min(longest, visible)), sms):
+            own = own_rings_pay(cut, longest, beside_mma_products, visible)
+            if mode:                     # (where there is no choice, a captured step has nothing to be planned again for)
+                ctx.extras[("attention_rings", splits, bool(beside_mma_products), visible)] = own
     if own if OWN_RINGS is None else OWN_RINGS:
         ring_bits |= 16
     side = None
